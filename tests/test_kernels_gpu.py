@@ -105,6 +105,25 @@ def test_gemm_simt(k, dtype, M, N, K):
     close(res, ref + res0.double(), dtype, "gemm accumulate")
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M,N,K", [(4, 40, 136), (8, 17, 8), (9, 500, 256), (17, 129, 520), (33, 64, 1000), (64, 1024, 264),
+                                   (65, 4800, 40), (20, 4800, 64), (129, 9472, 48), (640, 640, 80), (70, 200, 13)])
+def test_gemm_simt_forms_agree(k, dtype, M, N, K):
+    """Every form (few rows, three tile sizes, with and without 16-byte rows) adds an output's products in the order of k:
+    a row has the same bits alone and in any batch, and matches the float64 product within the bound of K ordered float32
+    sums, K * 2^-24 * sum |a w| (the products are exact for bfloat16 and rounded once with the sum for float32)."""
+    a = rnd((M, K), 5, dtype).cuda()
+    w = rnd((N, K), 6, dtype, 0.1).cuda()
+    got = k.gemm_simt(a, w, out_dtype=torch.float32)
+    bound = K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T) + 1e-30
+    assert ((got.double() - a.double() @ w.double().T).abs() <= bound).all()
+    for r in sorted({0, M // 2, M - 1}):
+        assert torch.equal(k.gemm_simt(a[r:r + 1], w, out_dtype=torch.float32)[0], got[r])
+    wide = torch.empty((M, K + 3), dtype=dtype, device="cuda")[:, 3:]      # rows that no 16-byte load can take
+    wide.copy_(a)
+    assert torch.equal(k.gemm_simt(wide, w, out_dtype=torch.float32), got)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 331, 80), (8, 6144, 2048), (5, 100, 8200), (16, 2048, 512), (9, 48, 64),
                                    (33, 257, 1000), (64, 1030, 2048), (3, 65536 + 8, 256)])
 def test_gemm_skinny(k, M, N, K):

@@ -5,12 +5,24 @@
 // walks k = 0 .. K-1 in order, so a row's result does not depend on M, on the row's place in
 // the batch or on the tile it falls in (reference: one dot product per output row,
 // src/model.zig:923-1026; float32 dot src/quant.zig:424-431; `accumulate` = residual add,
-// src/model.zig:918-920).
+// src/model.zig:918-920).  All kernels here keep that order, so they give the same bits and the
+// launcher may pick among them by size.
 #include "common.cuh"
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, PAD = 4;
+// ------------------------------------------------------------------------------ tiles
+// A block owns BM x BN outputs, a thread TM x TN of them in groups of 4 adjacent rows and 4 adjacent columns.  The
+// operands lie in shared memory as [k][row], so that a group is one 16-byte load; two buffers, PF k blocks further on being
+// fetched into registers while this one is multiplied (one barrier per k block).
+//
+// What bounds it: 128 FMAs a cycle and SM (74 TFLOP/s) against 128 bytes a cycle from shared memory into registers, which
+// 8 x 8 outputs per thread just balance (8 x 4 need 1.5 times, 4 x 4 twice the time of their FMAs for their loads); packed
+// FMAs (fma.rn.f32x2) leave the issue slots to the loads, 7 to 10 % over single ones.  8 x 16 outputs (one block of 128 threads
+// in place of two of 256 per SM) were no faster.  Float32, [450, K] rows, microseconds before (64 x 64 tiles, 4 x 4 outputs, one
+// buffer) and now: N = 9216, K = 1024 320 -> 192 (44 TFLOP/s); N = 65536 1962 -> 1230 (49 TFLOP/s); N = 1024, K = 4608
+// 334 -> 169; N = 1024, K = 1024 72 -> 42.
+constexpr int BK = 16, PAD = 4;
 
 template <typename T>
 __device__ __forceinline__ void load4(const T* __restrict__ p, bool vec_ok, int k0, int K, bool row_ok, float out[4]) {
@@ -34,78 +46,303 @@ __device__ __forceinline__ void load4(const T* __restrict__ p, bool vec_ok, int 
   for (int j = 0; j < 4; ++j) out[j] = (k0 + j < K) ? to_f32(p[k0 + j]) : 0.f;
 }
 
-template <typename TA, typename TW, typename TC>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W,
-                                                        TC* __restrict__ C, const float* __restrict__ bias, int M, int N,
-                                                        int K, int lda, int ldw, int ldc, int accumulate, int vecA,
-                                                        int vecW) {
-  __shared__ __align__(16) float As[BK][BM + PAD];
-  __shared__ __align__(16) float Ws[BK][BN + PAD];
+// Two float32 FMAs in one instruction, each rounded as fmaf rounds.
+__device__ __forceinline__ void fma2(float2& d, float a, float2 b) {
+  unsigned long long dd, aa, bb;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(aa) : "f"(a));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(bb) : "f"(b.x), "f"(b.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(dd) : "f"(d.x), "f"(d.y));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(dd) : "l"(aa), "l"(bb));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(dd));
+}
+
+template <int BM, int BN, int TM, int TN, int PF, typename TA, typename TW, typename TC>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN), TM * TN >= 64 ? 2 : 3)
+    gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restrict__ C, const float* __restrict__ bias,
+                     int M, int N, int K, int lda, int ldw, int ldc, int accumulate, int vecA, int vecW) {
+  constexpr int TX = BN / TN, TY = BM / TM, THREADS = TX * TY;
+  constexpr int GM = TM / 4, GN = TN / 4;                   // groups of 4 rows / columns per thread
+  constexpr int LA = BM * BK / 4 / THREADS, LW = BN * BK / 4 / THREADS;   // 4-value pieces a thread fetches per k block
+  static_assert(LA * THREADS * 4 == BM * BK && LW * THREADS * 4 == BN * BK, "whole pieces per thread");
+  __shared__ __align__(16) float As[2][BK][BM + PAD];
+  __shared__ __align__(16) float Ws[2][BK][BN + PAD];
   const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
+  const int tx = tid % TX, ty = tid / TX;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int lrow = tid >> 2, lk = (tid & 3) * 4;
 
-  float acc[4][4];
+  float2 acc[TM][TN / 2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int j = 0; j < TN / 2; ++j) acc[i][j] = make_float2(0.f, 0.f);
 
-  const bool a_ok = (m0 + lrow) < M, w_ok = (n0 + lrow) < N;
-  const TA* a_row = A + (size_t)(a_ok ? m0 + lrow : 0) * lda;
-  const TW* w_row = W + (size_t)(w_ok ? n0 + lrow : 0) * ldw;
-
-  for (int kb = 0; kb < K; kb += BK) {
-    float av[4], wv[4];
-    load4<TA>(a_row, vecA, kb + lk, K, a_ok, av);
-    load4<TW>(w_row, vecW, kb + lk, K, w_ok, wv);
+  float av[PF][LA][4], wv[PF][LW][4];
+  auto fetch = [&](int kb, int f) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      As[lk + j][lrow] = av[j];
-      Ws[lk + j][lrow] = wv[j];
+    for (int l = 0; l < LA; ++l) {
+      const int p = tid + l * THREADS, r = p >> 2, k = (p & 3) * 4;
+      const bool ok = m0 + r < M;
+      load4<TA>(A + (size_t)(ok ? m0 + r : 0) * lda, vecA, kb + k, K, ok, av[f][l]);
     }
-    __syncthreads();
 #pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      const float4 a = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
-      const float4 b = *reinterpret_cast<const float4*>(&Ws[k][tx * 4]);
-      const float ar[4] = {a.x, a.y, a.z, a.w};
-      const float br[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(ar[i], br[j], acc[i][j]);
+    for (int l = 0; l < LW; ++l) {
+      const int p = tid + l * THREADS, r = p >> 2, k = (p & 3) * 4;
+      const bool ok = n0 + r < N;
+      load4<TW>(W + (size_t)(ok ? n0 + r : 0) * ldw, vecW, kb + k, K, ok, wv[f][l]);
     }
-    __syncthreads();
+  };
+  auto put = [&](int buf, int f) {
+#pragma unroll
+    for (int l = 0; l < LA; ++l) {
+      const int p = tid + l * THREADS, r = p >> 2, k = (p & 3) * 4;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) As[buf][k + j][r] = av[f][l][j];
+    }
+#pragma unroll
+    for (int l = 0; l < LW; ++l) {
+      const int p = tid + l * THREADS, r = p >> 2, k = (p & 3) * 4;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) Ws[buf][k + j][r] = wv[f][l][j];
+    }
+  };
+
+  // PF k blocks are under way in registers; the body of PF rounds is unrolled so that each has registers of its own
+#pragma unroll
+  for (int f = 0; f < PF; ++f) fetch(f * BK, f);            // beyond K: zeros
+  put(0, 0);
+  __syncthreads();
+  int buf = 0;
+  for (int kb0 = 0; kb0 < K; kb0 += PF * BK) {
+#pragma unroll
+    for (int f = 0; f < PF; ++f) {
+      const int kb = kb0 + f * BK;
+      if (kb >= K) break;
+      fetch(kb + PF * BK, f);                               // this block's values are in shared memory since the round before
+#pragma unroll
+      for (int k = 0; k < BK; ++k) {
+        float a[TM];
+        float2 b[TN / 2];
+#pragma unroll
+        for (int i = 0; i < GM; ++i) {
+          const float4 v = *reinterpret_cast<const float4*>(&As[buf][k][i * (BM / GM) + ty * 4]);
+          a[4 * i] = v.x; a[4 * i + 1] = v.y; a[4 * i + 2] = v.z; a[4 * i + 3] = v.w;
+        }
+#pragma unroll
+        for (int j = 0; j < GN; ++j) {
+          const float4 v = *reinterpret_cast<const float4*>(&Ws[buf][k][j * (BN / GN) + tx * 4]);
+          b[2 * j] = make_float2(v.x, v.y);
+          b[2 * j + 1] = make_float2(v.z, v.w);
+        }
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN / 2; ++j) fma2(acc[i][j], a[i], b[j]);
+      }
+      if (kb + BK < K) {
+        put(buf ^ 1, (f + 1) % PF);
+        __syncthreads();
+        buf ^= 1;
+      }
+    }
   }
 
+  const bool vecC = sizeof(TC) == 4 && ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + (i / 4) * (BM / GM) + ty * 4 + (i & 3);
     if (m >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= N) continue;
-      float v = acc[i][j];
-      if (bias) v += bias[n];
+    for (int j = 0; j < GN; ++j) {
+      const int n = n0 + j * (BN / GN) + tx * 4;
+      float v[4] = {acc[i][2 * j].x, acc[i][2 * j].y, acc[i][2 * j + 1].x, acc[i][2 * j + 1].y};
       TC* c = C + (size_t)m * ldc + n;
-      if (accumulate) v += to_f32(*c);
-      *c = from_f32<TC>(v);
+      if (vecC && n + 3 < N) {
+        if constexpr (sizeof(TC) == 4) {
+          if (bias) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] += bias[n + e];
+          }
+          if (accumulate) {
+            const float4 o = *reinterpret_cast<const float4*>(c);
+            v[0] += o.x; v[1] += o.y; v[2] += o.z; v[3] += o.w;
+          }
+          *reinterpret_cast<float4*>(c) = make_float4(v[0], v[1], v[2], v[3]);
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (n + e >= N) continue;
+          float t = v[e];
+          if (bias) t += bias[n + e];
+          if (accumulate) t += to_f32(c[e]);
+          c[e] = from_f32<TC>(t);
+        }
+      }
     }
   }
 }
 
-template <typename TA, typename TW, typename TC>
-int launch(const void* A, const void* W, void* C, const float* bias, int M, int N, int K, int lda, int ldw, int ldc,
-           int accumulate, cudaStream_t stream) {
+// ------------------------------------------------------------------------------ few rows
+// Up to 64 rows of A (single-token steps, short prompts): what counts is that the weights stream and that the chain of K
+// dependent FMAs runs at its 4 cycles each.  A block owns 16 weight rows; its threads keep a ring of k blocks of W and
+// A under way with 16-byte asynchronous copies, and thread (row, group) adds the products of its weight row with the
+// rows group, group + GROUPS, ... of A in k order, the operands of the next 16 k in registers before they are needed.
+// A row of the ring is 16 bytes longer than its values, so that the 16-byte loads of 8 adjacent rows fall into different
+// banks.  Two float32 rows, microseconds before (the tiled form: 64 x 64, one buffer) and now: N = 1024, K = 4608 385 -> 23
+// (K dependent FMAs alone are 9.4); N = 9216, K = 1024 86 -> 17; N = 65536 278 -> 74 (3.6 TB/s).
+constexpr int FEW_ROWS = 16, FEW_MAX_M = 64;
+
+__device__ __forceinline__ void cp16(void* dst, const void* src, bool in) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = in ? 16 : 0;                                 // fewer source bytes than 16: the rest is zero-filled
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+
+template <typename T>
+__device__ __forceinline__ float4 four(const T* p) {
+  if constexpr (sizeof(T) == 4) {
+    return *reinterpret_cast<const float4*>(p);
+  } else {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&v.x);
+    const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&v.y);
+    return make_float4(__low2float(lo), __high2float(lo), __low2float(hi), __high2float(hi));
+  }
+}
+
+// GROUPS: threads per weight row; NT: rows of A per thread (GROUPS * NT >= M); STAGES of the ring.
+template <int GROUPS, int NT, int STAGES, typename T, typename TC>
+__global__ void __launch_bounds__(FEW_ROWS * GROUPS)
+    gemm_few_kernel(const T* __restrict__ A, const T* __restrict__ W, TC* __restrict__ C, const float* __restrict__ bias,
+                    int M, int N, int K, int lda, int ldw, int ldc, int accumulate) {
+  constexpr int THREADS = FEW_ROWS * GROUPS;
+  constexpr int PIECE = 16 / (int)sizeof(T), KC = 512 / (int)sizeof(T), LD = KC + PIECE;   // 512 bytes of a row per k block
+  extern __shared__ __align__(16) unsigned char few_smem[];
+  T* ring = reinterpret_cast<T*>(few_smem);
+  const int rows = FEW_ROWS + M;                             // W's rows, then A's
+  const int tid = threadIdx.x, n0 = blockIdx.x * FEW_ROWS;
+  const int n_kb = (K + KC - 1) / KC;
+  // a warp copies whole rows (32 pieces of 16 bytes): lane = piece, warps take rows in turn
+  const int e = (tid & 31) * PIECE;
+  auto request = [&](int kb) {
+    if (kb < n_kb) {
+      T* dst = ring + (size_t)(kb % STAGES) * rows * LD + e;
+      const int k = kb * KC + e;
+      const bool k_in = k < K;                               // K is a whole number of pieces
+      const T* wk = W + (k_in ? k : 0);
+      const T* ak = A + (k_in ? k : 0);
+#pragma unroll
+      for (int r = tid >> 5; r < FEW_ROWS; r += THREADS / 32) {
+        const bool in = k_in && n0 + r < N;
+        cp16(dst + r * LD, wk + (size_t)(in ? n0 + r : 0) * ldw, in);
+      }
+      for (int r = tid >> 5; r < M; r += THREADS / 32) cp16(dst + (FEW_ROWS + r) * LD, ak + (size_t)r * lda, k_in);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; ++s) request(s);
+  const int row = tid % FEW_ROWS, group = tid / FEW_ROWS;
+  float acc[NT];
+  int at[NT];                                                // where the rows of A lie in a stage
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    acc[t] = 0.f;
+    at[t] = (FEW_ROWS + (group + t * GROUPS < M ? group + t * GROUPS : 0)) * LD;   // no such row: another's, not stored
+  }
+  for (int kb = 0; kb < n_kb; ++kb) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+    __syncthreads();                                         // the k block is here, and nobody reads the one before it
+    const T* st = ring + (size_t)(kb % STAGES) * rows * LD;
+    float4 x[2][4], y[2][NT][4];
+    auto read = [&](int k, int b) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        x[b][i] = four(st + row * LD + k + 4 * i);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) y[b][t][i] = four(st + at[t] + k + 4 * i);
+      }
+    };
+    read(0, 0);
+    request(kb + STAGES - 1);
+#pragma unroll
+    for (int k = 0; k < KC; k += 16) {
+      const int b = (k >> 4) & 1;
+      if (k + 16 < KC) read(k + 16, b ^ 1);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].x, x[b][i].x, acc[t]);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].y, x[b][i].y, acc[t]);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].z, x[b][i].z, acc[t]);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].w, x[b][i].w, acc[t]);
+      }
+    }
+  }
+  const int n = n0 + row;
+  if (n >= N) return;
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    const int m = group + t * GROUPS;
+    if (m >= M) continue;
+    float v = acc[t];
+    if (bias) v += bias[n];
+    TC* c = C + (size_t)m * ldc + n;
+    if (accumulate) v += to_f32(*c);
+    *c = from_f32<TC>(v);
+  }
+}
+
+template <int BM, int BN, int TM, int TN, int PF, typename T, typename TC>
+int launch_tiles(const void* A, const void* W, void* C, const float* bias, int M, int N, int K, int lda, int ldw, int ldc,
+                 int accumulate, cudaStream_t stream) {
   const int vecA = (lda % 4 == 0) && ((uintptr_t)A % 16 == 0);
   const int vecW = (ldw % 4 == 0) && ((uintptr_t)W % 16 == 0);
   dim3 grid(ceil_div_i(N, BN), ceil_div_i(M, BM));
-  gemm_simt_kernel<TA, TW, TC><<<grid, 256, 0, stream>>>((const TA*)A, (const TW*)W, (TC*)C, bias, M, N, K, lda, ldw,
-                                                          ldc, accumulate, vecA, vecW);
+  gemm_simt_kernel<BM, BN, TM, TN, PF, T, T, TC><<<grid, (BM / TM) * (BN / TN), 0, stream>>>(
+      (const T*)A, (const T*)W, (TC*)C, bias, M, N, K, lda, ldw, ldc, accumulate, vecA, vecW);
   return ZK_LAUNCH_STATUS();
+}
+
+template <int GROUPS, int NT, int STAGES, typename T, typename TC>
+int launch_few(const void* A, const void* W, void* C, const float* bias, int M, int N, int K, int lda, int ldw, int ldc,
+               int accumulate, cudaStream_t stream) {
+  auto kern = gemm_few_kernel<GROUPS, NT, STAGES, T, TC>;
+  const size_t smem = (size_t)STAGES * (FEW_ROWS + M) * (512 + 16);
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  kern<<<ceil_div_i(N, FEW_ROWS), FEW_ROWS * GROUPS, smem, stream>>>((const T*)A, (const T*)W, (TC*)C, bias, M, N, K, lda, ldw,
+                                                                     ldc, accumulate);
+  return ZK_LAUNCH_STATUS();
+}
+
+template <typename T, typename TC>
+int launch(const void* A, const void* W, void* C, const float* bias, int M, int N, int K, int lda, int ldw, int ldc,
+           int accumulate, cudaStream_t stream) {
+  constexpr int PIECE = 16 / (int)sizeof(T);
+  const bool pieces = K % PIECE == 0 && lda % PIECE == 0 && ldw % PIECE == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0;
+  // The few-row form reads A once per 16 weight rows, which pays while the weights are the larger part or a tiled form would
+  // leave most SMs idle.  Microseconds at 20 rows, few / 32 x 32 tiles: N = 1024 15 / 27 (K = 1024), 50 / 117 (K = 4608);
+  // N = 9216 44 / 31.
+  if (pieces && (M <= 8 || (M <= FEW_MAX_M && ceil_div_i(N, FEW_ROWS) <= 2 * 148))) {
+    if (M <= 4) return launch_few<4, 1, 6, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
+    if (M <= 8) return launch_few<8, 1, 6, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
+    if (M <= 16) return launch_few<16, 1, 5, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
+    if (M <= 32) return launch_few<16, 2, 4, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
+    return launch_few<16, 4, 3, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
+  }
+  // The largest tile that still gives (nearly) every SM a block.  450 rows, microseconds with 128 x 128 / 64 x 64 / 32 x 32
+  // tiles: N = 9216, K = 1024 195 / 224 / 326; N = 1024, K = 4608 474 / 169 / 199; 100 rows of the latter 463 / 165 / 111.
+  if (ceil_div_i(M, 128) * ceil_div_i(N, 128) >= 148)
+    return launch_tiles<128, 128, 8, 8, 1, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
+  if (ceil_div_i(M, 64) * ceil_div_i(N, 64) >= 100)
+    return launch_tiles<64, 64, 8, 4, 2, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
+  return launch_tiles<32, 32, 4, 4, 4, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
 }
 
 }  // namespace
@@ -115,10 +352,10 @@ extern "C" int zk_gemm_simt(const void* A, const void* W, void* C, const float* 
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || lda < K || ldw < K || ldc < N) return ZK_EINVAL;
   if (in_dtype == ZK_F32 && out_dtype == ZK_F32)
-    return launch<float, float, float>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
+    return launch<float, float>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
   if (in_dtype == ZK_BF16 && out_dtype == ZK_F32)
-    return launch<bf16, bf16, float>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
+    return launch<bf16, float>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
   if (in_dtype == ZK_BF16 && out_dtype == ZK_BF16)
-    return launch<bf16, bf16, bf16>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
+    return launch<bf16, bf16>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
   return ZK_EINVAL;
 }
