@@ -890,3 +890,29 @@ def test_dependent_launches_keep_the_order_of_a_chain(k, rows):
     assert torch.isfinite(a).all() and a.abs().max() > 0
     assert torch.equal(a, b)
     assert k.status_word("cuda").item() == 0
+
+
+@pytest.mark.parametrize("M,splits", [(17, 1), (33, 2), (64, 4), (49, 8), (64, 1), (130, 1), (300, 1)])
+@pytest.mark.parametrize("glu", ["silu", "relu", "clamp"])
+def test_gemm_tc_gated_units_over_the_whole_range(k, M, splits, glu):
+    """Weights that pick column 0 as every gate and column 1 as every up: the unit alone, for gates from -1e4 to 1e4.
+    The float32 unit is a few ulp off (8 * 2^-23) and is rounded once to bfloat16, whose 8 significant bits
+    give 2^-8 of the value; below 1e-35 it may be 0."""
+    F, K = 256, 576
+    x = torch.zeros(M, K)
+    x[:, 0] = torch.cat([torch.linspace(-130, 130, M - 9), torch.tensor([-1e4, 1e4, 0.0, -0.0, -87.5, -88.0, -1e-3, 1e-3, 9.0])])
+    x[:, 1] = torch.linspace(-3, 5, M)
+    w = torch.zeros(2 * F, K)
+    w.view(F // 16, 2, 16, K)[:, 0, :, 0] = 1
+    w.view(F // 16, 2, 16, K)[:, 1, :, 1] = 1
+    x, w = x.bfloat16().cuda(), w.bfloat16().cuda()
+    g, u = x[:, 0].double(), x[:, 1].double()
+    if glu == "clamp":
+        g = g.clamp(max=7.0)
+        ref = g * torch.sigmoid(1.702 * g) * (u.clamp(-7.0, 7.0) + 1)
+        got = k.gemm_tc(x, w, swiglu=True, splits=splits, glu_clamp=(7.0, 1.702))
+    else:
+        ref = (g * torch.sigmoid(g) if glu == "silu" else torch.relu(g)) * u
+        got = k.gemm_tc(x, w, swiglu=True, splits=splits, glu_act=glu)
+    err = (got.double() - ref[:, None]).abs()
+    assert (err <= ref.abs()[:, None] * (2 ** -8 + 8 * 2 ** -23) + 1e-35).all()

@@ -43,14 +43,55 @@ constexpr int THREADS = 192;     // producer warp, MMA warp, four epilogue warps
 
 // The gated unit of the fused epilogues: silu(g) * u, with limit > 0 the clamped unit described in Params, with limit < 0
 // relu(g) * u.
+// A unit that is stored as bfloat16 divides with __fdividef (2 ulp of float32, 1 / 16,000 of the rounding that follows; the
+// denominator is 1 or more, and where it passes 2^126 a quotient of 1e-36 becomes 0).  What bounded the epilogues was one
+// warp per scheduler waiting through branch after branch: the IEEE division's way to its slow path and the choice of the
+// unit stood between any two of a thread's units, so that none overlapped.  The epilogue of a 256 x 256 tile, 128 units a
+// thread, took 14 us where the tile's MMAs take 4 (K = 1024) to 8 (K = 2048).  8,192 rows: w1|w3 with K = 1024, N = 9216
+// 225 us, without the division's branch 193, with the unit chosen outside the loop (glu_units) 103; K = 2048, N = 16384
+// 481 -> 353 us.
+template <typename TC>
+__device__ __forceinline__ float glu_quotient(float g, float e) {
+  if constexpr (sizeof(TC) == 2) return __fdividef(g, 1.0f + e);
+  else return g / (1.0f + e);
+}
+template <typename TC>
 __device__ __forceinline__ float glu_unit(float g, float u, float limit, float alpha) {
   if (limit > 0.f) {
     g = fminf(g, limit);
     u = fminf(fmaxf(u, -limit), limit) + 1.0f;
-    return g / (1.0f + expf(-alpha * g)) * u;
+    return glu_quotient<TC>(g, expf(-alpha * g)) * u;
   }
   if (limit < 0.f) return fmaxf(g, 0.f) * u;
-  return g / (1.0f + expf(-g)) * u;
+  return glu_quotient<TC>(g, expf(-g)) * u;
+}
+// N units, which one decided once and not per unit: f(j, unit of g[j] and u(j)).
+template <typename TC, int N, typename U, typename F>
+__device__ __forceinline__ void glu_units(const float* g, U u, float limit, float alpha, F f) {
+  if (limit == 0.f) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) f(j, glu_unit<TC>(g[j], u(j), 0.f, 0.f));
+  } else if (limit < 0.f) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) f(j, glu_unit<TC>(g[j], u(j), -1.f, 0.f));
+  } else {
+#pragma unroll
+    for (int j = 0; j < N; ++j) f(j, glu_unit<TC>(g[j], u(j), limit, alpha));
+  }
+}
+
+// v[2 H]: lanes below 16 hold gate rows, lane l + 16 the up row of lane l, one value per token.  Afterwards lane l has gate
+// and up of the tokens 0..H-1 and lane l + 16 of H..2H-1: every lane applies units, with one shuffle for two tokens.
+// w1|w3 of 64 tokens, K = 2048, N = 16384, weights not in L2: 24.3 us with units in half of the lanes, now 16.0 (unsplit).
+template <int H>
+__device__ __forceinline__ void share_units(const float* v, int lane, float (&gate)[H], float (&up)[H]) {
+  const bool upper = (lane & 16) != 0;
+#pragma unroll
+  for (int j = 0; j < H; ++j) {
+    const float got = __shfl_xor_sync(0xffffffffu, upper ? v[j] : v[j + H], 16);
+    gate[j] = upper ? got : v[j];
+    up[j] = upper ? v[j + H] : got;
+  }
 }
 
 struct Params {
@@ -303,7 +344,7 @@ __global__ void __launch_bounds__(THREADS)
             const int gc = (oc / 16) * 32 + (oc % 16);      // its gate's column; the up is 16 further
             if (h_base + oc < F) {
               const float gate = srow[gc], up = srow[gc + 16];
-              hrow[oc] = from_f32<TC>(glu_unit(gate, up, p.glu_limit, p.glu_alpha));
+              hrow[oc] = from_f32<TC>(glu_unit<TC>(gate, up, p.glu_limit, p.glu_alpha));
             }
           }
         }
@@ -378,14 +419,14 @@ __global__ void __launch_bounds__(THREADS)
         }
         if (p.swiglu) {
           // a warp's 32 rows are 16 gate rows and their 16 up rows (N is a multiple of 32, so the
-          // whole warp is on one side of N): lane l < 16 takes the up value of lane l + 16
-          const int f = (n >> 5) * 16 + (n & 15);   // output column of this gate row
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float up = __shfl_down_sync(0xffffffffu, v[j], 16);
-            if ((lane & 16) == 0 && n < p.N && c0 + j < p.M)
-              C[(size_t)(c0 + j) * p.ldc + f] = from_f32<TC>(glu_unit(v[j], up, p.glu_limit, p.glu_alpha));
-          }
+          // whole warp is on one side of N): lanes l and l + 16 share the 16 tokens of output column f
+          const int f = (n >> 5) * 16 + (n & 15);
+          float gate[8], up[8];
+          share_units<8>(v, lane, gate, up);
+          const int t0 = c0 + ((lane & 16) ? 8 : 0);
+          glu_units<TC, 8>(gate, [&](int j) { return up[j]; }, p.glu_limit, p.glu_alpha, [&](int j, float h) {
+            if (n < p.N && t0 + j < p.M) C[(size_t)(t0 + j) * p.ldc + f] = from_f32<TC>(h);
+          });
         } else {
           const bool n_in = n < p.N;
           const float b = (p.bias && n_in) ? p.bias[n] : 0.f;
@@ -446,23 +487,33 @@ __global__ void __launch_bounds__(THREADS)
                 pv[i][z] = t < p.M ? ld_remote_f32(base + (unsigned)(t * BM + row) * 4u, (unsigned)z) : 0.f;
               old[i] = (t < p.M && n_in && p.accumulate) ? to_f32(C[(size_t)t * p.ldc + n]) : 0.f;
             }
-            float sq[TOK];
+            float sq[TOK], sum[TOK];
+#pragma unroll
+            for (int i = 0; i < TOK; ++i) {
+              const int t = t0 + i * SP;
+              sum[i] = 0.f;
+#pragma unroll
+              for (int z = 0; z < SP; ++z) sum[i] += pv[i][z];
+              if (p.ssq_in && t < p.M) sum[i] *= row_scale[t];
+              sum[i] += b;
+            }
+            if (p.swiglu) {   // as in the unsplit epilogue: a warp's rows are 16 gate rows and their 16 up rows
+              float gate[TOK / 2], up[TOK / 2];
+              share_units<TOK / 2>(sum, lane, gate, up);
+              const int tl = t0 + ((lane & 16) ? TOK / 2 : 0) * SP;
+              glu_units<TC, TOK / 2>(gate, [&](int j) { return up[j]; }, p.glu_limit, p.glu_alpha, [&](int j, float h) {
+                const int t = tl + j * SP;
+                if (n_in && t < p.M) C[(size_t)t * p.ldc + (n >> 5) * 16 + (n & 15)] = from_f32<TC>(h);
+              });
+              continue;
+            }
 #pragma unroll
             for (int i = 0; i < TOK; ++i) {
               const int t = t0 + i * SP;
               sq[i] = 0.f;
               if (t >= p.M) continue;        // the same for every lane
-              float acc = 0.f;
-#pragma unroll
-              for (int z = 0; z < SP; ++z) acc += pv[i][z];
-              if (p.ssq_in) acc *= row_scale[t];
-              acc += b;
-              if (p.swiglu) {
-                // as in the unsplit epilogue: a warp's rows are 16 gate rows and their 16 up rows
-                const float up = __shfl_down_sync(0xffffffffu, acc, 16);
-                if ((lane & 16) == 0 && n_in)
-                  C[(size_t)t * p.ldc + (n >> 5) * 16 + (n & 15)] = from_f32<TC>(glu_unit(acc, up, p.glu_limit, p.glu_alpha));
-              } else if (n_in) {
+              float acc = sum[i];
+              if (n_in) {
                 acc += old[i];
                 C[(size_t)t * p.ldc + n] = from_f32<TC>(acc);
                 if (p.emit_x) {
@@ -728,8 +779,7 @@ __global__ void __launch_bounds__(THREADS, PAIR ? 1 : 0)
         unsigned char* row = my_stage + sb * S::PIECE_BYTES + lane * 128;
         if (p.swiglu) {    // columns: 16 gates, then their 16 ups
           float o[16];
-#pragma unroll
-          for (int j = 0; j < 16; ++j) o[j] = glu_unit(v[j], v[j + 16], p.glu_limit, p.glu_alpha);
+          glu_units<TC, 16>(v, [&](int j) { return v[j + 16]; }, p.glu_limit, p.glu_alpha, [&](int j, float h) { o[j] = h; });
           stage_row<TC, 16>(row, lane, part * (16 * (int)sizeof(TC) / 16), o);
         } else {
           if (p.bias) {

@@ -20,13 +20,15 @@ TC_SWAPPED_MIN_ROWS = 17
 
 
 def swapped_splits(n_weight_rows: int, sm_count: int) -> int:
-    """In how many parts K is cut (one per block of a cluster): the fewest that give every SM a block.
-    Measured at 64 rows, microseconds for 1 / 2 / 4 / 8 parts: N = 2048 (16 tiles of 128 weight rows)
-    13 / 9 / 7 / 7, with K = 8192 41 / 23 / 15 / 12; N = 3072 14 / 9 / 7.5 / 8; N = 6144 15 / 11 / 10 / 15;
-    N = 16384 18 / 17 / 21 / 34."""
+    """In how many parts K is cut (one per block of a cluster): the fewest that give 7 of 10 SMs a block.
+    Two blocks fit an SM: up to one per SM, the blocks of the next kernel all find a place and request their first
+    weights while this one runs; a second round of parts takes those places and adds partial sums to exchange.
+    Fewer blocks than that leave too few loads under way.  Whole single-token steps (ms) with parts until 0.6 / 0.7 /
+    1.0 x SMs: LFM2-1.2B with 64 rows 1.21 / 1.16 / 1.19, 32 rows 1.01 / 0.97 / 0.99; the 350M shape with 64 rows
+    0.87 / 0.85 / 0.92, 24 rows 0.62 / 0.60 / 0.65; the 2.6B shape with 24 rows 1.88 / 1.80 / 1.80."""
     tiles = -(-n_weight_rows // 128)
     s = 1
-    while s < 8 and tiles * s < sm_count:
+    while s < 8 and 10 * tiles * s < 7 * sm_count:
         s *= 2
     return s
 
