@@ -847,6 +847,31 @@ def test_tcgen05_prompt_attention_far_key_and_continued_prompt(k, H, Hkv, page):
     assert not torch.allclose(out[far - 1].float().cpu().reshape(H, hd), winner, atol=0.05), "a later key was seen"
 
 
+@pytest.mark.parametrize("H,Hkv", [(2, 2), (4, 2), (8, 2), (8, 1)])
+@pytest.mark.parametrize("T", [63, 64, 129, 330])
+@pytest.mark.parametrize("step", [0.5, 7.0, 9.0, 60.0, -9.0])
+def test_prompt_attention_when_scores_climb_and_fall(k, H, Hkv, T, step):
+    """Scores that climb (or fall) by `step` powers of two per tile of 64 keys, for half of the heads; the others' stay near
+    their first: the reference of the exponents stays, or moves in some rows of a warp, or in all and at every tile."""
+    from zinfer_b200.parts.attention import query_tiles as attn_tiles_host
+    dtype, hd, page = torch.bfloat16, 64, 64
+    scale = 1 / math.sqrt(hd)
+    q, kk, v = rnd((T, H, hd), 1, dtype, 0.3), rnd((T, Hkv, hd), 2, dtype, 0.3), rnd((T, Hkv, hd), 3, dtype)
+    kk[:, :, 0] = (torch.arange(T) * (step * math.log(2) / scale / 64))[:, None].to(dtype)
+    q[:, :, 0] = (torch.arange(H) % 2 == 0).to(dtype)
+    setup = PagedSetup([T], [1], 3, page, Hkv, hd, dtype, seed=5)
+    pages = torch.from_numpy(setup.table[1, :-(-T // page)].astype(np.int64)).cuda()
+    fill = torch.full(((-T) % page, Hkv, hd), float("nan"), dtype=dtype)
+    setup.k[pages] = torch.cat([kk, fill]).reshape(-1, page, Hkv, hd).permute(0, 2, 1, 3).cuda()
+    setup.v[pages] = torch.cat([v, fill]).reshape(-1, page, Hkv, hd).permute(0, 2, 1, 3).cuda()
+    tiles = torch.from_numpy(attn_tiles_host([T], k._fn("attention_prefill_tc5", "zk_attn_prefill_tc5_tile_tokens")(H, Hkv))).cuda()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32).cuda()
+    out = k.attention(q.reshape(T, H * hd).cuda(), setup.k, setup.v, tiles[0].contiguous(), tiles[1].contiguous(), i32([0, T]),
+                      i32([0]), i32([1]), setup.table_dev, H, Hkv, hd, scale, kind="prompt_tc5")
+    assert k.status_word("cuda").item() == 0 and not torch.isnan(out.float()).any()
+    close(out, attn_ref(q.double(), kk.double(), v.double(), 0, 0, scale).reshape(T, H * hd), dtype, "climbing scores")
+
+
 # ------------------------------------------------------------------------------- dependent launches
 
 @pytest.mark.parametrize("rows", [1, 8, 40, 300])

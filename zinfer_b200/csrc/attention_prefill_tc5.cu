@@ -5,32 +5,31 @@
 // GP heads of the group packed beside each other (the reference orders the queries of a KV head the
 // same way, src/model.zig:1352-1366), and walks the keys in tiles of 64 that lie inside one cache
 // page.  Roles:
-//   * warp 8 (one lane) is the producer: one 3-D TMA load brings the 128 x 64 query tile, then per
+//   * warp 4 (one lane) is the producer: one 3-D TMA load brings the 128 x 64 query tile, then per
 //     key tile two 2-D TMA loads bring K and V ([64 keys, 64] each, 128-byte swizzle) into a ring of
 //     four stages, so that the loads run three tiles ahead of the MMAs;
-//   * warp 9 (one lane) issues tcgen05.mma: S = Q K^T (M 128, N 64 keys, four k steps; K is the
+//   * warp 5 (one lane) issues tcgen05.mma: S = Q K^T (M 128, N 64 keys, four k steps; K is the
 //     K-major B operand) into one of two score buffers in tensor memory, and O += P V (N 64 columns,
-//     four k steps over the 64 keys; V as it lies in the cache is the MN-major B operand);
-//   * warps 0..7 are the softmax, two threads per row: threads r and r + 128 own row r of the tile
-//     (a warp reaches the 32 accumulator lanes 32 (w mod 4) .., so warps w and w + 4 share rows),
-//     the first the scores of keys 0..31 of the tile and columns 0..31 of O, the second the other
-//     halves.  Each reads its 32 scores with tcgen05.ld, applies the causal mask, the two exchange
-//     their maxima through shared memory (a named barrier per pair of warps), keep the running
-//     maximum and their halves of the sum of the online softmax (src/attention.zig:478-517, no tile
-//     skipped), rescale their halves of the row of O in tensor memory and write their halves of the
-//     row of P as bfloat16 into the shared-memory tile that is the A operand of P V.  A row's chain
-//     of dependent operations per key tile is half as long as with one thread, which is what bounds
-//     a block (its tiles form one chain softmax -> P V -> Q K^T -> softmax).
-// The scores have two buffers in tensor memory: Q K^T of tile t + 1 is issued before the MMA warp waits
-// for P of tile t, so it runs while the softmax warps work on tile t, and P V of tile t runs while they
-// work on tile t + 1.  One block needs 256 columns of tensor memory (two score buffers and O) and 99 KB
-// of shared memory, so two blocks share an SM.  Measured on a B200 for 32 heads on 8 KV heads: a
-// prompt of 8,192 tokens 832 -> 577 us a layer (476 TFLOP/s), of 2,048 tokens 90 -> 72 us, against the
-// version with one thread per row, one score buffer and two K/V stages.  (Computing a part of the
-// exponentials by polynomial on the FMA pipe, beside ex2.approx, made it slower: the softmax warps are
-// bound by instruction issue, not by the special-function unit.)  Scores stay unscaled in registers; the
+//     four k steps over the 64 keys; P is the A operand and lies in tensor memory, V as it lies in the
+//     cache is the MN-major B operand);
+//   * warps 0..3 are the softmax, a thread per row: it reads its 64 scores with tcgen05.ld, applies the
+//     causal mask, keeps the reference and the sum of the online softmax (src/attention.zig:478-517, no
+//     tile skipped) and writes its row of P as bfloat16 into one of two buffers in tensor memory.  The
+//     exponents refer to a score that moves only when one passes it by 2^8 (P has the same relative
+//     precision at every size, the sums are float32): then, and only then, O is rescaled, and only then does
+//     the softmax wait for P V of the tile before.
+// Q K^T of tile t + 1 is issued before the MMA warp waits for P of tile t, so it runs while the softmax
+// warps work on tile t, and P V of tile t runs while they work on tile t + 1.  One block needs 256
+// columns of tensor memory (two score buffers, O, two of P) and 82 KB of shared memory: two blocks share an SM.
+// What bounds it: the special-function unit (64 x 128 exponentials are 512 cycles of an SM, the MMAs of the
+// tile 256) at 62 % of its rate; the rest is a warp's chain from scores to P with two warps per scheduler.
+// Measured on a B200, microseconds a layer, against two threads per row that exchanged their maxima
+// every tile, P in shared memory and the blocks head after head: 16 heads on 8, 8,192 tokens 317 -> 255 with the
+// blocks as they were, 209 (658 TFLOP/s) with the longest first; 32 heads on 8, 8,192 tokens 638 -> 507 -> 485; 2,048 tokens
+// 62 -> 50 -> 38.  With one score buffer that P replaces (four blocks an SM, the scores read twice for the
+// registers): 618 in place of 507.  Scores stay unscaled in registers; the
 // scale is folded into the exponent (2^((s - m) * scale * log2 e), ex2.approx), tiles below the
-// diagonal skip the mask, and a warp whose rows keep their maximum skips the rescaling of O.
+// diagonal skip the mask.
 //
 // Options (the EXT form of the kernel): a table of numbers per (head, distance) added to the scaled scores, a mask in
 // stretches of positions (a query sees its own stretch only; the walk starts at the tile of the first query's stretch), and a
@@ -57,12 +56,12 @@ using namespace tc5;
 constexpr int HD = 64;            // head size
 constexpr int ROWS = 128;         // query rows per block = accumulator lanes
 constexpr int TK = 64;            // keys per tile
-constexpr int SM_THREADS = 256;   // eight softmax warps: two threads per row
+constexpr int SM_THREADS = ROWS;  // four softmax warps: a thread per row
 constexpr int THREADS = SM_THREADS + 64;   // then the producer warp and the MMA warp
-constexpr int Q_BYTES = ROWS * HD * 2, KV_BYTES = TK * HD * 2, P_BYTES = ROWS * TK * 2;
-constexpr int XCH_BYTES = 2 * 2 * ROWS * 4;   // the halves' maxima, double-buffered (the sums reuse it at the end)
+constexpr int PRODUCER_WARP = SM_THREADS / 32, MMA_WARP = PRODUCER_WARP + 1;
+constexpr int Q_BYTES = ROWS * HD * 2, KV_BYTES = TK * HD * 2;
 constexpr int NSTG = 4;           // K/V tiles in shared memory: the loads run three tiles ahead of the MMAs
-constexpr size_t SMEM_BYTES = Q_BYTES + 2 * NSTG * KV_BYTES + P_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/ + XCH_BYTES;
+constexpr size_t SMEM_BYTES = Q_BYTES + 2 * NSTG * KV_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 // EXT: a stage's slice of the distance table
 constexpr int DIST_FRONT = 192, DIST_BACK = 256;
 __host__ __device__ constexpr int dist_len_of(int gp) { return (ROWS / gp + TK - 1 + 3 + 3) / 4 * 4; }       // floats copied per head
@@ -70,7 +69,10 @@ __host__ __device__ constexpr int dist_ld(int gp) {      // floats between heads
   return gp == 1 ? dist_len_of(1) : gp == 2 ? 144 : gp == 4 ? 104 : 100;
 }
 static_assert(dist_ld(2) >= dist_len_of(2) && dist_ld(4) >= dist_len_of(4) && dist_ld(8) >= dist_len_of(8), "slices fit their rows");
-constexpr unsigned TMEM_COLS = 256;   // two score buffers at columns 0 and 64, O at column 128: two blocks fit an SM
+constexpr unsigned TMEM_COLS = 256;   // two blocks fit an SM
+constexpr unsigned T_S = 0, T_O = 128, T_P = 192;   // score buffers at columns 0 and 64, O, P at 192 and 224
+// A row's exponents refer to a maximum that is moved only when a score passes it by more than this many powers of two.
+constexpr float LAZY = 8.f;
 
 struct Params {
   bf16* out;
@@ -117,6 +119,23 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
   return *reinterpret_cast<const unsigned*>(&t);
 }
 
+// two float32 operations in one instruction; the results are those of the single ones
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\n"
+      "fma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
 template <bool EXT>
 __global__ void __launch_bounds__(THREADS, 2)
     attn_prefill_tc5_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
@@ -127,28 +146,29 @@ __global__ void __launch_bounds__(THREADS, 2)
   unsigned char* kv_sm = base + Q_BYTES;          // stage s: K at kv_sm + 2 s KV_BYTES, V behind it
   auto k_sm = [&](int s) { return kv_sm + 2 * s * KV_BYTES; };
   auto v_sm = [&](int s) { return kv_sm + (2 * s + 1) * KV_BYTES; };
-  unsigned char* p_sm = base + Q_BYTES + 2 * NSTG * KV_BYTES;
-  unsigned long long* bars = reinterpret_cast<unsigned long long*>(p_sm + P_BYTES);
+  unsigned char* bar_sm = base + Q_BYTES + 2 * NSTG * KV_BYTES;
+  unsigned long long* bars = reinterpret_cast<unsigned long long*>(bar_sm);
   unsigned long long* q_full = bars;            // 1
   unsigned long long* kv_full = bars + 1;               // [NSTG]
   unsigned long long* kv_empty = bars + 1 + NSTG;       // [NSTG]
   unsigned long long* s_full = bars + 1 + 2 * NSTG;     // [2]: one per score buffer
   unsigned long long* p_ready = bars + 3 + 2 * NSTG;    // 1, an arrival per softmax thread
-  unsigned long long* pv_done = bars + 4 + 2 * NSTG;    // 1
-  unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 5 + 2 * NSTG);
-  static_assert((5 + 2 * NSTG) * 8 + 16 <= 256, "the barriers fit their 256 bytes");
+  unsigned long long* pv_done = bars + 4 + 2 * NSTG;    // [2]: one per P buffer
+  unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 6 + 2 * NSTG);
+  static_assert((6 + 2 * NSTG) * 8 + 16 <= 256, "the barriers fit their 256 bytes");
   volatile int* aborted = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  volatile float* xch = reinterpret_cast<volatile float*>(p_sm + P_BYTES + 256);   // [2 buffers][2 halves][ROWS]
-  float* dist_sm = reinterpret_cast<float*>(p_sm + P_BYTES + 256 + XCH_BYTES);     // EXT: [NSTG][GP][dist_ld(GP)]
+  float* dist_sm = reinterpret_cast<float*>(bar_sm + 256);     // EXT: [NSTG][GP][dist_ld(GP)]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int GP = p.gp, G = p.H / p.Hkv, chunks = G / GP;
   const int BQ = ROWS / GP;                   // tokens per block
-  const int kvh = blockIdx.y / chunks, chunk = blockIdx.y % chunks;
+  const int packs = p.Hkv * chunks, pack = blockIdx.x % packs, kvh = pack / chunks, chunk = pack % chunks;
   const bool cross = p.part_o != nullptr;
   const int vh = cross ? blockIdx.z : kvh;
-  // tiles are taken from the last (a sequence's late tokens see the most keys) to the first
-  const int tile = gridDim.x - 1 - blockIdx.x;
+  // Tiles are taken from the last (a sequence's late tokens see the most keys) to the first, all heads of a tile before the
+  // next, so that what is left for the end is short.  Head after head, the last head's longest tiles began when 7 of 8 of the
+  // work was done, and SMs were busy for 80 % of the time (16 heads on 8, 8,192 tokens).
+  const int tile = (gridDim.x - 1 - blockIdx.x) / packs;
   const int b = p.tile_seq[tile], q0 = p.tile_q0[tile];
   const int t_base = p.cu_q[b], Tq = p.cu_q[b + 1] - t_base;
   const int start = p.seq_start[b];
@@ -169,23 +189,24 @@ __global__ void __launch_bounds__(THREADS, 2)
     mbar_init(&s_full[0], 1);
     mbar_init(&s_full[1], 1);
     mbar_init(p_ready, SM_THREADS);
-    mbar_init(pv_done, 1);
+    mbar_init(&pv_done[0], 1);
+    mbar_init(&pv_done[1], 1);
     *aborted = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
   }
-  if (warp == 9) tmem_alloc(tmem_slot, TMEM_COLS);
+  if (warp == MMA_WARP) tmem_alloc(tmem_slot, TMEM_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const unsigned tmem_base = *tmem_slot;
-  const unsigned tmem_o = tmem_base + 128;
+  const unsigned tmem_o = tmem_base + T_O;
   // Barriers and tensor memory are set up while the kernel before this one ends; q and the cache
   // are its results.  (The batch's index arrays read above were uploaded before the step began.)
   zk_let_next_start();
   zk_wait_prior();
 
-  if (warp == 8 && lane == 0) {
+  if (warp == PRODUCER_WARP && lane == 0) {
     // ---------------------------------------------------------------- producer
     const int* pt = p.page_table + (size_t)p.seq_slot[b] * p.pt_stride;
     mbar_expect_tx(q_full, Q_BYTES);
@@ -217,7 +238,7 @@ __global__ void __launch_bounds__(THREADS, 2)
       tma_load_2d(k_sm(s), &map_k, 0, row, &kv_full[s]);
       tma_load_2d(v_sm(s), &map_v, 0, row + (vh - kvh) * p.page_size, &kv_full[s]);
     }
-  } else if (warp == 9 && lane == 0) {
+  } else if (warp == MMA_WARP && lane == 0) {
     // ---------------------------------------------------------------- MMA issuer
     const unsigned idesc_s = instr_desc(ROWS, TK);                    // Q [128 x 64] . K^T: both K-major
     const unsigned idesc_o = instr_desc(ROWS, HD) | (1u << 16);       // P [128 x 64 keys] . V: V is MN-major
@@ -233,7 +254,7 @@ __global__ void __launch_bounds__(THREADS, 2)
       const unsigned long long dq = smem_desc(q_sm), dk = smem_desc(k_sm(s));
 #pragma unroll
       for (int k = 0; k < HD / 16; ++k)   // 32 bytes further along the swizzled rows per k step
-        umma_bf16(tmem_base + 64u * (unsigned)sb, dq + (unsigned long long)(2 * k), dk + (unsigned long long)(2 * k),
+        umma_bf16(tmem_base + T_S + 64u * (unsigned)sb, dq + (unsigned long long)(2 * k), dk + (unsigned long long)(2 * k),
                   idesc_s, k > 0 ? 1u : 0u);
       umma_commit(&s_full[sb]);
       return true;
@@ -246,31 +267,28 @@ __global__ void __launch_bounds__(THREADS, 2)
         ok = issue_s(t + 1);
         if (!ok) break;
       }
-      if (!mbar_wait(p_ready, t & 1)) {               // the scores are read, P of tile t is in shared memory, O is rescaled
+      if (!mbar_wait(p_ready, t & 1)) {               // the scores are read, P of tile t is in tensor memory, O is rescaled
         atomicExch(p.status, 16);
         ok = false;
         break;
       }
       tc_fence_after();
-      const unsigned long long dp = smem_desc(p_sm), dv = smem_desc(v_sm(t % NSTG));
+      const unsigned long long dv = smem_desc(v_sm(t % NSTG));
 #pragma unroll
-      for (int k = 0; k < TK / 16; ++k)   // P: 32 bytes along its rows; V: 16 key rows of 128 bytes further
-        umma_bf16(tmem_o, dp + (unsigned long long)(2 * k), dv + (unsigned long long)(128 * k), idesc_o,
-                  (t > 0 || k > 0) ? 1u : 0u);
+      for (int k = 0; k < TK / 16; ++k)   // P: 8 columns (16 keys) further; V: 16 key rows of 128 bytes further
+        umma_bf16_ta(tmem_o, tmem_base + T_P + 32u * (unsigned)(t & 1) + 8u * (unsigned)k, dv + (unsigned long long)(128 * k),
+                     idesc_o, (t > 0 || k > 0) ? 1u : 0u);
       umma_commit(&kv_empty[t % NSTG]);
-      umma_commit(pv_done);
+      umma_commit(&pv_done[t & 1]);
     }
     if (!ok) *aborted = 1;
-  } else if (warp < 8) {
+  } else if (warp < PRODUCER_WARP) {
     // ---------------------------------------------------------------- softmax and epilogue
-    constexpr int HK = TK / 2, HO = HD / 2;         // a thread's keys of a tile, its columns of O
-    const int half = warp >> 2;                     // 0: keys 0..31 of a tile, columns 0..31 of O; 1: the others
-    const int r = threadIdx.x & (ROWS - 1);         // row of the tile = accumulator lane
+    const int r = threadIdx.x;                      // row of the tile = accumulator lane
     const int tq = r / GP, hl = r % GP;
     const bool row_ok = q0 + tq < Tq;
     const int row_hi = start + q0 + tq + 1;          // this row sees keys [0, row_hi)
-    const unsigned lane_sel = (unsigned)((warp & 3) * 32) << 16;
-    const int pair_bar = 1 + (warp & 3);             // named barrier of the two warps that share these rows
+    const unsigned lane_sel = (unsigned)(warp * 32) << 16;
     // scores are kept raw; the scale goes into the exponent: p = 2^((s - m) * scale * log2(e))
     // (with a distance table the scores are scaled as they are read, and only log2(e) is left)
     const float c2 = (EXT && p.dist ? 1.0f : p.scale) * 1.4426950408889634f;
@@ -278,11 +296,21 @@ __global__ void __launch_bounds__(THREADS, 2)
     // EXT: this row sees keys from row_lo on, every row of the tile keys from lo_last on
     const int row_lo = EXT && p.mask_chunk > 0 ? (row_hi - 1) / p.mask_chunk * p.mask_chunk : 0;
     const int lo_last = EXT && p.mask_chunk > 0 ? (k_end - 1) / p.mask_chunk * p.mask_chunk : 0;
-    const float* row_dist = dist_sm + hl * dist_ld(GP) + tq + TK - 1 - half * HK;    // [-j]: key j of the thread's half of a tile
-    float m_run = -INFINITY, l_run = 0.f;            // l_run: the sum over this thread's keys only
+    const float* row_dist = dist_sm + hl * dist_ld(GP) + tq + TK - 1;    // [-j]: key j of a tile
+    float m_ref = -INFINITY, l_run = 0.f;            // the score the exponents refer to; the sum of the exponentials
     bool ok = true;
+    // P V of tile t (0 or later) has finished
+    auto pv_wait = [&](int t) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[t & 1], (t >> 1) & 1));
+      if (!ok) {
+        atomicExch(p.status, 18);
+        *aborted = 1;
+      }
+      tc_fence_after();
+      return ok;
+    };
     for (int t = 0; t < n_tiles; ++t) {
-      const int s = t & 1, kb = k_begin + t * TK + half * HK;
+      const int s = t & 1, kb = k_begin + t * TK;
       // (a warp decides as one: the tensor-memory loads and stores below are warp-collective)
       // the scores are there, so the tile has landed; its own barrier makes the slice that came with it visible to this thread
       ok = __all_sync(0xffffffffu, mbar_wait(&s_full[s], (t >> 1) & 1) &&
@@ -293,110 +321,93 @@ __global__ void __launch_bounds__(THREADS, 2)
         break;
       }
       tc_fence_after();
-      float sc[HK];
-#pragma unroll
-      for (int c0 = 0; c0 < HK; c0 += 16) tmem_ld16(tmem_base + 64u * (unsigned)s + lane_sel + (unsigned)(half * HK + c0), sc + c0);
+      float sc[TK];
+      tmem_ld64(tmem_base + T_S + 64u * (unsigned)s + lane_sel, sc);
       if (EXT) {
         if (p.dist) {
-          const float* d = row_dist + (t % NSTG) * GP * dist_ld(GP) + (dist_at(k_begin + t * TK) & 3);
+          const float* d = row_dist + (t % NSTG) * GP * dist_ld(GP) + (dist_at(kb) & 3);
 #pragma unroll
-          for (int j = 0; j < HK; ++j) sc[j] = fmaf(sc[j], p.scale, d[-j]);
+          for (int j = 0; j < TK; ++j) sc[j] = fmaf(sc[j], p.scale, d[-j]);
         }
         if (kb < lo_last) {
 #pragma unroll
-          for (int j = 0; j < HK; ++j) sc[j] = kb + j >= row_lo ? sc[j] : -INFINITY;
+          for (int j = 0; j < TK; ++j) sc[j] = kb + j >= row_lo ? sc[j] : -INFINITY;
         }
       }
-      if (kb + HK > all_visible || !row_ok) {          // a tile on the diagonal (or a row that does not exist): mask
+      if (kb + TK > all_visible || !row_ok) {          // a tile on the diagonal (or a row that does not exist): mask
+        const int lim = row_ok ? row_hi - kb : 0;      // keys of the tile that this row sees
 #pragma unroll
-        for (int j = 0; j < HK; ++j) sc[j] = (row_ok && kb + j < row_hi) ? sc[j] : -INFINITY;
+        for (int j = 0; j < TK; ++j) sc[j] = j < lim ? sc[j] : -INFINITY;
       }
-      float m_mine = -INFINITY;
+      float m4[4] = {sc[0], sc[1], sc[2], sc[3]};
 #pragma unroll
-      for (int j = 0; j < HK; ++j) m_mine = fmaxf(m_mine, sc[j]);
-      // the row's maximum over both halves
-      // (the two warps of a row leave this loop only where a bounded wait on a barrier they both wait for
-      // ran out, so neither can be left alone at the named barrier below)
-      volatile float* xm = xch + (t & 1) * 2 * ROWS;   // the buffers alternate: a value is read before it is replaced
-      xm[half * ROWS + r] = m_mine;
-      asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
-      const float m_other = xm[(half ^ 1) * ROWS + r];
-      const float m_new = fmaxf(m_run, fmaxf(m_mine, m_other));
-      const float mc = m_new == -INFINITY ? 0.f : m_new * c2;
-      const float alpha = ex2((m_run == -INFINITY ? -INFINITY : m_run * c2) - mc);
-      float row_sum = 0.f;
-      unsigned pk[HK / 2];
+      for (int j = 4; j < TK; j += 8)
 #pragma unroll
-      for (int j = 0; j < HK; j += 2) {
-        const float p0 = ex2(fmaf(sc[j], c2, -mc)), p1 = ex2(fmaf(sc[j + 1], c2, -mc));
-        row_sum += p0 + p1;
-        pk[j / 2] = pack_bf16(p0, p1);
-      }
-      l_run = l_run * alpha + row_sum;
-      const bool rescale = m_new != m_run;
-      m_run = m_new;
-      if (t > 0) {
-        // P V of the previous tile has finished: its P tile may be overwritten and O may be rescaled
-        ok = __all_sync(0xffffffffu, mbar_wait(pv_done, (t - 1) & 1));
-        if (!ok) {
-          atomicExch(p.status, 18);
-          *aborted = 1;
-          break;
-        }
-        tc_fence_after();
-        if (__any_sync(0xffffffffu, rescale)) {        // no row of the warp has a new maximum: O stays
+        for (int e = 0; e < 4; ++e) m4[e] = j + 4 + e < TK ? fmaxf(fmaxf(m4[e], sc[j + e]), sc[j + 4 + e]) : fmaxf(m4[e], sc[j + e]);
+      const float m_tile = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
+      // The first visible score sets the reference, a score far above it moves it; P and O are relative to the reference and
+      // P's 8 significant bits are the same at every size, so a smaller step would only rescale O more often.
+      const bool move = (m_tile - m_ref) * c2 > LAZY;   // (-inf - -inf: NaN, no)
+      if (__any_sync(0xffffffffu, move)) {
+        const float alpha = move ? ex2((m_ref - m_tile) * c2) : 1.0f;
+        if (move) m_ref = m_tile;
+        l_run *= alpha;
+        if (t > 0) {
+          if (!pv_wait(t - 1)) break;
 #pragma unroll
-          for (int c0 = 0; c0 < HO; c0 += 16) {
+          for (int c0 = 0; c0 < HD; c0 += 16) {
             float o[16];
-            tmem_ld16(tmem_o + lane_sel + (unsigned)(half * HO + c0), o);
+            tmem_ld16(tmem_o + lane_sel + (unsigned)c0, o);
 #pragma unroll
             for (int j = 0; j < 16; ++j) o[j] *= alpha;
-            tmem_st16(tmem_o + lane_sel + (unsigned)(half * HO + c0), o);
+            tmem_st16(tmem_o + lane_sel + (unsigned)c0, o);
           }
         }
       }
-      // this thread's half of the row of P: 4 chunks of 8 keys, chunk c at the swizzled place (c ^ (r & 7))
+      const float mc = m_ref == -INFINITY ? 0.f : m_ref * c2;
+      const float2 c22 = make_float2(c2, c2), mc2 = make_float2(-mc, -mc);
+      float2 sum0 = make_float2(0.f, 0.f), sum1 = sum0;
+      unsigned pk[TK / 2];
 #pragma unroll
-      for (int c = 0; c < HK / 8; ++c)
-        *reinterpret_cast<uint4*>(p_sm + r * 128 + (((half * (HK / 8) + c) ^ (r & 7)) * 16)) =
-            make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+      for (int j = 0; j < TK; j += 4) {
+        float2 a = fma2(make_float2(sc[j], sc[j + 1]), c22, mc2), b = fma2(make_float2(sc[j + 2], sc[j + 3]), c22, mc2);
+        a.x = ex2(a.x);
+        a.y = ex2(a.y);
+        b.x = ex2(b.x);
+        b.y = ex2(b.y);
+        sum0 = add2(sum0, a);
+        sum1 = add2(sum1, b);
+        pk[j / 2] = pack_bf16(a.x, a.y);
+        pk[j / 2 + 1] = pack_bf16(b.x, b.y);
+      }
+      l_run += (sum0.x + sum0.y) + (sum1.x + sum1.y);
+      if (t > 1 && !pv_wait(t - 2)) break;             // its P buffer may be overwritten
+      tmem_st32(tmem_base + T_P + 32u * (unsigned)s + lane_sel, pk);
       // rows of V beyond the last key of the sequence's step hold stale cache contents
-      if (k_begin + t * TK + TK > k_end) {
-        const int first = k_end - (k_begin + t * TK);   // 1 .. 63
+      if (kb + TK > k_end) {
+        const int first = k_end - kb;   // 1 .. 63
         for (int i = threadIdx.x; i < (TK - first) * 8; i += SM_THREADS)
           *reinterpret_cast<uint4*>(v_sm(t % NSTG) + (first + i / 8) * 128 + (i % 8) * 16) = make_uint4(0, 0, 0, 0);
+        fence_async_smem();
       }
-      fence_async_smem();
       tc_fence_before();
       mbar_arrive(p_ready);
     }
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(pv_done, (n_tiles - 1) & 1));
-    if (!ok) {
-      atomicExch(p.status, 18);
-      *aborted = 1;
-    }
-    tc_fence_after();
-    if (ok) {   // uniform in the warp: every lane reads its half of its row of O, the rows that exist store it
-      // the row's sum is the two halves' sums (both ran with the same maxima)
-      volatile float* xs = xch + (n_tiles & 1) * 2 * ROWS;
-      xs[half * ROWS + r] = l_run;
-      asm volatile("bar.sync %0, 64;" ::"r"(pair_bar) : "memory");
-      const float l_other = xs[(half ^ 1) * ROWS + r];
-      const float l_row = half == 0 ? l_run + l_other : l_other + l_run;   // first half + second half, in both threads
-      float inv = l_row > 0.f ? 1.0f / l_row : 0.f;
+    if (ok) pv_wait(n_tiles - 1);
+    if (ok) {   // uniform in the warp: every lane reads its row of O, the rows that exist store it
+      float inv = l_run > 0.f ? 1.0f / l_run : 0.f;
       if (EXT && p.gate)
         inv /= 1.0f + expf(-to_f32(p.gate[(size_t)(t_base + min(q0 + tq, Tq - 1)) * p.ld_gate + kvh * G + chunk * GP + hl]));
-      bf16* dst = p.out + (size_t)(t_base + min(q0 + tq, Tq - 1)) * p.H * HD + (size_t)(kvh * G + chunk * GP + hl) * HD +
-                  half * HO;
+      bf16* dst = p.out + (size_t)(t_base + min(q0 + tq, Tq - 1)) * p.H * HD + (size_t)(kvh * G + chunk * GP + hl) * HD;
       const size_t xrow = ((size_t)(t_base + min(q0 + tq, Tq - 1)) * p.H + (kvh * G + chunk * GP + hl)) * p.Hkv + vh;
-      if (cross && row_ok && half == 0) *reinterpret_cast<float2*>(p.part_ml + xrow * 2) = make_float2(0.f, 1.f);
+      if (cross && row_ok) *reinterpret_cast<float2*>(p.part_ml + xrow * 2) = make_float2(0.f, 1.f);
 #pragma unroll
-      for (int c0 = 0; c0 < HO; c0 += 16) {
+      for (int c0 = 0; c0 < HD; c0 += 16) {
         float o[16];
-        tmem_ld16(tmem_o + lane_sel + (unsigned)(half * HO + c0), o);
+        tmem_ld16(tmem_o + lane_sel + (unsigned)c0, o);
         if (cross) {
           if (row_ok) {
-            float* xdst = p.part_o + xrow * HD + half * HO + c0;
+            float* xdst = p.part_o + xrow * HD + c0;
 #pragma unroll
             for (int i = 0; i < 16; i += 4)
               *reinterpret_cast<float4*>(xdst + i) = make_float4(o[i] * inv, o[i + 1] * inv, o[i + 2] * inv, o[i + 3] * inv);
@@ -418,7 +429,7 @@ __global__ void __launch_bounds__(THREADS, 2)
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 9) tmem_dealloc(tmem_base, TMEM_COLS);
+  if (warp == MMA_WARP) tmem_dealloc(tmem_base, TMEM_COLS);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -507,7 +518,8 @@ int zk_attn_prefill_tc5(const void* q, const void* k_cache, const void* v_cache,
   const size_t smem = SMEM_BYTES + (dist ? (size_t)NSTG * gp * dist_ld(gp) * sizeof(float) : 0);
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  dim3 grid(n_tiles, Hkv * (G / gp), part_o ? Hkv : 1);
+  if ((long long)n_tiles * Hkv * (G / gp) > 0x7fffffffLL) return ZK_EINVAL;
+  dim3 grid(n_tiles * Hkv * (G / gp), 1, part_o ? Hkv : 1);
   return zk_launch_dependent(kern, grid, dim3(THREADS), smem, stream, mq, mk, mv, p);
 }
 
