@@ -852,7 +852,7 @@ def test_tcgen05_prompt_attention_far_key_and_continued_prompt(k, H, Hkv, page):
 @pytest.mark.parametrize("step", [0.5, 7.0, 9.0, 60.0, -9.0])
 def test_prompt_attention_when_scores_climb_and_fall(k, H, Hkv, T, step):
     """Scores that climb (or fall) by `step` powers of two per tile of 64 keys, for half of the heads; the others' stay near
-    their first: the reference of the exponents stays, or moves in some rows of a warp, or in all and at every tile."""
+    their first: the running maximum stays, or moves in some rows of a warp, or in all and at every tile."""
     from zinfer_b200.parts.attention import query_tiles as attn_tiles_host
     dtype, hd, page = torch.bfloat16, 64, 64
     scale = 1 / math.sqrt(hd)

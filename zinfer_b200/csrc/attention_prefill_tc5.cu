@@ -13,21 +13,22 @@
 //     four k steps over the 64 keys; P is the A operand and lies in tensor memory, V as it lies in the
 //     cache is the MN-major B operand);
 //   * warps 0..3 are the softmax, a thread per row: it reads its 64 scores with tcgen05.ld, applies the
-//     causal mask, keeps the reference and the sum of the online softmax (src/attention.zig:478-517, no
-//     tile skipped) and writes its row of P as bfloat16 into one of two buffers in tensor memory.  The
-//     exponents refer to a score that moves only when one passes it by 2^8 (P has the same relative
-//     precision at every size, the sums are float32): then, and only then, O is rescaled, and only then does
-//     the softmax wait for P V of the tile before.
+//     causal mask, keeps the running maximum and the sum of the online softmax (src/attention.zig:478-517, no
+//     tile skipped) and writes its row of P as bfloat16 into one of two buffers in tensor memory.  Only where
+//     a maximum moved does a warp wait for P V of the tile before and rescale O, and it does so behind the
+//     exponentials.  (A reference that stays until a score passes it by 2^8 is faster still, 209 us where this
+//     takes 230, but then the largest P is no longer 1 and is rounded: errors against 64 bits 1.77e-3 -> 2.16e-3
+//     with scores of a wide spread.)
 // Q K^T of tile t + 1 is issued before the MMA warp waits for P of tile t, so it runs while the softmax
 // warps work on tile t, and P V of tile t runs while they work on tile t + 1.  One block needs 256
 // columns of tensor memory (two score buffers, O, two of P) and 82 KB of shared memory: two blocks share an SM.
 // What bounds it: the special-function unit (64 x 128 exponentials are 512 cycles of an SM, the MMAs of the
 // tile 256) at 62 % of its rate; the rest is a warp's chain from scores to P with two warps per scheduler.
 // Measured on a B200, microseconds a layer, against two threads per row that exchanged their maxima
-// every tile, P in shared memory and the blocks head after head: 16 heads on 8, 8,192 tokens 317 -> 255 with the
-// blocks as they were, 209 (658 TFLOP/s) with the longest first; 32 heads on 8, 8,192 tokens 638 -> 507 -> 485; 2,048 tokens
-// 62 -> 50 -> 38.  With one score buffer that P replaces (four blocks an SM, the scores read twice for the
-// registers): 618 in place of 507.  Scores stay unscaled in registers; the
+// every tile, P in shared memory and the blocks head after head: 16 heads on 8, 8,192 tokens 317 -> 230 (598 TFLOP/s;
+// 261 with O rescaled before the exponentials); 32 heads on 8, 8,192 tokens 638 -> 520; 2,048 tokens 62 -> 43.  With one score
+// buffer that P replaces (four blocks an SM, the scores read twice for the registers) it took a fifth longer.  Scores stay
+// unscaled in registers; the
 // scale is folded into the exponent (2^((s - m) * scale * log2 e), ex2.approx), tiles below the
 // diagonal skip the mask.
 //
@@ -71,8 +72,6 @@ __host__ __device__ constexpr int dist_ld(int gp) {      // floats between heads
 static_assert(dist_ld(2) >= dist_len_of(2) && dist_ld(4) >= dist_len_of(4) && dist_ld(8) >= dist_len_of(8), "slices fit their rows");
 constexpr unsigned TMEM_COLS = 256;   // two blocks fit an SM
 constexpr unsigned T_S = 0, T_O = 128, T_P = 192;   // score buffers at columns 0 and 64, O, P at 192 and 224
-// A row's exponents refer to a maximum that is moved only when a score passes it by more than this many powers of two.
-constexpr float LAZY = 8.f;
 
 struct Params {
   bf16* out;
@@ -297,7 +296,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     const int row_lo = EXT && p.mask_chunk > 0 ? (row_hi - 1) / p.mask_chunk * p.mask_chunk : 0;
     const int lo_last = EXT && p.mask_chunk > 0 ? (k_end - 1) / p.mask_chunk * p.mask_chunk : 0;
     const float* row_dist = dist_sm + hl * dist_ld(GP) + tq + TK - 1;    // [-j]: key j of a tile
-    float m_ref = -INFINITY, l_run = 0.f;            // the score the exponents refer to; the sum of the exponentials
+    float m_run = -INFINITY, l_run = 0.f;            // the running maximum; the sum of the exponentials
     bool ok = true;
     // P V of tile t (0 or later) has finished
     auto pv_wait = [&](int t) {
@@ -345,26 +344,11 @@ __global__ void __launch_bounds__(THREADS, 2)
 #pragma unroll
         for (int e = 0; e < 4; ++e) m4[e] = j + 4 + e < TK ? fmaxf(fmaxf(m4[e], sc[j + e]), sc[j + 4 + e]) : fmaxf(m4[e], sc[j + e]);
       const float m_tile = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-      // The first visible score sets the reference, a score far above it moves it; P and O are relative to the reference and
-      // P's 8 significant bits are the same at every size, so a smaller step would only rescale O more often.
-      const bool move = (m_tile - m_ref) * c2 > LAZY;   // (-inf - -inf: NaN, no)
-      if (__any_sync(0xffffffffu, move)) {
-        const float alpha = move ? ex2((m_ref - m_tile) * c2) : 1.0f;
-        if (move) m_ref = m_tile;
-        l_run *= alpha;
-        if (t > 0) {
-          if (!pv_wait(t - 1)) break;
-#pragma unroll
-          for (int c0 = 0; c0 < HD; c0 += 16) {
-            float o[16];
-            tmem_ld16(tmem_o + lane_sel + (unsigned)c0, o);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) o[j] *= alpha;
-            tmem_st16(tmem_o + lane_sel + (unsigned)c0, o);
-          }
-        }
-      }
-      const float mc = m_ref == -INFINITY ? 0.f : m_ref * c2;
+      const bool move = m_tile > m_run;
+      const float alpha = move ? ex2((m_run - m_tile) * c2) : 1.0f;
+      if (move) m_run = m_tile;
+      l_run *= alpha;
+      const float mc = m_run == -INFINITY ? 0.f : m_run * c2;
       const float2 c22 = make_float2(c2, c2), mc2 = make_float2(-mc, -mc);
       float2 sum0 = make_float2(0.f, 0.f), sum1 = sum0;
       unsigned pk[TK / 2];
@@ -381,7 +365,20 @@ __global__ void __launch_bounds__(THREADS, 2)
         pk[j / 2 + 1] = pack_bf16(b.x, b.y);
       }
       l_run += (sum0.x + sum0.y) + (sum1.x + sum1.y);
-      if (t > 1 && !pv_wait(t - 2)) break;             // its P buffer may be overwritten
+      if (t > 0 && __any_sync(0xffffffffu, move)) {    // O follows the new maximum once P V of the tile before is complete
+        if (!pv_wait(t - 1)) break;
+#pragma unroll
+        for (int c0 = 0; c0 < HD; c0 += 32) {
+          float o[32];
+          tmem_ld32(tmem_o + lane_sel + (unsigned)c0, o);
+          unsigned w[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) w[j] = __float_as_uint(o[j] * alpha);
+          tmem_st32(tmem_o + lane_sel + (unsigned)c0, w);
+        }
+      } else if (t > 1) {                              // its P buffer may be overwritten
+        if (!pv_wait(t - 2)) break;
+      }
       tmem_st32(tmem_base + T_P + 32u * (unsigned)s + lane_sel, pk);
       // rows of V beyond the last key of the sequence's step hold stale cache contents
       if (kb + TK > k_end) {
