@@ -39,6 +39,22 @@ def test_argmax_first_maximum_wins_and_nan_never_does(k):
     assert k.argmax(torch.from_numpy(big).cuda()).cpu().tolist() == np.argmax(big, axis=1).tolist()
 
 
+@pytest.mark.parametrize("V", [4095, 4096, 16384, 16388, 16400, 65536, 65541, 131072])
+def test_argmax_in_vectors_and_remainders(k, V):
+    """Pieces that are whole vectors, have a remainder, or do not begin on 16 bytes; ties within a vector, between threads, warps
+    and pieces, zeros of both signs, a row of -inf, one of NaN and -inf."""
+    x = logits_rows(9, V, V)
+    for row, at in enumerate([[V - 1], [0], [V // 2, V // 2 + 1], [5, 6, V - 1], [1027, 40, V // 3], [V - 2, V // 16]]):
+        x[row, at] = 99.0
+    x[6] = -1.0
+    x[6, [V - 3, V // 2, 77]] = [0.0, -0.0, -0.0]
+    x[7] = -np.inf
+    x[8] = -np.inf
+    x[8, :9] = np.nan
+    got = k.argmax(torch.from_numpy(x).cuda()).cpu().tolist()
+    assert got[:8] == np.argmax(x[:8], axis=1).tolist() and got[8] == 0
+
+
 @pytest.mark.parametrize("V", [331, 5000, 65536])
 @pytest.mark.parametrize("opts", [dict(temp=1.0), dict(temp=0.8, top_k=40, top_p=0.95, min_p=0.05),
                                   dict(temp=0.5, top_k=7), dict(temp=1.3, top_p=0.5), dict(temp=1.0, min_p=0.3),

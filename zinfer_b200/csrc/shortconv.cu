@@ -139,6 +139,14 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
   for (int r = 0; r < RUN; ++r)
     craw[r] = *reinterpret_cast<const uint4*>(bcx + (size_t)min(t0 + r, n_tokens - 1) * 3 * D + cc);
+  // Each token's sequence and place in its sequence's part of this step, looked up beside the loads above.  Looked up token by
+  // token further down, they were a chain of loads behind them: 8,192 tokens of 2,048 channels 52.9 -> 46 us, of 1,024
+  // channels 20.7 -> 18.0.
+  int seq[RUN], place[RUN];
+#pragma unroll
+  for (int r = 0; r < RUN; ++r) seq[r] = tok_seq[min(t0 + r, n_tokens - 1)];
+#pragma unroll
+  for (int r = 0; r < RUN; ++r) place[r] = t0 + r - cu_q[seq[r]];
   float wk[K][8];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
@@ -163,8 +171,7 @@ __global__ void __launch_bounds__(128)
   for (int r = 0; r < RUN; ++r) {
     const int t = t0 + r;
     if (t >= n_tokens) break;
-    const int b = tok_seq[t];
-    const int i = t - cu_q[b];            // the token's place in its sequence's part of this step
+    const int b = seq[r], i = place[r];
     float acc[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) acc[e] = 0.f;
