@@ -345,10 +345,13 @@ __global__ void __launch_bounds__(THREADS, 2)
         for (int e = 0; e < 4; ++e) m4[e] = j + 4 + e < TK ? fmaxf(fmaxf(m4[e], sc[j + e]), sc[j + 4 + e]) : fmaxf(m4[e], sc[j + e]);
       const float m_tile = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
       const bool move = m_tile > m_run;
-      const float alpha = move ? ex2((m_run - m_tile) * c2) : 1.0f;
+      // both maxima scaled and rounded as the exponents below have them, so that what was summed relative to the old one is
+      // brought to the new one exactly, however large the scores are
+      const float mc_old = m_run == -INFINITY ? -INFINITY : m_run * c2;
       if (move) m_run = m_tile;
-      l_run *= alpha;
       const float mc = m_run == -INFINITY ? 0.f : m_run * c2;
+      const float alpha = move ? ex2(mc_old - mc) : 1.0f;
+      l_run *= alpha;
       const float2 c22 = make_float2(c2, c2), mc2 = make_float2(-mc, -mc);
       float2 sum0 = make_float2(0.f, 0.f), sum1 = sum0;
       unsigned pk[TK / 2];
