@@ -219,11 +219,12 @@ def sm_count(device=None) -> int:
 # object each time (some 5 us, a fifth of the host's time per launch of an unrecorded step); the
 # raw getter behind it returns the handle itself.  Where a torch build lacks it the public call does.
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_raw_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream() -> int:
     if _raw_stream is not None:
-        return _raw_stream(torch.cuda.current_device())
+        return _raw_stream(_raw_device())
     return torch.cuda.current_stream().cuda_stream
 
 
@@ -234,13 +235,12 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 def _need(t: torch.Tensor, name: str, dtype=None, shape=None, contiguous=True) -> None:
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise KernelError(f"{name}: expected a CUDA tensor")
-    if dtype is not None:
-        ok = t.dtype in dtype if isinstance(dtype, (tuple, list)) else t.dtype == dtype
-        if not ok:
+    if dtype is not None and t.dtype is not dtype:
+        if not isinstance(dtype, (tuple, list)) or t.dtype not in dtype:
             raise KernelError(f"{name}: dtype {t.dtype}, expected {dtype}")
     if contiguous and not t.is_contiguous():
         raise KernelError(f"{name}: must be contiguous")
-    if shape is not None:
+    if shape is not None and t.shape != shape:      # sizes given as None are free
         if t.dim() != len(shape) or any(s is not None and s != d for s, d in zip(shape, t.shape)):
             raise KernelError(f"{name}: shape {tuple(t.shape)}, expected {tuple(shape)}")
 
@@ -1130,19 +1130,26 @@ def _skinny_input(a):
 def gemm_skinny_takes(a, w: torch.Tensor) -> bool:
     """Whether the skinny kernels take this contraction: bfloat16 weights, few rows, 16-byte
     aligned rows.  `a` is a bfloat16 tensor [M <= 64, K], a NormInput or a ScaledInput [M <= 16, K]."""
-    if not (w.dtype == torch.bfloat16 and w.dim() == 2 and w.stride(1) == 1 and w.stride(0) % 8 == 0
-            and w.data_ptr() % 16 == 0 and w.shape[1] % 8 == 0):
+    if w.dtype is not torch.bfloat16 or w.dim() != 2:
+        return False
+    K = w.shape[1]
+    ldw, step = w.stride()
+    if step != 1 or ldw % 8 or K % 8 or w.data_ptr() % 16:
         return False
     if isinstance(a, NormInput):
         x = a.x
-        return (x.shape[0] <= gemm_skinny_fused_max_m() and x.shape[1] == w.shape[1] and x.stride(1) == 1
-                and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0 and a.weight.data_ptr() % 16 == 0)
+        ldx, step = x.stride()
+        return (x.shape[0] <= gemm_skinny_fused_max_m() and x.shape[1] == K and step == 1
+                and ldx % 4 == 0 and x.data_ptr() % 16 == 0 and a.weight.data_ptr() % 16 == 0)
     if isinstance(a, ScaledInput):
         if a.xw.shape[0] > gemm_skinny_fused_max_m() or not a.ssq.is_contiguous():
             return False
         a = a.xw
-    return (a.dtype == torch.bfloat16 and a.dim() == 2 and a.shape[0] <= gemm_skinny_max_m()
-            and a.shape[1] == w.shape[1] and a.stride(1) == 1 and a.stride(0) % 8 == 0 and a.data_ptr() % 16 == 0)
+    if a.dtype is not torch.bfloat16 or a.dim() != 2:
+        return False
+    lda, step = a.stride()
+    return (a.shape[0] <= gemm_skinny_max_m() and a.shape[1] == K and step == 1 and lda % 8 == 0
+            and a.data_ptr() % 16 == 0)
 
 
 def gemm_skinny_fused_takes(a, w: torch.Tensor) -> bool:
@@ -1159,14 +1166,15 @@ def gemm_skinny_emits(a, out: Optional[torch.Tensor]) -> bool:
 def gemm_skinny(a, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_dtype=None,
                 accumulate: bool = False, bias: Optional[torch.Tensor] = None,
                 emit: Optional[NormEmit] = None, col_scale: Optional[torch.Tensor] = None,
-                act: Optional[str] = None) -> torch.Tensor:
+                act: Optional[str] = None, taken: bool = False) -> torch.Tensor:
     """out (+)= a @ w.T (+ bias) for a [M <= 64, K] on the tensor cores, every weight read once.
+    `taken`: the caller has just asked `gemm_skinny_takes` and need not pay for it twice.
     `act` ("relu_squared") is applied to the sums, then `col_scale` (float32 [N], one number per column)
     multiplies them, before they are stored or added to `out`.
     With a NormInput the RMSNorm of the rows is applied inside the kernel; with a ScaledInput the
     sums are scaled by the rows' 1/rms.  `emit` (see `gemm_skinny_emits`) is filled for the norm
     that reads `out` next."""
-    if not gemm_skinny_takes(a, w):
+    if not taken and not gemm_skinny_takes(a, w):
         raise KernelError(f"gemm_skinny: a {tuple(a.shape)} / w {tuple(w.shape)} need few rows, "
                           "K a multiple of 8 and 16-byte aligned rows")
     X, Xf, nw, eps, M, K, ldx, ssq, ssq_parts = _skinny_input(a)
@@ -1200,12 +1208,12 @@ def gemm_skinny(a, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_dtyp
     return out
 
 
-def gemm_skinny_swiglu(a, w_gate_up: torch.Tensor, act: str = "silu") -> torch.Tensor:
+def gemm_skinny_swiglu(a, w_gate_up: torch.Tensor, act: str = "silu", taken: bool = False) -> torch.Tensor:
     """h = act(a W_gate^T) * (a W_up^T) (act one of GATED_EPILOGUES) in one kernel; w_gate_up [2F, K] holds groups of 16 gate
-    rows followed by their 16 up rows."""
+    rows followed by their 16 up rows.  `taken`: the caller has just asked `gemm_skinny_fused_takes`."""
     if act not in GATED_EPILOGUES:
         raise KernelError(f"gemm_skinny_swiglu: no gated epilogue with the activation {act!r}")
-    if not gemm_skinny_fused_takes(a, w_gate_up) or w_gate_up.shape[0] % 32:
+    if not (taken or gemm_skinny_fused_takes(a, w_gate_up)) or w_gate_up.shape[0] % 32:
         raise KernelError("gemm_skinny_swiglu: at most 16 rows, K a multiple of 8, 16-byte aligned rows")
     X, Xf, nw, eps, M, K, ldx, ssq, ssq_parts = _skinny_input(a)
     F = w_gate_up.shape[0] // 2

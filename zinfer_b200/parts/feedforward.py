@@ -9,7 +9,8 @@ import torch
 from .. import kernels
 from .base import FEED_FORWARDS, FeedForward, WeightSpec
 from .linear import FUSION_GROUP, as_tensor, fused_input, interleave_rows, linear, scaled_or_tensor
-from .linear_bf16 import TC_SWAPPED_MIN_ROWS, swapped_splits
+from . import linear_bf16
+from .linear_bf16 import swapped_splits
 
 
 class SwiGLU(FeedForward):
@@ -39,12 +40,11 @@ class SwiGLU(FeedForward):
     def forward(self, ctx, xn, out, accumulate):
         w, h = self.w_gate_up, None
         if self.interleave and w.dtype == torch.bfloat16:
-            from . import linear_bf16
             rows_in = xn.shape[0]
             tc_rows = linear_bf16.TC_SWAPPED_MIN_ROWS <= rows_in <= kernels.gemm_skinny_max_m()
             x = None if tc_rows or self.clamp else fused_input(xn, w, need_fused_rows=True, blocks=self.ffn_dim // 16)
             if x is not None:                       # few rows: gate, up and the activation in one kernel
-                h = kernels.gemm_skinny_swiglu(x, w, act=self.gate_act)
+                h = kernels.gemm_skinny_swiglu(x, w, act=self.gate_act, taken=True)
             else:
                 x = scaled_or_tensor(xn) if tc_rows else as_tensor(xn)
                 if not kernels.gemm_tc_takes(x, w):

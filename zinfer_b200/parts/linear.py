@@ -21,6 +21,7 @@ from typing import Optional, Union
 import torch
 
 from .. import kernels
+from . import linear_bf16
 
 
 class NormedRows:
@@ -152,7 +153,6 @@ def linear(a: Union[torch.Tensor, NormedRows], w: torch.Tensor,
     if isinstance(out, ResidualSink):
         sink, out = out, out.rows
     if w.dtype == torch.bfloat16:
-        from . import linear_bf16
         y = linear_bf16.try_linear(a, w, out, out_dtype, accumulate, bias, sink)
         if y is not None:
             return y
@@ -174,7 +174,7 @@ def _linear_with_epilogue(a, w, out, out_dtype, accumulate, bias, act):
         x = fused_input(a, w)
         if x is not None:                # few rows: activation and scale in the weight-streaming kernel's epilogue
             return kernels.gemm_skinny(x, w, out=out, out_dtype=out_dtype, accumulate=accumulate, bias=bias,
-                                       col_scale=scale, act=act)
+                                       col_scale=scale, act=act, taken=True)
     if w.dtype == torch.bfloat16 and (act is None or act == "relu_squared") and a.shape[0] > kernels.GEMM_TC_SWAPPED_MAX_M:
         t = as_tensor(a)
         if kernels.gemm_tc_fuses(t, w, out, accumulate, out_dtype):   # many rows: the persistent tcgen05 forms' epilogue

@@ -6,6 +6,8 @@ pending RMSNorm itself.  More rows (prompt steps): the TMA-fed tcgen05 kernel wi
 accumulator in tensor memory."""
 from __future__ import annotations
 
+import sys
+
 from .. import kernels
 
 
@@ -34,8 +36,8 @@ def swapped_splits(n_weight_rows: int, sm_count: int) -> int:
 
 
 def try_linear(a, w, out, out_dtype, accumulate, bias, sink=None):
-    from .linear import as_tensor, fused_input, scaled_or_tensor
-
+    rows = sys.modules[__package__ + ".linear"]      # which imports this module, and is loaded when this is called
+    as_tensor, fused_input, scaled_or_tensor = rows.as_tensor, rows.fused_input, rows.scaled_or_tensor
     if TC_SWAPPED_MIN_ROWS <= a.shape[0] <= kernels.gemm_skinny_max_m():
         t = scaled_or_tensor(a)
         if not kernels.gemm_tc_takes(t, w, out):
@@ -54,7 +56,7 @@ def try_linear(a, w, out, out_dtype, accumulate, bias, sink=None):
         emit = None
         if sink is not None and kernels.gemm_skinny_emits(x, out):
             emit = kernels.NormEmit(sink.norm_weight)
-        y = kernels.gemm_skinny(x, w, out=out, out_dtype=out_dtype, accumulate=accumulate, bias=bias, emit=emit)
+        y = kernels.gemm_skinny(x, w, out=out, out_dtype=out_dtype, accumulate=accumulate, bias=bias, emit=emit, taken=True)
         if emit is not None:
             sink.emit = emit
         return y
