@@ -872,6 +872,37 @@ def test_prompt_attention_when_scores_climb_and_fall(k, H, Hkv, T, step):
     close(out, attn_ref(q.double(), kk.double(), v.double(), 0, 0, scale).reshape(T, H * hd), dtype, "climbing scores")
 
 
+@pytest.mark.parametrize("H,Hkv", [(2, 2), (8, 1)])
+@pytest.mark.parametrize("start,T", [(0, 2112), (4000, 5), (4001, 37)])
+@pytest.mark.parametrize("climbing", [(0,), (3,), (0, 1, 3)])
+def test_prompt_attention_when_the_warps_are_a_tile_apart(k, H, Hkv, start, T, climbing):
+    """The maxima of some softmax warps (32 rows each) move at every tile and those of the others stay from the first tile on, so
+    that the others run ahead; a whole prompt, and few tokens behind a long cache, where most rows do not exist.  The result is
+    the reference's, and the same bits in each of 50 runs."""
+    from zinfer_b200.parts.attention import query_tiles as attn_tiles_host
+    dtype, hd, page = torch.bfloat16, 64, 64
+    scale, n = 1 / math.sqrt(hd), start + T
+    tile_tokens = k._fn("attention_prefill_tc5", "zk_attn_prefill_tc5_tile_tokens")(H, Hkv)
+    q, kk, v = rnd((T, H, hd), 1, dtype, 0.3), rnd((n, Hkv, hd), 2, dtype, 0.3), rnd((n, Hkv, hd), 3, dtype)
+    kk[:, :, 0] = (torch.arange(n) * (2.0 * math.log(2) / scale / 64))[:, None].to(dtype)     # a factor of 4 per tile
+    warp = torch.arange(T) % tile_tokens // (tile_tokens // 4)
+    q[:, :, 0] = torch.where(torch.isin(warp, torch.tensor(climbing)), 1.0, -1.0)[:, None].to(dtype)
+    setup = PagedSetup([n], [1], 3, page, Hkv, hd, dtype, seed=5)
+    pages = torch.from_numpy(setup.table[1, :-(-n // page)].astype(np.int64)).cuda()
+    fill = torch.full(((-n) % page, Hkv, hd), float("nan"), dtype=dtype)
+    setup.k[pages] = torch.cat([kk, fill]).reshape(-1, page, Hkv, hd).permute(0, 2, 1, 3).cuda()
+    setup.v[pages] = torch.cat([v, fill]).reshape(-1, page, Hkv, hd).permute(0, 2, 1, 3).cuda()
+    tiles = torch.from_numpy(attn_tiles_host([T], tile_tokens)).cuda()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32).cuda()
+    args = (q.reshape(T, H * hd).cuda(), setup.k, setup.v, tiles[0].contiguous(), tiles[1].contiguous(), i32([0, T]),
+            i32([start]), i32([1]), setup.table_dev, H, Hkv, hd, scale)
+    out = k.attention(*args, kind="prompt_tc5")
+    close(out, attn_ref(q.double(), kk.double(), v.double(), start, 0, scale).reshape(T, H * hd), dtype, "warps apart")
+    for _ in range(49):
+        assert torch.equal(k.attention(*args, kind="prompt_tc5"), out)
+    assert k.status_word("cuda").item() == 0
+
+
 # ------------------------------------------------------------------------------- dependent launches
 
 @pytest.mark.parametrize("rows", [1, 8, 40, 300])

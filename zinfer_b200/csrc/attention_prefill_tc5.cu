@@ -14,9 +14,9 @@
 //     cache is the MN-major B operand);
 //   * warps 0..3 are the softmax, a thread per row: it reads its 64 scores with tcgen05.ld, applies the
 //     causal mask, keeps the running maximum and the sum of the online softmax (src/attention.zig:478-517, no
-//     tile skipped) and writes its row of P as bfloat16 into one of two buffers in tensor memory.  Only where
-//     a maximum moved does a warp wait for P V of the tile before and rescale O, and it does so behind the
-//     exponentials.  (A reference that stays until a score passes it by 2^8 is faster still, 209 us where this
+//     tile skipped) and writes its row of P as bfloat16 into one of two buffers in tensor memory, each with barriers of
+//     its own (see NP below).  Only where a maximum moved does a warp wait for P V of the tile before and rescale O, and it does
+//     so behind the exponentials.  (A reference that stays until a score passes it by 2^8 is faster still, 209 us where this
 //     takes 230, but then the largest P is no longer 1 and is rounded: errors against 64 bits 1.77e-3 -> 2.16e-3
 //     with scores of a wide spread.)
 // Q K^T of tile t + 1 is issued before the MMA warp waits for P of tile t, so it runs while the softmax
@@ -72,6 +72,12 @@ __host__ __device__ constexpr int dist_ld(int gp) {      // floats between heads
 static_assert(dist_ld(2) >= dist_len_of(2) && dist_ld(4) >= dist_len_of(4) && dist_ld(8) >= dist_len_of(8), "slices fit their rows");
 constexpr unsigned TMEM_COLS = 256;   // two blocks fit an SM
 constexpr unsigned T_S = 0, T_O = 128, T_P = 192;   // score buffers at columns 0 and 64, O, P at 192 and 224
+// Buffers of P, and for each a barrier "P is written" and a barrier "P V is complete".  A warp whose maxima stay does not wait for
+// P V of the tile before, so it may be a tile ahead of another warp; the scores of tile t + 1 are there before P of tile t is
+// complete.  So the arrivals for t and t + 1 must not meet on one barrier: those of the fast warp for t + 1 would stand for
+// the slow warp's for t, and P V of t would run on rows of P and of O that the slow warp is still at.  With a barrier per buffer they
+// cannot: a warp that arrives for t + 2 has waited for P V of t or of t + 1, and neither begins before every warp arrived for t.
+constexpr int NP = 2;
 
 struct Params {
   bf16* out;
@@ -151,10 +157,10 @@ __global__ void __launch_bounds__(THREADS, 2)
   unsigned long long* kv_full = bars + 1;               // [NSTG]
   unsigned long long* kv_empty = bars + 1 + NSTG;       // [NSTG]
   unsigned long long* s_full = bars + 1 + 2 * NSTG;     // [2]: one per score buffer
-  unsigned long long* p_ready = bars + 3 + 2 * NSTG;    // 1, an arrival per softmax thread
-  unsigned long long* pv_done = bars + 4 + 2 * NSTG;    // [2]: one per P buffer
-  unsigned* tmem_slot = reinterpret_cast<unsigned*>(bars + 6 + 2 * NSTG);
-  static_assert((6 + 2 * NSTG) * 8 + 16 <= 256, "the barriers fit their 256 bytes");
+  unsigned long long* p_ready = bars + 3 + 2 * NSTG;    // [NP]: one per P buffer, an arrival per softmax thread
+  unsigned long long* pv_done = p_ready + NP;           // [NP]: one per P buffer
+  unsigned* tmem_slot = reinterpret_cast<unsigned*>(pv_done + NP);
+  static_assert((3 + 2 * NP + 2 * NSTG) * 8 + 16 <= 256, "the barriers fit their 256 bytes");
   volatile int* aborted = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* dist_sm = reinterpret_cast<float*>(bar_sm + 256);     // EXT: [NSTG][GP][dist_ld(GP)]
 
@@ -187,9 +193,10 @@ __global__ void __launch_bounds__(THREADS, 2)
     }
     mbar_init(&s_full[0], 1);
     mbar_init(&s_full[1], 1);
-    mbar_init(p_ready, SM_THREADS);
-    mbar_init(&pv_done[0], 1);
-    mbar_init(&pv_done[1], 1);
+    for (int i = 0; i < NP; ++i) {
+      mbar_init(&p_ready[i], SM_THREADS);
+      mbar_init(&pv_done[i], 1);
+    }
     *aborted = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
@@ -266,7 +273,8 @@ __global__ void __launch_bounds__(THREADS, 2)
         ok = issue_s(t + 1);
         if (!ok) break;
       }
-      if (!mbar_wait(p_ready, t & 1)) {               // the scores are read, P of tile t is in tensor memory, O is rescaled
+      // the scores are read, P of tile t is in tensor memory, O is rescaled, in every warp
+      if (!mbar_wait(&p_ready[t % NP], (t / NP) & 1)) {
         atomicExch(p.status, 16);
         ok = false;
         break;
@@ -275,10 +283,10 @@ __global__ void __launch_bounds__(THREADS, 2)
       const unsigned long long dv = smem_desc(v_sm(t % NSTG));
 #pragma unroll
       for (int k = 0; k < TK / 16; ++k)   // P: 8 columns (16 keys) further; V: 16 key rows of 128 bytes further
-        umma_bf16_ta(tmem_o, tmem_base + T_P + 32u * (unsigned)(t & 1) + 8u * (unsigned)k, dv + (unsigned long long)(128 * k),
+        umma_bf16_ta(tmem_o, tmem_base + T_P + 32u * (unsigned)(t % NP) + 8u * (unsigned)k, dv + (unsigned long long)(128 * k),
                      idesc_o, (t > 0 || k > 0) ? 1u : 0u);
       umma_commit(&kv_empty[t % NSTG]);
-      umma_commit(&pv_done[t & 1]);
+      umma_commit(&pv_done[t % NP]);
     }
     if (!ok) *aborted = 1;
   } else if (warp < PRODUCER_WARP) {
@@ -300,7 +308,7 @@ __global__ void __launch_bounds__(THREADS, 2)
     bool ok = true;
     // P V of tile t (0 or later) has finished
     auto pv_wait = [&](int t) {
-      ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[t & 1], (t >> 1) & 1));
+      ok = __all_sync(0xffffffffu, mbar_wait(&pv_done[t % NP], (t / NP) & 1));
       if (!ok) {
         atomicExch(p.status, 18);
         *aborted = 1;
@@ -379,10 +387,10 @@ __global__ void __launch_bounds__(THREADS, 2)
           for (int j = 0; j < 32; ++j) w[j] = __float_as_uint(o[j] * alpha);
           tmem_st32(tmem_o + lane_sel + (unsigned)c0, w);
         }
-      } else if (t > 1) {                              // its P buffer may be overwritten
-        if (!pv_wait(t - 2)) break;
+      } else if (t >= NP) {                            // its P buffer may be overwritten
+        if (!pv_wait(t - NP)) break;
       }
-      tmem_st32(tmem_base + T_P + 32u * (unsigned)s + lane_sel, pk);
+      tmem_st32(tmem_base + T_P + 32u * (unsigned)(t % NP) + lane_sel, pk);
       // rows of V beyond the last key of the sequence's step hold stale cache contents
       if (kb + TK > k_end) {
         const int first = k_end - kb;   // 1 .. 63
@@ -391,7 +399,7 @@ __global__ void __launch_bounds__(THREADS, 2)
         fence_async_smem();
       }
       tc_fence_before();
-      mbar_arrive(p_ready);
+      mbar_arrive(&p_ready[t % NP]);
     }
     if (ok) pv_wait(n_tiles - 1);
     if (ok) {   // uniform in the warp: every lane reads its row of O, the rows that exist store it
