@@ -24,26 +24,52 @@ namespace {
 // 334 -> 169; N = 1024, K = 1024 72 -> 42.
 constexpr int BK = 16, PAD = 4;
 
-template <typename T>
-__device__ __forceinline__ void load4(const T* __restrict__ p, bool vec_ok, int k0, int K, bool row_ok, float out[4]) {
-  if (!row_ok) {
-    out[0] = out[1] = out[2] = out[3] = 0.f;
-    return;
+// Four adjacent values of a row, as they are stored until they are put into shared memory: widened at the load, bfloat16 values
+// were waited for there, and no k block was under way beside the FMAs.  PACKED: bfloat16 rows that allow 8-byte loads, two values
+// to a register.  [450, 1024] x 9216 with bfloat16 operands, microseconds with values widened at the load and now: 260 -> 197
+// (305 with 64 x 64 tiles, 4 x 4 outputs, one buffer); K = 1022, whose rows allow no 8-byte loads, 277 -> 231 (391);
+// [16, 1024] x 9216 104 -> 35 (96); [128, 1022] x 4736 182 -> 57 (119).
+template <typename T, bool PACKED> struct Four { T v[4]; };
+template <> struct Four<bf16, true> { uint2 v; };
+
+template <typename T, bool PACKED>
+__device__ __forceinline__ float nth(const Four<T, PACKED>& f, int j) {
+  if constexpr (PACKED) {
+    const unsigned w = j < 2 ? f.v.x : f.v.y;
+    return __uint_as_float((j & 1) ? w & 0xffff0000u : w << 16);
+  } else {
+    return to_f32(f.v[j]);
   }
-  if (vec_ok && k0 + 3 < K) {
-    if constexpr (sizeof(T) == 4) {
-      const float4 v = *reinterpret_cast<const float4*>(p + k0);
-      out[0] = v.x; out[1] = v.y; out[2] = v.z; out[3] = v.w;
-    } else {
-      const uint2 v = *reinterpret_cast<const uint2*>(p + k0);
-      const __nv_bfloat162 lo = *reinterpret_cast<const __nv_bfloat162*>(&v.x);
-      const __nv_bfloat162 hi = *reinterpret_cast<const __nv_bfloat162*>(&v.y);
-      out[0] = __low2float(lo); out[1] = __high2float(lo); out[2] = __low2float(hi); out[3] = __high2float(hi);
+}
+
+// Values beyond K, and those of a row that does not exist, are zeros.
+template <typename T, bool PACKED>
+__device__ __forceinline__ void load4(const T* __restrict__ p, bool vec_ok, int k0, int K, bool row_ok, Four<T, PACKED>& out) {
+  if constexpr (PACKED) {
+    if (row_ok && k0 + 3 < K) {
+      out.v = *reinterpret_cast<const uint2*>(p + k0);
+      return;
     }
-    return;
-  }
+    unsigned h[3];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) out[j] = (k0 + j < K) ? to_f32(p[k0 + j]) : 0.f;
+    for (int j = 0; j < 3; ++j) h[j] = row_ok && k0 + j < K ? __bfloat16_as_ushort(p[k0 + j]) : 0;
+    out.v = make_uint2(h[0] | h[1] << 16, h[2]);
+  } else if constexpr (sizeof(T) == 4) {
+    if (!row_ok) {
+      out.v[0] = out.v[1] = out.v[2] = out.v[3] = 0.f;
+      return;
+    }
+    if (vec_ok && k0 + 3 < K) {
+      const float4 v = *reinterpret_cast<const float4*>(p + k0);
+      out.v[0] = v.x; out.v[1] = v.y; out.v[2] = v.z; out.v[3] = v.w;
+      return;
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out.v[j] = (k0 + j < K) ? p[k0 + j] : 0.f;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out.v[j] = row_ok && k0 + j < K ? p[k0 + j] : from_f32<T>(0.f);
+  }
 }
 
 // Two float32 FMAs in one instruction, each rounded as fmaf rounds.
@@ -56,9 +82,10 @@ __device__ __forceinline__ void fma2(float2& d, float a, float2 b) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(dd));
 }
 
-template <int BM, int BN, int TM, int TN, int PF, typename TA, typename TW, typename TC>
+// vecA, vecW: rows that allow loads of four float32 values (PACKED: both operands' rows allow loads of four bfloat16 values).
+template <int BM, int BN, int TM, int TN, int PF, bool PACKED, typename T, typename TC>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN), TM * TN >= 64 ? 2 : 3)
-    gemm_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TC* __restrict__ C, const float* __restrict__ bias,
+    gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ W, TC* __restrict__ C, const float* __restrict__ bias,
                      int M, int N, int K, int lda, int ldw, int ldc, int accumulate, int vecA, int vecW) {
   constexpr int TX = BN / TN, TY = BM / TM, THREADS = TX * TY;
   constexpr int GM = TM / 4, GN = TN / 4;                   // groups of 4 rows / columns per thread
@@ -76,19 +103,19 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), TM * TN >= 64 ? 2 : 3)
 #pragma unroll
     for (int j = 0; j < TN / 2; ++j) acc[i][j] = make_float2(0.f, 0.f);
 
-  float av[PF][LA][4], wv[PF][LW][4];
+  Four<T, PACKED> av[PF][LA], wv[PF][LW];
   auto fetch = [&](int kb, int f) {
 #pragma unroll
     for (int l = 0; l < LA; ++l) {
       const int p = tid + l * THREADS, r = p >> 2, k = (p & 3) * 4;
       const bool ok = m0 + r < M;
-      load4<TA>(A + (size_t)(ok ? m0 + r : 0) * lda, vecA, kb + k, K, ok, av[f][l]);
+      load4<T, PACKED>(A + (size_t)(ok ? m0 + r : 0) * lda, vecA, kb + k, K, ok, av[f][l]);
     }
 #pragma unroll
     for (int l = 0; l < LW; ++l) {
       const int p = tid + l * THREADS, r = p >> 2, k = (p & 3) * 4;
       const bool ok = n0 + r < N;
-      load4<TW>(W + (size_t)(ok ? n0 + r : 0) * ldw, vecW, kb + k, K, ok, wv[f][l]);
+      load4<T, PACKED>(W + (size_t)(ok ? n0 + r : 0) * ldw, vecW, kb + k, K, ok, wv[f][l]);
     }
   };
   auto put = [&](int buf, int f) {
@@ -96,13 +123,13 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), TM * TN >= 64 ? 2 : 3)
     for (int l = 0; l < LA; ++l) {
       const int p = tid + l * THREADS, r = p >> 2, k = (p & 3) * 4;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) As[buf][k + j][r] = av[f][l][j];
+      for (int j = 0; j < 4; ++j) As[buf][k + j][r] = nth(av[f][l], j);
     }
 #pragma unroll
     for (int l = 0; l < LW; ++l) {
       const int p = tid + l * THREADS, r = p >> 2, k = (p & 3) * 4;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) Ws[buf][k + j][r] = wv[f][l][j];
+      for (int j = 0; j < 4; ++j) Ws[buf][k + j][r] = nth(wv[f][l], j);
     }
   };
 
@@ -302,8 +329,11 @@ int launch_tiles(const void* A, const void* W, void* C, const float* bias, int M
   const int vecA = (lda % 4 == 0) && ((uintptr_t)A % 16 == 0);
   const int vecW = (ldw % 4 == 0) && ((uintptr_t)W % 16 == 0);
   dim3 grid(ceil_div_i(N, BN), ceil_div_i(M, BM));
-  gemm_simt_kernel<BM, BN, TM, TN, PF, T, T, TC><<<grid, (BM / TM) * (BN / TN), 0, stream>>>(
-      (const T*)A, (const T*)W, (TC*)C, bias, M, N, K, lda, ldw, ldc, accumulate, vecA, vecW);
+  auto kern = gemm_simt_kernel<BM, BN, TM, TN, PF, false, T, TC>;
+  if constexpr (sizeof(T) == 2)
+    if (vecA && vecW) kern = gemm_simt_kernel<BM, BN, TM, TN, PF, true, T, TC>;
+  kern<<<grid, (BM / TM) * (BN / TN), 0, stream>>>((const T*)A, (const T*)W, (TC*)C, bias, M, N, K, lda, ldw, ldc, accumulate,
+                                                   vecA, vecW);
   return ZK_LAUNCH_STATUS();
 }
 
