@@ -358,19 +358,22 @@ int launch(const void* A, const void* W, void* C, const float* bias, int M, int 
   const bool pieces = K % PIECE == 0 && lda % PIECE == 0 && ldw % PIECE == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0;
   // The few-row form reads A once per 16 weight rows, which pays while the weights are the larger part or a tiled form would
   // leave most SMs idle.  Microseconds at 20 rows, few / 32 x 32 tiles: N = 1024 15 / 27 (K = 1024), 50 / 117 (K = 4608);
-  // N = 9216 44 / 31.
-  if (pieces && (M <= 8 || (M <= FEW_MAX_M && ceil_div_i(N, FEW_ROWS) <= 2 * 148))) {
+  // N = 9216 44 / 31.  A k block is 512 bytes of a row, and what K leaves of it is zeros: with less than one block the form pays
+  // only where both hold (K = 64, bfloat16, few / tiles: 8 x 65536 33 / 21, 40 x 4736 16 / 8, 8 x 3072 8 / 8).
+  const bool little = M <= 8, narrow = ceil_div_i(N, FEW_ROWS) <= 2 * 148, whole = K * sizeof(T) >= 512;
+  if (pieces && M <= FEW_MAX_M && (whole ? little || narrow : little && narrow)) {
     if (M <= 4) return launch_few<4, 1, 6, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
     if (M <= 8) return launch_few<8, 1, 6, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
     if (M <= 16) return launch_few<16, 1, 5, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
     if (M <= 32) return launch_few<16, 2, 4, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
     return launch_few<16, 4, 3, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
   }
-  // The largest tile that still gives (nearly) every SM a block.  450 rows, microseconds with 128 x 128 / 64 x 64 / 32 x 32
+  // The largest tile that still gives (nearly) every SM a block, and no taller than the rows need: 128 rows of A cost their
+  // FMAs whether they exist or not (16 rows, N = 65536, K = 1024: 350 / 190 / 154, and 277 with one buffer).  450 rows, microseconds with 128 x 128 / 64 x 64 / 32 x 32
   // tiles: N = 9216, K = 1024 195 / 224 / 326; N = 1024, K = 4608 474 / 169 / 199; 100 rows of the latter 463 / 165 / 111.
-  if (ceil_div_i(M, 128) * ceil_div_i(N, 128) >= 148)
+  if (M > 64 && ceil_div_i(M, 128) * ceil_div_i(N, 128) >= 148)
     return launch_tiles<128, 128, 8, 8, 1, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
-  if (ceil_div_i(M, 64) * ceil_div_i(N, 64) >= 100)
+  if (M > 32 && ceil_div_i(M, 64) * ceil_div_i(N, 64) >= 100)
     return launch_tiles<64, 64, 8, 4, 2, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
   return launch_tiles<32, 32, 4, 4, 4, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
 }
