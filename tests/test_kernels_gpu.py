@@ -124,6 +124,40 @@ def test_gemm_simt_forms_agree(k, dtype, M, N, K):
     assert torch.equal(k.gemm_simt(wide, w, out_dtype=torch.float32), got)
 
 
+def in_threads(calls, times):
+    """Every call of `calls` run `times` times in a thread and on a stream of its own; the statuses that were not 0."""
+    import threading
+    failed, gate = [], threading.Barrier(len(calls))
+
+    def work(call):
+        stream = torch.cuda.Stream()
+        gate.wait()
+        failed.extend(s for s in (call(stream.cuda_stream) for _ in range(times)) if s)
+        stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(c,)) for c in calls]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    return failed
+
+
+@pytest.mark.parametrize("rows", [(64, 33), (4, 1), (16, 9)])
+def test_gemm_simt_of_few_rows_in_threads(k, rows):
+    """Two row counts that one instantiation serves, with unequal shared memory: no thread takes away what another's launch needs."""
+    K, N = 128, 64
+    fn, w = k._fn("gemm_simt", "zk_gemm_simt"), rnd((N, K), 6, torch.float32).cuda()
+    ins = [rnd((M, K), M, torch.float32).cuda() for M in rows]
+    outs = [torch.zeros((M, N), device="cuda") for M in rows]
+    torch.cuda.synchronize()
+    calls = [lambda stream, a=a, o=o: fn(a.data_ptr(), w.data_ptr(), o.data_ptr(), None, a.shape[0], N, K, K, K, N, k.F32, k.F32,
+                                         0, stream) for a, o in zip(ins, outs)]
+    assert in_threads(calls, 3000) == []
+    for a, o in zip(ins, outs):
+        close(o, a.double() @ w.double().T, torch.float32, "few rows in threads")
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 331, 80), (8, 6144, 2048), (5, 100, 8200), (16, 2048, 512), (9, 48, 64),
                                    (33, 257, 1000), (64, 1030, 2048), (3, 65536 + 8, 256)])
 def test_gemm_skinny(k, M, N, K):

@@ -341,9 +341,14 @@ template <int GROUPS, int NT, int STAGES, typename T, typename TC>
 int launch_few(const void* A, const void* W, void* C, const float* bias, int M, int N, int K, int lda, int ldw, int ldc,
                int accumulate, cudaStream_t stream) {
   auto kern = gemm_few_kernel<GROUPS, NT, STAGES, T, TC>;
-  const size_t smem = (size_t)STAGES * (FEW_ROWS + M) * (512 + 16);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  constexpr size_t ROW = (size_t)STAGES * (512 + 16);
+  // The limit belongs to the instantiation and is shared by all threads of the process: every call sets it to what the largest M
+  // needs, so that none lowers it between another's setting and launch.
+  constexpr size_t LIMIT = ROW * (FEW_ROWS + GROUPS * NT);
+  const size_t smem = ROW * (FEW_ROWS + M);
+  if (smem > LIMIT) return ZK_EINVAL;
+  if constexpr (LIMIT > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIMIT);
     if (e != cudaSuccess) return (int)e;
   }
   kern<<<ceil_div_i(N, FEW_ROWS), FEW_ROWS * GROUPS, smem, stream>>>((const T*)A, (const T*)W, (TC*)C, bias, M, N, K, lda, ldw,
