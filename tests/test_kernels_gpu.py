@@ -131,6 +131,7 @@ def in_threads(calls, times):
 
     def work(call):
         stream = torch.cuda.Stream()
+        torch.zeros(1, device="cuda")          # the runtime makes the device's context the thread's with a thread's first launch
         gate.wait()
         failed.extend(s for s in (call(stream.cuda_stream) for _ in range(times)) if s)
         stream.synchronize()
@@ -935,6 +936,41 @@ def test_prompt_attention_when_the_warps_are_a_tile_apart(k, H, Hkv, start, T, c
     for _ in range(49):
         assert torch.equal(k.attention(*args, kind="prompt_tc5"), out)
     assert k.status_word("cuda").item() == 0
+
+
+def test_prompt_attention_options_in_threads(k):
+    """Calls with and without a distance table share a kernel and need unequal shared memory: neither takes away what the other's
+    launch needs."""
+    from zinfer_b200.parts.attention import query_tiles as attn_tiles_host
+    H, Hkv, hd, page, T = 8, 1, 64, 64, 100
+    setup = PagedSetup([T], [0], 1, page, Hkv, hd, torch.bfloat16, seed=5)
+    setup.k.normal_()
+    setup.v.normal_()
+    fn = k._fn("attention_prefill_tc5", "zk_attn_prefill_tc5")
+    tiles = torch.from_numpy(attn_tiles_host([T], k._fn("attention_prefill_tc5", "zk_attn_prefill_tc5_tile_tokens")(H, Hkv))).cuda()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32).cuda()
+    q, gate = rnd((T, H * hd), 1, torch.bfloat16).cuda(), rnd((T, H), 2, torch.bfloat16).cuda()
+    table = k.DistanceTable(rnd((H, 50), 3, torch.float32).cuda()).padded()
+    cu, zero = i32([0, T]), i32([0])
+    outs = [torch.zeros_like(q) for _ in range(4)]
+    status = k.status_word("cuda")
+
+    def call(out, dist):
+        return lambda stream: fn(q.data_ptr(), setup.k.data_ptr(), setup.v.data_ptr(), out.data_ptr(), tiles[0].data_ptr(),
+                                 tiles[1].data_ptr(), cu.data_ptr(), zero.data_ptr(), zero.data_ptr(), setup.table_dev.data_ptr(),
+                                 setup.table_dev.stride(0), tiles.shape[1], T, setup.k.shape[0], H, Hkv, hd, page, 0.125,
+                                 status.data_ptr(), None, None, table.data_ptr() if dist else None, table.shape[1] if dist else 0, 0,
+                                 gate.data_ptr(), H, stream)
+
+    calls = [call(o, i % 2 == 0) for i, o in enumerate(outs)]
+    torch.cuda.synchronize()
+    alone = []
+    for c, o in zip(calls, outs):
+        assert c(torch.cuda.current_stream().cuda_stream) == 0
+        alone.append(o.clone())
+    torch.cuda.synchronize()
+    assert in_threads(calls, 2000) == [] and status.item() == 0
+    assert all(torch.equal(o, a) for o, a in zip(outs, alone)) and not torch.equal(alone[0], alone[1])
 
 
 # ------------------------------------------------------------------------------- dependent launches

@@ -70,6 +70,8 @@ __host__ __device__ constexpr int dist_ld(int gp) {      // floats between heads
   return gp == 1 ? dist_len_of(1) : gp == 2 ? 144 : gp == 4 ? 104 : 100;
 }
 static_assert(dist_ld(2) >= dist_len_of(2) && dist_ld(4) >= dist_len_of(4) && dist_ld(8) >= dist_len_of(8), "slices fit their rows");
+constexpr size_t DIST_BYTES = (size_t)NSTG * 8 * dist_ld(8) * sizeof(float);      // slices of all stages with the most heads
+static_assert(dist_ld(1) <= 8 * dist_ld(8) && 2 * dist_ld(2) <= 8 * dist_ld(8) && 4 * dist_ld(4) <= 8 * dist_ld(8), "8 heads need the most");
 constexpr unsigned TMEM_COLS = 256;   // two blocks fit an SM
 constexpr unsigned T_S = 0, T_O = 128, T_P = 192;   // score buffers at columns 0 and 64, O, P at 192 and 224
 // Buffers of P, and for each a barrier "P is written" and a barrier "P V is complete".  A warp whose maxima stay does not wait for
@@ -524,7 +526,10 @@ int zk_attn_prefill_tc5(const void* q, const void* k_cache, const void* v_cache,
   p.dist = dist; p.dist_row = dist_row; p.mask_chunk = mask_chunk; p.gate = (const bf16*)gate; p.ld_gate = ld_gate;
   auto kern = ext ? attn_prefill_tc5_kernel<true> : attn_prefill_tc5_kernel<false>;
   const size_t smem = SMEM_BYTES + (dist ? (size_t)NSTG * gp * dist_ld(gp) * sizeof(float) : 0);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // The limit belongs to the kernel and is shared by all threads of the process: every call sets it to the most that any call
+  // needs, so that none lowers it between another's setting and launch.
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(SMEM_BYTES + (ext ? DIST_BYTES : 0)));
   if (e != cudaSuccess) return (int)e;
   if ((long long)n_tiles * Hkv * (G / gp) > 0x7fffffffLL) return ZK_EINVAL;
   dim3 grid(n_tiles * Hkv * (G / gp), 1, part_o ? Hkv : 1);
