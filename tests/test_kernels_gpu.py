@@ -1022,11 +1022,13 @@ def test_dependent_launches_keep_the_order_of_a_chain(k, rows):
 @pytest.mark.parametrize("glu", ["silu", "relu", "clamp"])
 def test_gemm_tc_gated_units_over_the_whole_range(k, M, splits, glu):
     """Weights that pick column 0 as every gate and column 1 as every up: the unit alone, for gates from -1e4 to 1e4.
-    The float32 unit is a few ulp off (8 * 2^-23) and is rounded once to bfloat16, whose 8 significant bits
-    give 2^-8 of the value; below 1e-35 it may be 0."""
+    The float32 unit is a few ulp off (8 * 2^-23, and what rounding its argument does to the clamped unit's exponential) and is
+    rounded once to bfloat16, whose 8 significant bits give 2^-8 of the value, or half of the smallest number (2^-133).  Where
+    the exponential is beyond float32 (a gate below -88.7) the unit is 0."""
     F, K = 256, 576
     x = torch.zeros(M, K)
-    x[:, 0] = torch.cat([torch.linspace(-130, 130, M - 9), torch.tensor([-1e4, 1e4, 0.0, -0.0, -87.5, -88.0, -1e-3, 1e-3, 9.0])])
+    x[:, 0] = torch.cat([torch.linspace(-130, 130, M - 11),
+                         torch.tensor([-1e4, 1e4, 0.0, -0.0, -44.5, -51.5, -87.5, -88.0, -88.5, -1e-3, 9.0])])
     x[:, 1] = torch.linspace(-3, 5, M)
     w = torch.zeros(2 * F, K)
     w.view(F // 16, 2, 16, K)[:, 0, :, 0] = 1
@@ -1035,10 +1037,14 @@ def test_gemm_tc_gated_units_over_the_whole_range(k, M, splits, glu):
     g, u = x[:, 0].double(), x[:, 1].double()
     if glu == "clamp":
         g = g.clamp(max=7.0)
-        ref = g * torch.sigmoid(1.702 * g) * (u.clamp(-7.0, 7.0) + 1)
+        arg = 1.702 * g
+        ref = g * torch.sigmoid(arg) * (u.clamp(-7.0, 7.0) + 1)
         got = k.gemm_tc(x, w, swiglu=True, splits=splits, glu_clamp=(7.0, 1.702))
     else:
+        arg = g if glu == "silu" else torch.relu(g)
         ref = (g * torch.sigmoid(g) if glu == "silu" else torch.relu(g)) * u
         got = k.gemm_tc(x, w, swiglu=True, splits=splits, glu_act=glu)
     err = (got.double() - ref[:, None]).abs()
-    assert (err <= ref.abs()[:, None] * (2 ** -8 + 8 * 2 ** -23) + 1e-35).all()
+    rel = 2 ** -8 + 8 * 2 ** -23 + (arg.abs() * 2 ** -23 if glu == "clamp" else 0)
+    bound = torch.where(arg < -88.7, ref.abs(), ref.abs() * rel + 2.0 ** -134)
+    assert (err <= bound[:, None]).all()

@@ -43,17 +43,23 @@ constexpr int THREADS = 192;     // producer warp, MMA warp, four epilogue warps
 
 // The gated unit of the fused epilogues: silu(g) * u, with limit > 0 the clamped unit described in Params, with limit < 0
 // relu(g) * u.
-// A unit that is stored as bfloat16 divides with __fdividef (2 ulp of float32, 1 / 16,000 of the rounding that follows; the
-// denominator is 1 or more, and where it passes 2^126 a quotient of 1e-36 becomes 0).  What bounded the epilogues was one
-// warp per scheduler waiting through branch after branch: the IEEE division's way to its slow path and the choice of the
-// unit stood between any two of a thread's units, so that none overlapped.  The epilogue of a 256 x 256 tile, 128 units a
-// thread, took 14 us where the tile's MMAs take 4 (K = 1024) to 8 (K = 2048).  8,192 rows: w1|w3 with K = 1024, N = 9216
-// 225 us, without the division's branch 193, with the unit chosen outside the loop (glu_units) 103; K = 2048, N = 16384
-// 481 -> 353 us.
+// A unit that is stored as bfloat16 divides with __fdividef (2 ulp of float32, 1 / 16,000 of the rounding that follows).  That
+// gives 0 for a divisor beyond 2^126, which gates from -87.4 to -88.7 reach, so a large divisor and its dividend are first made
+// smaller by the same power of two.  A million units of each spread (gates and ups of 0.3, 1, 4, 20 standard deviations, gates
+// from -90 to -80): the error against 64 bits is the IEEE division's in eight digits, 3 to 5 stored values in a million differ.
+// What bounded the epilogues was one warp per scheduler waiting through branch after branch: the IEEE division's way to its slow
+// path and the choice of the unit stood between any two of a thread's units, so that none overlapped.  The epilogue of a 256 x 256
+// tile, 128 units a thread, took 14 us where the tile's MMAs take 4 (K = 1024) to 8 (K = 2048).  w1|w3 of 8,192 rows, K = 1024,
+// N = 9216, with both 225 us, with the unit chosen outside the loop (glu_units) 179, and this division 114 (112 without the
+// power of two); 300 rows, K = 2048, N = 16384 72 -> 39, clamped 80 -> 47.
 template <typename TC>
 __device__ __forceinline__ float glu_quotient(float g, float e) {
-  if constexpr (sizeof(TC) == 2) return __fdividef(g, 1.0f + e);
-  else return g / (1.0f + e);
+  if constexpr (sizeof(TC) == 2) {
+    const float d = 1.0f + e, s = d > 0x1p64f ? 0x1p-64f : 1.0f;
+    return __fdividef(g * s, d * s);
+  } else {
+    return g / (1.0f + e);
+  }
 }
 template <typename TC>
 __device__ __forceinline__ float glu_unit(float g, float u, float limit, float alpha) {
