@@ -1,5 +1,6 @@
 """The ctypes signatures in zinfer_b200/kernels.py must match the C prototypes in csrc/*.cu:
 a mismatch would pass garbage to a kernel launcher."""
+import inspect
 import re
 from pathlib import Path
 
@@ -41,3 +42,9 @@ def test_every_exported_launcher_has_a_signature():
         exported = set(re.findall(r"\b(?:int|long long)\s+(zk_\w+)\s*\(", cu.read_text()))
         known = set(kernels._SIGNATURES.get(cu.stem, {}))
         assert exported <= known, f"{cu.name}: {sorted(exported - known)} have no ctypes signature"
+
+
+def test_no_public_contraction_takes_the_callers_word_for_its_checks():
+    for fn, names in ((kernels.gemm_skinny, "a w out out_dtype accumulate bias emit col_scale act"),
+                      (kernels.gemm_skinny_swiglu, "a w_gate_up act")):
+        assert list(inspect.signature(fn).parameters) == names.split()

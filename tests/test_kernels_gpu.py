@@ -176,6 +176,12 @@ def test_gemm_skinny(k, M, N, K):
     close(res, ref + res0.double(), torch.float32, "skinny accumulate")
     assert not k.gemm_skinny_takes(rnd((65, K), 1, torch.bfloat16).cuda(), w)
     assert not k.gemm_skinny_takes(rnd((2, 12), 1, torch.bfloat16).cuda(), rnd((4, 12), 1, torch.bfloat16).cuda())
+    for bad in (rnd((2, K + 8), 1, torch.bfloat16).cuda(), rnd((2, K), 1, torch.float32).cuda(),
+                rnd((K, 2), 1, torch.bfloat16).cuda().T):
+        with pytest.raises(k.KernelError):
+            k.gemm_skinny(bad, w)
+        with pytest.raises(k.KernelError):
+            k.gemm_skinny_swiglu(bad, rnd((32, K), 2, torch.bfloat16).cuda())
 
 
 @pytest.mark.parametrize("M,N,K", [(128, 128, 64), (200, 331 * 8, 2048), (2048, 6144, 2048), (130, 264, 8200),
