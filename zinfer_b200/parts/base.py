@@ -134,7 +134,7 @@ class Norm(Part):
 
     def pending(self, ctx, x: torch.Tensor):
         """The norm of all rows of `x` as an object that a consumer with `takes_pending_norm`
-        resolves itself (parts.linear.NormedRows), or None if this norm has no such form; the
+        resolves itself (parts.rows.NormedRows), or None if this norm has no such form; the
         caller then uses `forward`.  A norm that also has `ahead(ctx, x)` takes what that returned
         as a third argument."""
         return None

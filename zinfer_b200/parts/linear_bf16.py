@@ -6,9 +6,8 @@ pending RMSNorm itself.  More rows (prompt steps): the TMA-fed tcgen05 kernel wi
 accumulator in tensor memory."""
 from __future__ import annotations
 
-import sys
-
 from .. import kernels
+from .rows import as_tensor, fused_input, scaled_or_tensor
 
 
 # From 17 to 64 rows the tcgen05 kernel with the weights on its 128-row side beats the mma.sync
@@ -36,8 +35,6 @@ def swapped_splits(n_weight_rows: int, sm_count: int) -> int:
 
 
 def try_linear(a, w, out, out_dtype, accumulate, bias, sink=None):
-    rows = sys.modules[__package__ + ".linear"]      # which imports this module, and is loaded when this is called
-    as_tensor, fused_input, scaled_or_tensor = rows.as_tensor, rows.fused_input, rows.scaled_or_tensor
     if TC_SWAPPED_MIN_ROWS <= a.shape[0] <= kernels.gemm_skinny_max_m():
         t = scaled_or_tensor(a)
         if not kernels.gemm_tc_takes(t, w, out):
