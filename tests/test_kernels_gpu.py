@@ -124,6 +124,37 @@ def test_gemm_simt_forms_agree(k, dtype, M, N, K):
     assert torch.equal(k.gemm_simt(wide, w, out_dtype=torch.float32), got)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M,N,K", [(129, 9477, 52), (129, 9476, 45), (129, 9476, 48), (200, 1924, 37), (70, 4803, 40), (450, 1026, 104),
+                                   (33, 6404, 24), (17, 4804, 19), (3, 4805, 24), (2, 65540, 64), (12, 200, 264), (24, 201, 264),
+                                   (64, 4731, 520), (8, 4731, 136), (300, 31, 21), (1, 3, 5)])
+def test_gemm_simt_edges_of_every_form(k, dtype, M, N, K):
+    """Weight rows, rows and values of k beyond the last tile of each tile size and of the few-row form, with a bias, summed into
+    what is there, stored as bfloat16, into rows that take 16-byte stores and rows that do not (N a multiple of 4 or not).
+    The bound: K float32 sums in order (and two more additions), then one rounding to bfloat16 (2^-8 of the value)."""
+    a = rnd((M, K), 5, dtype).cuda()
+    w = rnd((N, K), 6, dtype, 0.1).cuda()
+    bias, old = rnd((N,), 7, torch.float32).cuda(), rnd((M, N), 8, torch.float32).cuda()
+    ref = a.double() @ w.double().T
+    sums = K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+
+    def check(got, want, terms, rounds=0.0):
+        bound = sums + 2 * 2.0 ** -24 * terms + rounds * (want.abs() + sums + 2.0 ** -22 * terms) + 1e-30
+        assert ((got.double() - want).abs() <= bound).all()
+
+    check(k.gemm_simt(a, w, out_dtype=torch.float32), ref, 0 * ref)
+    check(k.gemm_simt(a, w, bias=bias, out_dtype=torch.float32), ref + bias.double(), ref.abs() + bias.double().abs())
+    out = old.clone()
+    k.gemm_simt(a, w, out=out, accumulate=True, bias=bias)
+    check(out, ref + bias.double() + old.double(), ref.abs() + 2 * bias.double().abs() + old.double().abs())
+    if dtype == torch.bfloat16:
+        check(k.gemm_simt(a, w), ref, 0 * ref, 2.0 ** -8)
+        out = old.bfloat16()
+        k.gemm_simt(a, w, out=out, accumulate=True)
+        want = ref + old.bfloat16().double()
+        check(out, want, ref.abs() + old.abs().double(), 2.0 ** -8)
+
+
 def in_threads(calls, times):
     """Every call of `calls` run `times` times in a thread and on a stream of its own; the statuses that were not 0."""
     import threading
