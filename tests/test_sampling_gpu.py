@@ -39,10 +39,10 @@ def test_argmax_first_maximum_wins_and_nan_never_does(k):
     assert k.argmax(torch.from_numpy(big).cuda()).cpu().tolist() == np.argmax(big, axis=1).tolist()
 
 
-@pytest.mark.parametrize("V", [4095, 4096, 16384, 16388, 16400, 65536, 65541, 131072])
+@pytest.mark.parametrize("V", [4095, 4096, 16384, 16388, 16400, 32768, 65536, 65541, 65544, 80000, 100000, 131072, 131100])
 def test_argmax_in_vectors_and_remainders(k, V):
-    """Pieces that are whole vectors, have a remainder, or do not begin on 16 bytes; ties within a vector, between threads, warps
-    and pieces, zeros of both signs, a row of -inf, one of NaN and -inf."""
+    """Pieces without a span of 4,096 logits (below 65,521), of one or two spans, with a remainder, or that do not begin on 16
+    bytes; ties within a vector, between threads, warps and pieces, zeros of both signs, a row of -inf, one of NaN and -inf."""
     x = logits_rows(9, V, V)
     for row, at in enumerate([[V - 1], [0], [V // 2, V // 2 + 1], [5, 6, V - 1], [1027, 40, V // 3], [V - 2, V // 16]]):
         x[row, at] = 99.0

@@ -337,7 +337,9 @@ __global__ void argmax_kernel(const float* __restrict__ logits, int V, int* __re
   };
   // A step waits for this kernel, and it is one chain of waits: so four 16-byte loads under way per thread (with one number at
   // a time a piece of 4,096 was 16 trips to memory), and value and index in one number and one reduction.  65,536 logits,
-  // microseconds added to a step: 1 row 8.2 -> 5.1, 8 rows 10.2 -> 7.1, 64 rows 12.8 -> 9.1.
+  // microseconds added to a step: 1 row 8.2 -> 5.1, 8 rows 10.2 -> 7.1, 64 rows 12.8 -> 9.1.  The loads go by whole spans of 4,096
+  // logits that begin on 16 bytes: rows are cut into 16 pieces, so rows of some 65,520 logits and more have them; what a span
+  // does not cover, and shorter rows (32,768 logits: 8 trips), are read one at a time.
   int i0 = lo;
   if (((reinterpret_cast<uintptr_t>(row + lo)) & 15) == 0) {
     const int span = 16 * blockDim.x;
