@@ -16,19 +16,20 @@
 //     causal mask, keeps the running maximum and the sum of the online softmax (src/attention.zig:478-517, no
 //     tile skipped) and writes its row of P as bfloat16 into one of two buffers in tensor memory, each with barriers of
 //     its own (see NP below).  Only where a maximum moved does a warp wait for P V of the tile before and rescale O, and it does
-//     so behind the exponentials.  (A reference that stays until a score passes it by 2^8 is faster still, 209 us where this
-//     takes 230, but then the largest P is no longer 1 and is rounded: errors against 64 bits 1.77e-3 -> 2.16e-3
+//     so behind the exponentials.  (A reference that stays until a score passes it by 2^8 is faster still, 209 us against
+//     230, but then the largest P is no longer 1 and is rounded: errors against 64 bits 1.77e-3 -> 2.16e-3
 //     with scores of a wide spread.)
 // Q K^T of tile t + 1 is issued before the MMA warp waits for P of tile t, so it runs while the softmax
 // warps work on tile t, and P V of tile t runs while they work on tile t + 1.  One block needs 256
 // columns of tensor memory (two score buffers, O, two of P) and 82 KB of shared memory: two blocks share an SM.
 // What bounds it: the special-function unit (64 x 128 exponentials are 512 cycles of an SM, the MMAs of the
-// tile 256) at 62 % of its rate; the rest is a warp's chain from scores to P with two warps per scheduler.
-// Measured on a B200, microseconds a layer, against two threads per row that exchanged their maxima
-// every tile, P in shared memory and the blocks head after head: 16 heads on 8, 8,192 tokens 317 -> 230 (598 TFLOP/s;
-// 261 with O rescaled before the exponentials); 32 heads on 8, 8,192 tokens 638 -> 520; 2,048 tokens 62 -> 43.  With one score
-// buffer that P replaces (four blocks an SM, the scores read twice for the registers) it took a fifth longer.  Scores stay
-// unscaled in registers; the
+// tile 256), whose pipe is busy for 58 % of the cycles (8,192 tokens; the clock is 1.69 GHz under this load); the rest is a
+// warp's chain from scores to P with two warps per scheduler.
+// Measured on a B200, microseconds a layer with flushed caches, against two threads per row that exchanged their maxima
+// every tile, P in shared memory and the blocks head after head: 8,192 tokens, 16 heads on 8 332 -> 240 (573 TFLOP/s),
+// 32 heads on 8 554 -> 453; 2,048 tokens 46 -> 38 and 70 -> 51; with a distance table 461 -> 330 (8,192 tokens, 16 heads).  With O
+// rescaled before the exponentials it took 261 where this form took 230; with one score buffer that P replaces (four blocks an
+// SM, the scores read twice for the registers) a fifth longer.  Scores stay unscaled in registers; the
 // scale is folded into the exponent (2^((s - m) * scale * log2 e), ex2.approx), tiles below the
 // diagonal skip the mask.
 //

@@ -13,10 +13,10 @@ from .rows import as_tensor, fused_input, scaled_or_tensor
 # From 17 to 64 rows the tcgen05 kernel with the weights on its 128-row side beats the mma.sync
 # kernel (measured at 64 rows on the LFM2-1.2B shapes: 17 us against 44 us for N = 16384, 10 against
 # 22 for N = 6144, 7 against 12 for N = 2048, 12 against 38 for N = 2048 with K = 8192).  Up to 16
-# rows the mma.sync kernel is as fast or faster (16 rows: 3.1 against 5.0 us for out_proj, 9.0
-# against 10.3 for w2, 5.9 against 6.1 for qkv, 9.3 against 8.6 for in_proj, 16.4 against 15.7 for
-# w1|w3), fuses the short convolution and needs no cluster: whole steps of 9 / 12 / 16 sequences
-# 0.83 / 0.84 / 0.88 ms against 0.90 / 0.91 / 0.97.
+# rows the mma.sync kernel needs no cluster and applies pending norms itself.  Whole steps of 9 / 12 / 16 sequences at
+# 500 tokens, ms, mma.sync against tcgen05 (the short convolution fused in both): the 350M shape 0.43 / 0.47 / 0.49 against
+# 0.54 / 0.56 / 0.57; LFM2-1.2B 0.72 / 0.76 / 0.80 against 0.83 / 0.86 / 0.86; the 2.6B shape 1.51 / 1.59 / 1.66 against
+# 1.58 / 1.61 / 1.64.
 TC_SWAPPED_MIN_ROWS = 17
 
 
