@@ -1176,11 +1176,6 @@ def gemm_skinny(a, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_dtyp
     if not gemm_skinny_takes(a, w):
         raise KernelError(f"gemm_skinny: a {tuple(a.shape)} / w {tuple(w.shape)} need few rows, "
                           "K a multiple of 8 and 16-byte aligned rows")
-    return _gemm_skinny(a, w, out, out_dtype, accumulate, bias, emit, col_scale, act)
-
-
-def _gemm_skinny(a, w, out=None, out_dtype=None, accumulate=False, bias=None, emit=None, col_scale=None, act=None):
-    """`gemm_skinny` for the place that has just asked `gemm_skinny_takes` of these two."""
     X, Xf, nw, eps, M, K, ldx, ssq, ssq_parts = _skinny_input(a)
     N = w.shape[0]
     if out is None:
@@ -1215,17 +1210,10 @@ def _gemm_skinny(a, w, out=None, out_dtype=None, accumulate=False, bias=None, em
 def gemm_skinny_swiglu(a, w_gate_up: torch.Tensor, act: str = "silu") -> torch.Tensor:
     """h = act(a W_gate^T) * (a W_up^T) (act one of GATED_EPILOGUES) in one kernel; w_gate_up [2F, K] holds groups of 16 gate
     rows followed by their 16 up rows."""
-    if not gemm_skinny_fused_takes(a, w_gate_up):
-        raise KernelError("gemm_skinny_swiglu: at most 16 rows, K a multiple of 8, 16-byte aligned rows")
-    return _gemm_skinny_swiglu(a, w_gate_up, act)
-
-
-def _gemm_skinny_swiglu(a, w_gate_up, act="silu"):
-    """`gemm_skinny_swiglu` for the place that has just asked `gemm_skinny_fused_takes` of these two."""
     if act not in GATED_EPILOGUES:
         raise KernelError(f"gemm_skinny_swiglu: no gated epilogue with the activation {act!r}")
-    if w_gate_up.shape[0] % 32:
-        raise KernelError("gemm_skinny_swiglu: the weights hold groups of 16 gate rows and 16 up rows")
+    if not gemm_skinny_fused_takes(a, w_gate_up) or w_gate_up.shape[0] % 32:
+        raise KernelError("gemm_skinny_swiglu: at most 16 rows, K a multiple of 8, 16-byte aligned rows")
     X, Xf, nw, eps, M, K, ldx, ssq, ssq_parts = _skinny_input(a)
     F = w_gate_up.shape[0] // 2
     h = torch.empty((M, F), dtype=torch.bfloat16, device=w_gate_up.device)
