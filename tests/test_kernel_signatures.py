@@ -44,7 +44,9 @@ def test_every_exported_launcher_has_a_signature():
         assert exported <= known, f"{cu.name}: {sorted(exported - known)} have no ctypes signature"
 
 
-def test_no_public_contraction_takes_the_callers_word_for_its_checks():
+def test_only_a_private_keyword_lets_a_contraction_take_its_callers_word():
     for fn, names in ((kernels.gemm_skinny, "a w out out_dtype accumulate bias emit col_scale act"),
                       (kernels.gemm_skinny_swiglu, "a w_gate_up act")):
-        assert list(inspect.signature(fn).parameters) == names.split()
+        params = inspect.signature(fn).parameters.values()
+        assert [p.name for p in params if not p.name.startswith("_")] == names.split()
+        assert all(p.kind == p.KEYWORD_ONLY and p.default is False for p in params if p.name.startswith("_"))

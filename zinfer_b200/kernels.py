@@ -1166,14 +1166,15 @@ def gemm_skinny_emits(a, out: Optional[torch.Tensor]) -> bool:
 def gemm_skinny(a, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_dtype=None,
                 accumulate: bool = False, bias: Optional[torch.Tensor] = None,
                 emit: Optional[NormEmit] = None, col_scale: Optional[torch.Tensor] = None,
-                act: Optional[str] = None) -> torch.Tensor:
+                act: Optional[str] = None, *, _taken: bool = False) -> torch.Tensor:
     """out (+)= a @ w.T (+ bias) for a [M <= 64, K] on the tensor cores, every weight read once.
     `act` ("relu_squared") is applied to the sums, then `col_scale` (float32 [N], one number per column)
     multiplies them, before they are stored or added to `out`.
     With a NormInput the RMSNorm of the rows is applied inside the kernel; with a ScaledInput the
     sums are scaled by the rows' 1/rms.  `emit` (see `gemm_skinny_emits`) is filled for the norm
     that reads `out` next."""
-    if not gemm_skinny_takes(a, w):
+    # _taken: the package's own callers that have just asked `gemm_skinny_takes` of these two (2 us of host time a launch)
+    if not _taken and not gemm_skinny_takes(a, w):
         raise KernelError(f"gemm_skinny: a {tuple(a.shape)} / w {tuple(w.shape)} need few rows, "
                           "K a multiple of 8 and 16-byte aligned rows")
     X, Xf, nw, eps, M, K, ldx, ssq, ssq_parts = _skinny_input(a)
@@ -1207,12 +1208,12 @@ def gemm_skinny(a, w: torch.Tensor, out: Optional[torch.Tensor] = None, out_dtyp
     return out
 
 
-def gemm_skinny_swiglu(a, w_gate_up: torch.Tensor, act: str = "silu") -> torch.Tensor:
+def gemm_skinny_swiglu(a, w_gate_up: torch.Tensor, act: str = "silu", *, _taken: bool = False) -> torch.Tensor:
     """h = act(a W_gate^T) * (a W_up^T) (act one of GATED_EPILOGUES) in one kernel; w_gate_up [2F, K] holds groups of 16 gate
     rows followed by their 16 up rows."""
     if act not in GATED_EPILOGUES:
         raise KernelError(f"gemm_skinny_swiglu: no gated epilogue with the activation {act!r}")
-    if not gemm_skinny_fused_takes(a, w_gate_up) or w_gate_up.shape[0] % 32:
+    if not (_taken or gemm_skinny_fused_takes(a, w_gate_up)) or w_gate_up.shape[0] % 32:     # _taken: as in gemm_skinny
         raise KernelError("gemm_skinny_swiglu: at most 16 rows, K a multiple of 8, 16-byte aligned rows")
     X, Xf, nw, eps, M, K, ldx, ssq, ssq_parts = _skinny_input(a)
     F = w_gate_up.shape[0] // 2

@@ -44,7 +44,7 @@ class SwiGLU(FeedForward):
             tc_rows = linear_bf16.TC_SWAPPED_MIN_ROWS <= rows_in <= kernels.gemm_skinny_max_m()
             x = None if tc_rows or self.clamp else fused_input(xn, w, need_fused_rows=True, blocks=self.ffn_dim // 16)
             if x is not None:                       # few rows: gate, up and the activation in one kernel
-                h = kernels.gemm_skinny_swiglu(x, w, act=self.gate_act)
+                h = kernels.gemm_skinny_swiglu(x, w, act=self.gate_act, _taken=True)
             else:
                 x = scaled_or_tensor(xn) if tc_rows else as_tensor(xn)
                 if not kernels.gemm_tc_takes(x, w):

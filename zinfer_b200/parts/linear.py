@@ -106,7 +106,7 @@ def _linear_with_epilogue(a, w, out, out_dtype, accumulate, bias, act):
         x = fused_input(a, w)
         if x is not None:                # few rows: activation and scale in the weight-streaming kernel's epilogue
             return kernels.gemm_skinny(x, w, out=out, out_dtype=out_dtype, accumulate=accumulate, bias=bias,
-                                       col_scale=scale, act=act)
+                                       col_scale=scale, act=act, _taken=True)
     if w.dtype == torch.bfloat16 and (act is None or act == "relu_squared") and a.shape[0] > kernels.GEMM_TC_SWAPPED_MAX_M:
         t = as_tensor(a)
         if kernels.gemm_tc_fuses(t, w, out, accumulate, out_dtype):   # many rows: the persistent tcgen05 forms' epilogue

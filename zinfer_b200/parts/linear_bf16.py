@@ -53,7 +53,7 @@ def try_linear(a, w, out, out_dtype, accumulate, bias, sink=None):
         emit = None
         if sink is not None and kernels.gemm_skinny_emits(x, out):
             emit = kernels.NormEmit(sink.norm_weight)
-        y = kernels.gemm_skinny(x, w, out=out, out_dtype=out_dtype, accumulate=accumulate, bias=bias, emit=emit)
+        y = kernels.gemm_skinny(x, w, out=out, out_dtype=out_dtype, accumulate=accumulate, bias=bias, emit=emit, _taken=True)
         if emit is not None:
             sink.emit = emit
         return y
