@@ -38,6 +38,21 @@ def k():
     return kernels
 
 
+def test_what_the_tensor_check_takes_and_refuses(k):
+    t = torch.zeros((3, 4), device="cuda")
+    for good in (dict(), dict(dtype=torch.float32), dict(dtype=(torch.bfloat16, torch.float32)), dict(dtype=[torch.float32]),
+                 dict(shape=(3, 4)), dict(shape=[3, 4]), dict(shape=(None, 4)), dict(shape=t.shape), dict(shape=(None, None))):
+        k._need(t, "t", **good)
+    k._need(t.T, "t", torch.float32, (4, 3), contiguous=False)
+    for bad in (dict(dtype=torch.bfloat16), dict(dtype=(torch.bfloat16, torch.int32)), dict(shape=(3,)), dict(shape=(3, 4, 1)),
+                dict(shape=(4, 3)), dict(shape=(None, 5)), dict(shape=())):
+        with pytest.raises(k.KernelError):
+            k._need(t, "t", **bad)
+    for other in (t.T, t.cpu(), None, 3.0):
+        with pytest.raises(k.KernelError):
+            k._need(other, "t")
+
+
 # ------------------------------------------------------------------------------- row kernels
 
 @pytest.mark.parametrize("dtype", DTYPES)
