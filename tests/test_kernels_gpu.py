@@ -1100,3 +1100,70 @@ def test_gemm_tc_gated_units_over_the_whole_range(k, M, splits, glu):
     rel = 2 ** -8 + 8 * 2 ** -23 + (arg.abs() * 2 ** -23 if glu == "clamp" else 0)
     bound = torch.where(arg < -88.7, ref.abs(), ref.abs() * rel + 2.0 ** -134)
     assert (err <= bound[:, None]).all()
+
+
+@pytest.mark.parametrize("D,F,E,top,n", [(64, 48, 5, 2, 1), (72, 40, 3, 3, 8), (2048, 24, 4, 2, 9), (256, 2048, 16, 2, 64), (520, 264, 6, 4, 33),
+                                         (48, 1032, 130, 8, 16), (128, 64, 2, 1, 129), (64, 32, 40, 33, 5)])
+@pytest.mark.parametrize("kind", ["table", "routed", "ungated", "weight_in"])
+def test_experts_of_few_rows(k, D, F, E, top, n, kind):
+    """The bfloat16 kernels that read an expert's weights once for all of its rows: output units beyond the last 16, K of no whole
+    32 and less than a step per warp, clusters of 1 to 8, experts with no row, one, more than 8 and more than 16, tokens cut at
+    128 pairs, identity experts, a table that names an expert twice.  The bound: two float32 sums (K 2^-23 of the absolute
+    terms), the unit's slope of at most 1.1 and its own few ulp, one rounding of h to bfloat16 (2^-8)."""
+    g = torch.Generator().manual_seed(D + F + n)
+    x, gated = rnd((n, D), 1, torch.bfloat16), kind != "ungated"
+    il = 16 if F % 16 == 0 and kind in ("table", "weight_in") else 0
+    gate, up = rnd((E, F, D), 2, torch.bfloat16, D ** -0.5), rnd((E, F, D), 3, torch.bfloat16, D ** -0.5)
+    down = rnd((E, D, F), 4, torch.bfloat16, F ** -0.5)
+    ident = 3 if kind == "routed" else 0
+    ids = torch.stack([torch.randperm(E + ident, generator=g)[:top] for _ in range(n)]).int()
+    ids[: n // 2, 0] = 1                                   # an expert with many rows
+    if kind == "table":
+        ids[-1] = 0                                        # one expert for all of a token's places
+    else:
+        for i in range(n // 2):
+            ids[i, 1:][ids[i, 1:] == 1] = 0
+    wts = torch.rand((n, top), generator=g) + 0.1
+    if not gated:
+        w1 = up
+    elif il:
+        w1 = torch.stack([gate.view(E, F // il, il, D), up.view(E, F // il, il, D)], 2).reshape(E, 2 * F, D)
+    else:
+        w1 = torch.cat([gate, up], 1)
+    old = rnd((n, D), 5, torch.float32)
+    status = k.status_word("cuda")
+
+    def call(lo, hi, out):
+        xs, w = x[lo:hi].cuda(), wts[lo:hi].cuda()
+        if kind == "table":
+            toks = torch.arange(lo, hi, dtype=torch.int32).cuda()
+            return k.moe_table(xs, toks, ids.cuda(), w1.cuda(), il, down.cuda(), status, out=out, accumulate=True)
+        return k.moe_routed(xs, ids[lo:hi].cuda(), w, w1.cuda(), il, down.cuda(), status, out=out, accumulate=True, n_identity=ident,
+                            act=None if gated else "relu_squared", weight_input=kind == "weight_in")
+
+    got = call(0, n, old.clone().cuda())
+    ref, bound = old.double().clone(), 2.0 ** -23 * old.double().abs()
+    for t in range(n):
+        for j in range(top):
+            e, w = int(ids[t, j]), (1.0 / top if kind == "table" else float(wts[t, j]))
+            xt = x[t].double()
+            if e >= E:
+                ref[t] += w * xt
+                bound[t] += 2.0 ** -22 * (w * xt).abs()
+                continue
+            wi, wo = (w, 1.0) if kind == "weight_in" else (1.0, w)
+            zu, eu = wi * (up[e].double() @ xt), (D + 2) * 2.0 ** -23 * wi * (up[e].double().abs() @ xt.abs())
+            if gated:
+                zg, eg = wi * (gate[e].double() @ xt), (D + 2) * 2.0 ** -23 * wi * (gate[e].double().abs() @ xt.abs())
+                s = zg * torch.sigmoid(zg)
+                h, eh = s * zu, 1.1 * eg * (zu.abs() + eu) + s.abs() * eu
+            else:
+                h = torch.relu(zu) ** 2
+                eh = 2 * zu.abs() * eu + eu ** 2
+            eh = eh + (2.0 ** -8 + 2.0 ** -19) * h.abs()
+            ref[t] += wo * (down[e].double() @ h)
+            bound[t] += wo * (down[e].double().abs() @ (eh + (F + 4) * 2.0 ** -23 * (h.abs() + eh)))
+    assert ((got.double().cpu() - ref).abs() <= bound).all()
+    assert int(status.item()) == 0
+    for i in sorted({0, n // 2, n - 1}):                  # a token's result is the same bits alone
+        assert torch.equal(call(i, i + 1, old[i:i + 1].clone().cuda())[0], got[i])

@@ -1,10 +1,11 @@
 // Mixture of small gated feed-forwards whose experts are picked by a TABLE indexed with the token id
 // (no router): token t uses experts table[token_t][0 .. top), each with weight 1/top.
 //   y_t = (1/top) * sum_k W_down[e_k] (silu(W_gate[e_k] x_t) * (W_up[e_k] x_t))
-// Two weight-streaming kernels.  (1) gate/up: one block per (token, k) and slice of the expert's
-// hidden units; a warp owns a hidden unit at a time, its lanes walk the input row, sums in float32,
-// silu in float32.  (2) down: one block per token and slice of the outputs; the `top` experts are
-// added in the order of k, so a token's result does not depend on the rest of the batch.
+// Two weight-streaming kernels, for float32 and for rows that come in no 16-byte pieces.  (1) gate/up: one block per
+// (token, k) and slice of the expert's hidden units; a warp owns a hidden unit at a time, its lanes walk the input row, sums
+// in float32, silu in float32.  (2) down: one block per token and slice of the outputs; the `top` experts are
+// added in the order of k, so a token's result does not depend on the rest of the batch.  bfloat16 rows in such pieces take
+// expert_rows_kernel instead, which reads an expert's weights once for all of its rows.
 // Weights are stacked in the run dtype: gate and up as ONE tensor [experts, 2F, D] whose rows are
 // [gate (F) | up (F)] (il = 0) or groups of il gate rows followed by their il up rows (il > 0, the layout
 // the contraction kernels with an activation epilogue want), down as [experts, D, F]; x and h are the run
@@ -211,6 +212,287 @@ __global__ void __launch_bounds__(MOE_WARPS * 32)
   }
 }
 
+namespace {
+
+// ------------------------------------------------------------------------------ experts of few rows, bfloat16
+// The two kernels above read an expert's matrix once per (token, expert) PAIR.  What bounds a step of few tokens is reading
+// each matrix once from memory, so here a block owns 16 output units (hidden units, or outputs) of EVERY expert: it sorts
+// the step's pairs by expert in shared memory, walks the experts that have any, reads 16 rows of each once, straight into the
+// fragments of mma.m16n8k16, and multiplies them with up to 16 of the expert's rows (8 to a fragment).  The products of
+// bfloat16 values are exact and the sums float32, as before.  A lane takes 16 contiguous bytes of a weight row and of an
+// input row for two MMAs; both use the same order of k inside 32, which a sum does not see.  K is split over the block's
+// warps and over the blocks of a cluster, so that all SMs stream whatever the sizes; the loads of the next expert are under way
+// while this one is multiplied (a ring of registers that runs on across experts).  All partial sums wait in shared
+// memory and are added in the order of warps, then of blocks; a result depends on K and the cluster's size alone, which the
+// sizes of the model decide: not on the step's other tokens.  Everything a token needs is in one cluster, so its experts are
+// added in the order of k without another kernel.
+// 8 tokens with 2 of 16 experts each (10 different ones), D = F = 2048, one layer of a single-token step, microseconds before and
+// now: gate/up 50 -> 37 (174 MB of weights: 4.7 TB/s), both kernels 102 -> 71; the step 1.00 -> 0.79 ms.
+constexpr int PAIRS_MAX = 128;       // pairs a cluster takes (tokens are cut into grid.y chunks of PAIRS_MAX / top)
+
+enum { EXPERT_GATED = 0, EXPERT_UNGATED = 1, EXPERT_DOWN = 2 };
+
+struct ExpertArgs {
+  const bf16* x;             // UP: [n, D] the rows the experts read; DOWN: the same, for identity experts
+  const bf16* h_in;          // DOWN: [n, top, F]
+  bf16* h_out;               // UP: [n, top, F]
+  float* y;                  // DOWN: [n, D]
+  const int* tokens;
+  const int* table;
+  const bf16* w;
+  const float* route_w;      // DOWN: weight of each pair, or null
+  const float* in_w;         // UP: weight of each pair's input, or null
+  int* status;
+  int n, D, F, top, vocab, n_experts, n_ident, il, act, accumulate, chunk;   // chunk: tokens per cluster
+  float weight;
+};
+
+__device__ __forceinline__ uint4 ld_weights(const bf16* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+
+__device__ __forceinline__ void mma_bf16(float c[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+__device__ __forceinline__ float ld_cluster(const float* local, unsigned rank) {
+  unsigned remote;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int TILES> constexpr int EXPERT_LD = TILES * 16 + 4;   // floats per pair and warp: adjacent pairs' rows in other banks
+
+// NG: groups of 8 input rows multiplied at once (1 where no expert can have more than 8 pairs); RING: loads of 32 k under way.
+// Shared memory: PAIRS_MAX ints each of experts by pair, pairs in sorted order, places by pair, walks; then the partial
+// sums [warp][pair in sorted order][row of the tiles].
+template <int MODE, int NG, int RING>
+__global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const ExpertArgs a) {
+  constexpr int TILES = MODE == EXPERT_GATED ? 2 : 1, LD = EXPERT_LD<TILES>;
+  extern __shared__ __align__(16) float ex_smem[];
+  int* pair_expert = reinterpret_cast<int*>(ex_smem);
+  int* sorted = pair_expert + PAIRS_MAX;
+  int* place = sorted + PAIRS_MAX;
+  int* walks = place + PAIRS_MAX;                  // first place of each walk
+  int* n_walks_p = walks + PAIRS_MAX;
+  float* part = ex_smem + 4 * PAIRS_MAX + 4;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, c = lane & 3;
+  unsigned rank, ranks;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+  const int unit0 = (int)(blockIdx.x / ranks) * 16;
+  const int K = MODE == EXPERT_DOWN ? a.F : a.D, units = MODE == EXPERT_DOWN ? a.D : a.F;
+  const int t0 = blockIdx.y * a.chunk, n_pairs = min(a.chunk, a.n - t0) * a.top;
+  zk_let_next_start();
+  zk_wait_prior();
+
+  // the pairs sorted by expert, each expert's in their own order; identity experts' pairs behind all others
+  for (int i = tid; i < n_pairs; i += MOE_WARPS * 32) {
+    const int t = t0 + i / a.top, k = i % a.top;
+    int e, bound = a.n_experts;
+    if (!a.tokens) {
+      e = a.table[(size_t)t * a.top + k];
+      bound += a.n_ident;
+    } else {
+      int tok = a.tokens[t];
+      if (tok < 0 || tok >= a.vocab) tok = 0;      // the embedding kernel has flagged it
+      e = a.table[(size_t)tok * a.top + k];
+    }
+    if (e < 0 || e >= bound) {
+      atomicExch(a.status, 4);
+      e = 0;
+    }
+    pair_expert[i] = e;
+  }
+  __syncthreads();
+  for (int i = tid; i < n_pairs; i += MOE_WARPS * 32) {
+    const int e = pair_expert[i];
+    int p = 0;
+    for (int j = 0; j < n_pairs; ++j) p += pair_expert[j] < e || (pair_expert[j] == e && j < i);
+    sorted[p] = i;
+    place[i] = p;
+  }
+  __syncthreads();
+  if (warp == 0) {           // a walk begins at every 8 NG-th pair of an expert
+    int n_walks = 0;
+    for (int base = 0; base < n_pairs; base += 32) {
+      const int p = base + lane;
+      bool head = false;
+      if (p < n_pairs) {
+        const int i = sorted[p], e = pair_expert[i];
+        if (e < a.n_experts) {
+          int before = 0;    // pairs of the same expert in front of this one
+          while (before < p && pair_expert[sorted[p - before - 1]] == e) ++before;
+          head = before % (8 * NG) == 0;
+        }
+      }
+      const unsigned heads = __ballot_sync(0xffffffffu, head);
+      if (head) walks[n_walks + __popc(heads & ((1u << lane) - 1))] = p;
+      n_walks += __popc(heads);
+    }
+    if (lane == 0) *n_walks_p = n_walks;
+  }
+  __syncthreads();
+  const int n_walks = *n_walks_p;
+
+  // this warp's stretch of K, in steps of 32
+  const int steps = (K + 31) / 32, shares = (int)ranks * MOE_WARPS, share = (int)rank * MOE_WARPS + warp;
+  const int s0 = steps * share / shares, s1 = steps * (share + 1) / shares;
+
+  struct Stage { uint4 w[TILES][2], x[NG]; };
+  Stage ring[RING];
+  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+  // the fetching walk: its expert's rows of this lane, and the input rows of this lane's columns
+  int fetch_walk = 0, fetch_s = s0;
+  const bf16* wrow[TILES][2];
+  const bf16* xrow[NG];
+  bool wok[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) wok[h] = unit0 + g + 8 * h < units;
+  auto enter = [&](int walk) {
+    const int first = walks[walk], e = pair_expert[sorted[first]];
+    const bf16* base = a.w + (size_t)e * (MODE == EXPERT_GATED ? 2 : 1) * units * K;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int f = wok[h] ? unit0 + g + 8 * h : 0;
+      if constexpr (MODE == EXPERT_GATED) {
+        const int grow = a.il ? (f / a.il) * 2 * a.il + f % a.il : f;
+        wrow[0][h] = base + (size_t)grow * K;
+        wrow[TILES - 1][h] = base + (size_t)(a.il ? grow + a.il : a.F + f) * K;
+      } else {
+        wrow[0][h] = base + (size_t)f * K;
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < NG; ++t) {
+      const int p = first + t * 8 + g;
+      xrow[t] = nullptr;
+      if (p < n_pairs && pair_expert[sorted[p]] == e) {
+        const int i = sorted[p];
+        xrow[t] = MODE == EXPERT_DOWN ? a.h_in + ((size_t)t0 * a.top + i) * K : a.x + (size_t)(t0 + i / a.top) * K;
+      }
+    }
+  };
+  auto fetch = [&](Stage& st) {
+    if (fetch_walk >= n_walks) return;
+    if (fetch_s == s0) enter(fetch_walk);
+    const int k = fetch_s * 32 + 8 * c;
+    const bool in = k < K;                         // K % 8 == 0: a piece is all in or all out
+#pragma unroll
+    for (int t = 0; t < TILES; ++t)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) st.w[t][h] = in && wok[h] ? ld_weights(wrow[t][h] + k) : zero;
+#pragma unroll
+    for (int t = 0; t < NG; ++t) st.x[t] = in && xrow[t] ? *reinterpret_cast<const uint4*>(xrow[t] + k) : zero;
+    if (++fetch_s == s1) {
+      fetch_s = s0;
+      ++fetch_walk;
+    }
+  };
+
+  if (s0 < s1) {
+#pragma unroll
+    for (int r = 0; r < RING; ++r) fetch(ring[r]);
+    float acc[TILES][NG][4];
+#pragma unroll
+    for (int t = 0; t < TILES; ++t)
+#pragma unroll
+      for (int u = 0; u < NG; ++u)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[t][u][j] = 0.f;
+    int walk = 0, s = s0;
+    while (walk < n_walks) {
+#pragma unroll
+      for (int r = 0; r < RING; ++r) {
+        if (walk >= n_walks) break;
+        const Stage& st = ring[r];
+#pragma unroll
+        for (int t = 0; t < TILES; ++t)
+#pragma unroll
+          for (int u = 0; u < NG; ++u) {
+            mma_bf16(acc[t][u], st.w[t][0].x, st.w[t][1].x, st.w[t][0].y, st.w[t][1].y, st.x[u].x, st.x[u].y);
+            mma_bf16(acc[t][u], st.w[t][0].z, st.w[t][1].z, st.w[t][0].w, st.w[t][1].w, st.x[u].z, st.x[u].w);
+          }
+        fetch(ring[r]);
+        if (++s < s1) continue;
+        // this warp's share of the walk: rows g and g + 8 of each tile, columns 2c and 2c + 1 of each 8
+        const int first = walks[walk], last = walk + 1 < n_walks ? walks[walk + 1] : n_pairs;
+#pragma unroll
+        for (int u = 0; u < NG; ++u)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int p = first + u * 8 + 2 * c + (j & 1);
+#pragma unroll
+            for (int t = 0; t < TILES; ++t) {
+              if (p < last) part[((size_t)warp * n_pairs + p) * LD + t * 16 + g + 8 * (j >> 1)] = acc[t][u][j];
+              acc[t][u][j] = 0.f;
+            }
+          }
+        s = s0;
+        ++walk;
+      }
+    }
+  } else {                                         // fewer steps than warps: nothing of K is this warp's
+    for (int i = lane; i < n_pairs * LD; i += 32) part[(size_t)warp * n_pairs * LD + i] = 0.f;
+  }
+  __syncthreads();
+  for (int i = tid; i < n_pairs * TILES * 16; i += MOE_WARPS * 32) {
+    const int at = i / (TILES * 16) * LD + i % (TILES * 16);
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < MOE_WARPS; ++w) v += part[(size_t)w * n_pairs * LD + at];
+    part[at] = v;
+  }
+  cluster_barrier();
+  auto sum = [&](int pair, int row) {
+    const float* p = part + place[pair] * LD + row;
+    float v = 0.f;
+    for (unsigned r = 0; r < ranks; ++r) v += ld_cluster(p, r);
+    return v;
+  };
+  if constexpr (MODE != EXPERT_DOWN) {
+    for (int i = rank * MOE_WARPS * 32 + tid; i < n_pairs * 16; i += ranks * MOE_WARPS * 32) {
+      const int pair = i / 16, f = i % 16;
+      if (unit0 + f >= units || pair_expert[pair] >= a.n_experts) continue;
+      const size_t at = (size_t)t0 * a.top + pair;
+      const float wi = a.in_w ? a.in_w[at] : 1.0f;
+      const float z = wi * sum(pair, f);
+      float v;
+      if constexpr (MODE == EXPERT_GATED) v = z / (1.0f + expf(-z)) * (wi * sum(pair, 16 + f));
+      else v = zk_activate(z, a.act);
+      a.h_out[at * a.F + unit0 + f] = __float2bfloat16_rn(v);
+    }
+  } else {
+    for (int i = rank * MOE_WARPS * 32 + tid; i < n_pairs / a.top * 16; i += ranks * MOE_WARPS * 32) {
+      const int t = i / 16, d = unit0 + i % 16;
+      if (d >= units) continue;
+      float v = 0.f;
+      for (int k = 0; k < a.top; ++k) {
+        const int pair = t * a.top + k;
+        const float wk = a.route_w ? a.route_w[(size_t)t0 * a.top + pair] : a.weight;
+        v += wk * (pair_expert[pair] >= a.n_experts ? to_f32(a.x[(size_t)(t0 + t) * a.D + d]) : sum(pair, i % 16));
+      }
+      float* dst = a.y + (size_t)(t0 + t) * a.D + d;
+      *dst = a.accumulate ? *dst + v : v;
+    }
+  }
+  cluster_barrier();         // nobody leaves while its partial sums may still be read
+}
+
+}  // namespace
+
 template <typename T>
 __global__ void moe_gather_kernel(const T* __restrict__ x, const int* __restrict__ row_token, T* __restrict__ xg, int D,
                                   const float* __restrict__ pair_w, int top) {
@@ -401,6 +683,42 @@ __global__ void __launch_bounds__(MOE_WARPS * 32)
 
 namespace {
 
+// Blocks of a cluster over which K is split: as many as give two blocks to (nearly) every SM, while every warp has 32 k or
+// more.  The model's sizes alone decide, so that a token's sums are the same in every step.
+int expert_split(int units, int K) {
+  const int slices = ceil_div_i(units, 16), steps = ceil_div_i(K, 32);
+  int split = 1;
+  while (split < 8 && slices * split < 200 && steps >= 2 * split * MOE_WARPS) split *= 2;
+  return split;
+}
+
+template <int MODE, int NG, int RING>
+int launch_experts(const ExpertArgs& a, cudaStream_t stream) {
+  const int units = MODE == EXPERT_DOWN ? a.D : a.F, K = MODE == EXPERT_DOWN ? a.F : a.D;
+  constexpr size_t HEAD = sizeof(float) * (4 * PAIRS_MAX + 4);
+  constexpr size_t PAIR = sizeof(float) * MOE_WARPS * EXPERT_LD<MODE == EXPERT_GATED ? 2 : 1>;
+  // The limit is shared by all threads of the process: always what the most pairs need.
+  cudaError_t e = cudaFuncSetAttribute(expert_rows_kernel<MODE, NG, RING>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(HEAD + PAIR * PAIRS_MAX));
+  if (e != cudaSuccess) return (int)e;
+  const int split = expert_split(units, K);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ceil_div_i(units, 16) * split, ceil_div_i(a.n, a.chunk));
+  cfg.blockDim = dim3(MOE_WARPS * 32);
+  cfg.dynamicSmemBytes = HEAD + PAIR * (size_t)(a.n < a.chunk ? a.n : a.chunk) * a.top;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = split;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return (int)cudaLaunchKernelEx(&cfg, expert_rows_kernel<MODE, NG, RING>, a);
+}
+
 template <typename T>
 int launch_moe(const void* x, const int* tokens, const int* table, const void* w_gu, int il,
                const void* w_down, void* h, float* y, int n, int D, int F, int top, int vocab, int n_experts,
@@ -409,6 +727,10 @@ int launch_moe(const void* x, const int* tokens, const int* table, const void* w
   auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   const bool vec_gu = D % 8 == 0 && D % per == 0 && aligned(w_gu);
   const bool vec_dn = F % 8 == 0 && F % per == 0 && aligned(w_down);
+  // Rows of bfloat16 in 16-byte pieces: each expert's matrix is read once per chunk of tokens.  Otherwise (float32, whose sums
+  // stay chains of float32 FMAs, and sizes or addresses without such pieces) once per pair.
+  const bool by_expert = sizeof(T) == 2 && top <= PAIRS_MAX;
+  const bool up_by_expert = by_expert && vec_gu && aligned(x), down_by_expert = by_expert && vec_dn && aligned(h);
   // enough blocks to fill the GPU when the tokens are few, whole experts per block when they are many
   int units = F, outs = D;
   const long long pairs = (long long)n * top;
@@ -443,13 +765,30 @@ int launch_moe(const void* x, const int* tokens, const int* table, const void* w
                              (const T*)w_down, y, D, F, top, vocab, n_experts, outs, accumulate, status, route_w,     \
                              n_ident, (const T*)x, in_w ? 1.0f : 1.0f / (float)top);                                  \
   } while (0)
-  if (act < 0) {
+  ExpertArgs ea{};
+  ea.x = (const bf16*)x; ea.h_in = (const bf16*)h; ea.h_out = (bf16*)h; ea.y = y; ea.tokens = tokens; ea.table = table;
+  ea.w = (const bf16*)w_gu; ea.route_w = route_w; ea.in_w = in_w; ea.status = status;
+  ea.n = n; ea.D = D; ea.F = F; ea.top = top; ea.vocab = vocab; ea.n_experts = n_experts; ea.n_ident = n_ident; ea.il = il;
+  ea.act = act; ea.accumulate = accumulate; ea.weight = in_w ? 1.0f : 1.0f / (float)top;
+  ea.chunk = by_expert ? PAIRS_MAX / top : 0;
+  const bool few = n <= 8;         // then no expert has more than 8 rows (unless a table names one twice: another walk)
+  if (up_by_expert) {
+    if (act < 0) rc = few ? launch_experts<EXPERT_GATED, 1, 3>(ea, stream) : launch_experts<EXPERT_GATED, 2, 2>(ea, stream);
+    else rc = few ? launch_experts<EXPERT_UNGATED, 1, 6>(ea, stream) : launch_experts<EXPERT_UNGATED, 2, 4>(ea, stream);
+  } else if (act < 0) {
     if (vec_gu) ZK_MOE_GU(true, true); else ZK_MOE_GU(false, true);
   } else {
     if (vec_gu) ZK_MOE_GU(true, false); else ZK_MOE_GU(false, false);
   }
   if (rc != 0) return rc;
-  if (vec_dn) ZK_MOE_DN(true); else ZK_MOE_DN(false);
+  if (down_by_expert) {
+    ea.w = (const bf16*)w_down;
+    rc = few ? launch_experts<EXPERT_DOWN, 1, 6>(ea, stream) : launch_experts<EXPERT_DOWN, 2, 4>(ea, stream);
+  } else if (vec_dn) {
+    ZK_MOE_DN(true);
+  } else {
+    ZK_MOE_DN(false);
+  }
   return rc;
 #undef ZK_MOE_GU
 #undef ZK_MOE_DN
