@@ -241,3 +241,38 @@ def test_repetition_penalty_from_the_window_on_the_device(k):
         for r, t in zip(rows, toks.tolist()):
             hist[r].append(t)
     assert seen.cpu().tolist() == [len(h) for h in hist] and max(len(h) for h in hist) > W
+
+
+@pytest.mark.parametrize("V", [8191, 8192, 8200, 20004, 32768, 65536, 65541, 131080])
+@pytest.mark.parametrize("opts", [dict(temp=0.8, top_k=40, top_p=0.95, min_p=0.05), dict(temp=1.0, top_k=1), dict(temp=0.7, top_k=1024),
+                                  dict(temp=1.1, top_p=0.4), dict(temp=1.0, top_k=3, xtc_probability=1.0, xtc_threshold=0.1)])
+def test_rows_cut_over_a_cluster(k, V, opts):
+    """Rows from 8,192 logits on are read by a cluster: lengths that leave the last pieces short, rows that do not begin on 16 bytes,
+    the best tokens in one piece or at both ends of every piece, ties across pieces, NaN, a row of one value (too many ties
+    for the list), a row of -inf.  Against the plain chain, and the same row alone."""
+    n = 12
+    x = logits_rows(n, V, V + 1)
+    per = ((V + 7) // 8 + 3) // 4 * 4
+    x[0, :50] += 20.0
+    x[1, V - 50:] += 20.0
+    x[2, [i * per for i in range(8)] + [min(V, (i + 1) * per) - 1 for i in range(8)]] = 17.0
+    x[3, ::7] = np.nan
+    x[4] = 1.25
+    x[5] = -np.inf
+    x[5, V // 2:V // 2 + 4] = 0.5
+    u = np.random.default_rng(4).random((n, 2)).astype(np.float32)
+    dev, du = torch.from_numpy(x).cuda(), torch.from_numpy(u).cuda()
+    got = k.sample(dev, du, **opts).cpu().numpy()
+    exact = 0
+    for i in range(n):
+        row = np.where(np.isnan(x[i]), -np.inf, x[i]).astype(np.float32)
+        if "xtc_probability" not in opts:
+            p = P.filtered_probs(row, opts["temp"], opts.get("top_k", 0), opts.get("top_p", 1.0), opts.get("min_p", 0.0))
+            assert p[got[i]] > 0, f"row {i}: token {got[i]}"
+            exact += int(got[i] == expected_pick(p, float(u[i, 0])))
+        else:
+            best = np.argsort(-row, kind="stable")[:3]
+            assert got[i] in best, f"row {i}: token {got[i]}"
+            exact += 1
+        assert int(k.sample(dev[i:i + 1].clone(), du[i:i + 1], **opts)) == got[i]
+    assert exact >= n - 1

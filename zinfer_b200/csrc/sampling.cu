@@ -1,4 +1,4 @@
-// Sampling on the device, one thread block per row of float32 logits [n, V].
+// Sampling on the device, one thread block (a cluster of 8 for long rows) per row of float32 logits [n, V].
 //
 // The reference's chain (src/sampler.zig:36-37, 190-276): repetition penalty, DRY penalty,
 // greedy if temp <= 0, else top-k, top-p and min-p on untempered probabilities relative to the
@@ -422,120 +422,190 @@ __device__ __forceinline__ float counter_uniform(unsigned long long seed, int re
 // at or above the bin in which the k-th best lies) and the rest of the chain runs on that list
 // in shared memory: the same prefixes, ties, predicates and index-order draw as the passes over
 // the whole row further down, at a tenth of their time.
+//
+// A row is one chain of waits, and one SM needed most of it for the two passes: 65,536 additions to a few dozen busy
+// words of shared memory, 64 loads a thread.  So the blocks of a cluster take a piece of the row each: every block adds up the
+// cluster's histograms for itself, gathers its piece's candidates, and block 0 fetches the lists and goes on alone.  Which
+// tokens are candidates, and every sum over them, is what one block made of the whole row: the same bits.
+// Temperature, top-k 40, top-p and min-p over 8 rows of 65,536 logits, microseconds: 35.7 -> 20.0.
 constexpr int CAND_MAX = 1024;
 constexpr int HIST_BITS = 11, HIST_BINS = 1 << HIST_BITS;
 
-struct Small {
+struct __align__(16) Small {
   float l[CAND_MAX];       // candidates in index order
   int idx[CAND_MAX];
   float l2[CAND_MAX];      // as gathered
   int idx2[CAND_MAX];
   float w[CAND_MAX];       // masses exp(l - mx), then weights exp((l - mx) / temp)
-  unsigned char in[CAND_MAX];
+  unsigned key[CAND_MAX];  // of l
+  int order[CAND_MAX];     // places in the descending order
   int hist[HIST_BINS];
-  int count, bin, above;
+  int warp_sum[32];
+  int count, bin, n_c;       // what this block gathered; the deciding bin; candidates of the whole row
 };
 
-// Returns false, with nothing decided, if the list does not suffice; the caller then takes the
-// passes over the whole row.  k_eff: how many of the best the top-k stage keeps (V if it is off).
-__device__ bool sample_small(const float* row, int V, int k_eff, float temp, float top_p, float min_p,
-                             float xtc_probability, float xtc_threshold, int xtc_min_keep, float u_draw, float u_xtc,
-                             Shared& sh, Small& sm, int* picked_out) {
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int k_list = min(k_eff, CAND_MAX);           // the list holds the k_list best
-  // 1. histogram of the upper bits; equal bins of a warp are added as one
-  for (int b = tid; b < HIST_BINS; b += blockDim.x) sm.hist[b] = 0;
+__device__ __forceinline__ int ld_cluster(const int* local, unsigned rank) {
+  unsigned remote;
+  int v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(rank));
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
+  return v;
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// f(i, value) for the elements of [lo, hi); eight loads under way per thread.  vec: row + lo is 16-byte aligned.
+template <typename F>
+__device__ __forceinline__ void walk_piece(const float* row, int lo, int hi, bool vec, F f) {
+  const int tid = threadIdx.x;
+  for (int base = lo; base < hi; base += SAMP_THREADS * 8) {
+    float4 q[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = base + (u * SAMP_THREADS + tid) * 4;
+      if (vec && i + 3 < hi) {
+        q[u] = *reinterpret_cast<const float4*>(row + i);
+      } else {
+        q[u].x = i < hi ? row[i] : 0.f;
+        q[u].y = i + 1 < hi ? row[i + 1] : 0.f;
+        q[u].z = i + 2 < hi ? row[i + 2] : 0.f;
+        q[u].w = i + 3 < hi ? row[i + 3] : 0.f;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = base + (u * SAMP_THREADS + tid) * 4;
+      if (i < hi) f(i, q[u].x);
+      if (i + 1 < hi) f(i + 1, q[u].y);
+      if (i + 2 < hi) f(i + 2, q[u].z);
+      if (i + 3 < hi) f(i + 3, q[u].w);
+    }
+  }
+}
+
+// The candidates of a row, all that lie at or above the bin of the k_list-th best, in block 0's l2 and idx2 (in any order);
+// returns their number in block 0, 0 in the others, or more than CAND_MAX, with no list, in all of them if too many values
+// share the deciding bin.  Every block of the cluster calls it.
+__device__ __forceinline__ int gather_candidates(const float* row, int V, int k_list, Small& sm) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned rank, ranks;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+  const int per = ((V + (int)ranks - 1) / (int)ranks + 3) & ~3;
+  const int lo = min(V, (int)rank * per), hi = min(V, lo + per);
+  const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+  // 1. histogram of the upper bits
+  for (int b = tid; b < HIST_BINS; b += SAMP_THREADS) sm.hist[b] = 0;
   if (tid == 0) sm.count = 0;
   __syncthreads();
-  // (sixteen loads under way per thread: one at a time, a pass over the row is its latency 64 times)
-  constexpr int UN = 16;
-  for (int base = 0; base < V; base += blockDim.x * UN) {
-    float v[UN];
+  walk_piece(row, lo, hi, vec, [&](int, float v) { atomicAdd(&sm.hist[key_of(v) >> (32 - HIST_BITS)], 1); });
+  cluster_barrier();
+  // 2. the bin of the k_list-th best.  Thread t owns bins top - 1 and top - 2 with top = HIST_BINS - 2 t: the scan over the
+  //    threads runs down the values.
+  static_assert(HIST_BINS == 2 * SAMP_THREADS, "two bins per thread");
+  const int top = HIST_BINS - 2 * tid;
+  int upper = 0, lower = 0;
+  for (unsigned r = 0; r < ranks; ++r) {
+    upper += ld_cluster(&sm.hist[top - 1], r);
+    lower += ld_cluster(&sm.hist[top - 2], r);
+  }
+  int incl = upper + lower;
 #pragma unroll
-    for (int u = 0; u < UN; ++u) {
-      const int i = base + u * blockDim.x + tid;
-      v[u] = i < V ? row[i] : 0.f;
-    }
+  for (int o = 1; o < 32; o <<= 1) {
+    const int n = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += n;
+  }
+  if (lane == 31) sm.warp_sum[warp] = incl;
+  __syncthreads();
+  int before_warp = lane < warp ? sm.warp_sum[lane] : 0;
 #pragma unroll
-    for (int u = 0; u < UN; ++u)
-      if (base + u * blockDim.x + tid < V) atomicAdd(&sm.hist[key_of(v[u]) >> (32 - HIST_BITS)], 1);
+  for (int o = 16; o > 0; o >>= 1) before_warp += __shfl_xor_sync(0xffffffffu, before_warp, o);
+  incl += before_warp;
+  const int before = incl - upper - lower;             // elements in bins above this thread's
+  if (before < k_list && incl >= k_list) {             // exactly one thread (V >= k_list elements exist)
+    const bool in_upper = before + upper >= k_list;
+    sm.bin = in_upper ? top - 1 : top - 2;
+    sm.n_c = before + upper + (in_upper ? 0 : lower);
   }
   __syncthreads();
-  // 2. the bin of the k_list-th best: warp 0, lane j owns bins [HIST_BINS - 64 (j + 1), HIST_BINS - 64 j)
-  if (tid < 32) {
-    constexpr int PER = HIST_BINS / 32;
-    const int top = HIST_BINS - PER * lane;           // one past this lane's highest bin
-    int mine = 0;
-    for (int b = top - 1; b >= top - PER; --b) mine += sm.hist[b];
-    int incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int n = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += n;
-    }
-    const int before = incl - mine;                    // elements in bins above this lane's
-    if (before < k_list && incl >= k_list) {           // exactly one lane (V >= k_list elements exist)
-      int acc = before, b = top - 1;
-      for (; b > top - PER; --b) {
-        if (acc + sm.hist[b] >= k_list) break;
-        acc += sm.hist[b];
-      }
-      sm.bin = b;
-      sm.above = acc;
-    }
-  }
-  __syncthreads();
-  const int bin0 = sm.bin;
-  const int n_c = sm.above + sm.hist[bin0];
-  if (n_c > CAND_MAX) return false;                    // too many values share the deciding bin
-  // 3. gather everything at or above that bin
-  for (int base = 0; base < V; base += blockDim.x * UN) {
-    float v[UN];
-#pragma unroll
-    for (int u = 0; u < UN; ++u) {
-      const int i = base + u * blockDim.x + tid;
-      v[u] = i < V ? row[i] : 0.f;
-    }
-#pragma unroll
-    for (int u = 0; u < UN; ++u) {
-      const int i = base + u * blockDim.x + tid;
-      if (i < V && (int)(key_of(v[u]) >> (32 - HIST_BITS)) >= bin0) {
+  const int bin0 = sm.bin, n_c = sm.n_c;
+  if (n_c <= CAND_MAX) {
+    // 3. gather everything at or above that bin
+    walk_piece(row, lo, hi, vec, [&](int i, float v) {
+      if ((int)(key_of(v) >> (32 - HIST_BITS)) >= bin0) {
         const int pos = atomicAdd(&sm.count, 1);
-        sm.l2[pos] = v[u] == v[u] ? v[u] : -INFINITY;     // NaN read as -inf, as ld() does
+        sm.l2[pos] = v == v ? v : -INFINITY;           // NaN read as -inf, as ld() does
         sm.idx2[pos] = i;
       }
-    }
+    });
   }
+  if (ranks > 1) {
+    cluster_barrier();
+    if (rank == 0 && n_c <= CAND_MAX) {                // the other blocks' lists behind this one's
+      int at = sm.count;
+      for (unsigned r = 1; r < ranks; ++r) {
+        const int n = ld_cluster(&sm.count, r);
+        if (tid < n) {
+          sm.l2[at + tid] = __int_as_float(ld_cluster(reinterpret_cast<const int*>(&sm.l2[tid]), r));
+          sm.idx2[at + tid] = ld_cluster(&sm.idx2[tid], r);
+        }
+        at += n;
+      }
+    }
+    cluster_barrier();                                 // nobody leaves while its list may still be read
+  } else {
+    __syncthreads();
+  }
+  return n_c <= CAND_MAX && rank != 0 ? 0 : n_c;
+}
+
+// Returns false, with nothing decided, if the list does not suffice; the caller then takes the
+// passes over the whole row.  k_eff: how many of the best the top-k stage keeps (V if it is off); n_c: the candidates in l2, idx2.
+__device__ bool sample_small(const float* row, int V, int k_eff, float temp, float top_p, float min_p,
+                             float xtc_probability, float xtc_threshold, int xtc_min_keep, float u_draw, float u_xtc,
+                             Shared& sh, Small& sm, int n_c, int* picked_out) {
+  const int tid = threadIdx.x;
+  const int k_list = min(k_eff, CAND_MAX);           // the list holds the k_list best
+  // 4. into index order (the gather's order is whatever the atomics made it).  The list is padded to whole pieces of four: a
+  //    walk over it is one 16-byte load per four candidates.
+  const int n_4 = (n_c + 3) & ~3;
+  if (tid >= n_c && tid < n_4) sm.idx2[tid] = 0x7fffffff;
   __syncthreads();
-  // 4. into index order (the gather's order is whatever the atomics made it)
-  if (tid < n_c) {
+  const bool have = tid < n_c;
+  if (have) {
     const int my = sm.idx2[tid];
     int rank = 0;
-    for (int j = 0; j < n_c; ++j) rank += sm.idx2[j] < my;
+    for (int j = 0; j < n_4; j += 4) {
+      const int4 o = *reinterpret_cast<const int4*>(&sm.idx2[j]);
+      rank += (o.x < my) + (o.y < my) + (o.z < my) + (o.w < my);
+    }
     sm.l[rank] = sm.l2[tid];
+    sm.key[rank] = key_of(sm.l2[tid]);
     sm.idx[rank] = my;
   }
+  if (tid >= n_c && tid < n_4) sm.key[tid] = 0u;       // below every key of a number
   __syncthreads();
   // 5. the k_list best of them: descending value, ties in index order
-  const bool have = tid < n_c;
   const float my_l = have ? sm.l[tid] : -INFINITY;
   const unsigned my_key = key_of(my_l);
-  int rank_desc = 0;
-  if (have)
-    for (int j = 0; j < n_c; ++j) {
-      const unsigned kj = key_of(sm.l[j]);
-      rank_desc += kj > my_key || (kj == my_key && j < tid);
+  int rank_desc = n_4;
+  if (have) {
+    rank_desc = 0;
+    for (int j = 0; j < n_4; j += 4) {
+      const uint4 o = *reinterpret_cast<const uint4*>(&sm.key[j]);
+      rank_desc += (o.x > my_key || (o.x == my_key && j < tid)) + (o.y > my_key || (o.y == my_key && j + 1 < tid)) +
+                   (o.z > my_key || (o.z == my_key && j + 2 < tid)) + (o.w > my_key || (o.w == my_key && j + 3 < tid));
     }
+  }
   bool member = have && rank_desc < k_list;
   const float mx = block_reduce_max(member ? my_l : -INFINITY, sh);
   const float e = member ? expf(my_l - mx) : 0.f;
   auto minp_ok = [&](float l, float mass) { return min_p <= 0.f || l == mx || mass >= min_p; };
   // 6. top-p: the shortest prefix of the descending order whose mass reaches top_p * total
-  sm.w[tid < CAND_MAX ? tid : 0] = 0.f;                 // (blockDim.x == CAND_MAX)
-  __syncthreads();
-  if (have) sm.w[tid] = e;
-  sm.in[tid] = member;
-  __syncthreads();
+  sm.w[tid] = e;                                         // (blockDim.x == CAND_MAX)
+  sm.order[tid] = rank_desc;
   float total_e = block_reduce_sum(e, sh);               // a fixed order of additions: the same in every run
   if (k_eff > k_list) {
     // The list is a cut of a longer candidate set: the mass is the whole row's, and the list must be
@@ -552,10 +622,14 @@ __device__ bool sample_small(const float* row, int V, int k_eff, float temp, flo
   if (top_p < 1.0f) {
     const float target = top_p * total_e;
     float before = 0.f;
-    if (member)
-      for (int j = 0; j < n_c; ++j) {
-        const unsigned kj = key_of(sm.l[j]);
-        if (sm.in[j] && (kj > my_key || (kj == my_key && j < tid))) before += sm.w[j];
+    if (member)                                          // all that stand before a member are members
+      for (int j = 0; j < n_4; j += 4) {
+        const int4 o = *reinterpret_cast<const int4*>(&sm.order[j]);
+        const float4 w = *reinterpret_cast<const float4*>(&sm.w[j]);
+        before += o.x < rank_desc ? w.x : 0.f;
+        before += o.y < rank_desc ? w.y : 0.f;
+        before += o.z < rank_desc ? w.z : 0.f;
+        before += o.w < rank_desc ? w.w : 0.f;
       }
     member = member && before < target;
   }
@@ -566,8 +640,6 @@ __device__ bool sample_small(const float* row, int V, int k_eff, float temp, flo
   float wgt = member ? expf((my_l - mx) * inv_t) : 0.f;
   __syncthreads();
   sm.w[tid] = wgt;
-  sm.in[tid] = member;
-  __syncthreads();
   float total = block_reduce_sum(wgt, sh);
   const int n_keep = block_reduce_isum(member ? 1 : 0, sh);
   // 8. XTC (src/sampler.zig:244-268): drop every survivor whose probability reaches the threshold
@@ -589,8 +661,6 @@ __device__ bool sample_small(const float* row, int V, int k_eff, float temp, flo
       }
       __syncthreads();
       sm.w[tid] = wgt;
-      sm.in[tid] = member;
-      __syncthreads();
       total = block_reduce_sum(wgt, sh);
     }
   }
@@ -598,14 +668,20 @@ __device__ bool sample_small(const float* row, int V, int k_eff, float temp, flo
   const float r = u_draw * total;
   float incl = 0.f;
   if (have)
-    for (int j = 0; j <= tid; ++j) incl += sm.w[j];
+    for (int j = 0; j <= tid; j += 4) {
+      const float4 w = *reinterpret_cast<const float4*>(&sm.w[j]);
+      incl += w.x;
+      incl += j + 1 <= tid ? w.y : 0.f;
+      incl += j + 2 <= tid ? w.z : 0.f;
+      incl += j + 3 <= tid ? w.w : 0.f;
+    }
   const int picked = block_reduce_imin((member && incl >= r) ? sm.idx[tid] : 0x7fffffff, sh);
   const int last_member = block_reduce_imax(member ? sm.idx[tid] : -1, sh);
   *picked_out = picked != 0x7fffffff ? picked : max(last_member, 0);
   return true;
 }
 
-// One draw per row.  Its two uniforms in [0, 1) (one for the draw, one for the XTC chance) are
+// One draw per row, a cluster each.  Its two uniforms in [0, 1) (one for the draw, one for the XTC chance) are
 // uniforms[row] if given; else they are computed here from (seed, req_ids[row], draws[req_ids[row]]),
 // and that request's count of draws goes up by one: the host then has nothing to send per step.
 __global__ void __launch_bounds__(SAMP_THREADS)
@@ -615,32 +691,37 @@ __global__ void __launch_bounds__(SAMP_THREADS)
                   int* __restrict__ out) {
   __shared__ Shared sh;
   __shared__ float s_u[2];
-  if (threadIdx.x == 0) {
+  __shared__ Small sm;
+  unsigned rank, ranks;        // block 0 of a row's cluster makes the draw
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+  const int at = blockIdx.x / ranks;
+  if (rank == 0 && threadIdx.x == 0) {
     if (uniforms) {
-      s_u[0] = uniforms[(size_t)blockIdx.x * 2];
-      s_u[1] = uniforms[(size_t)blockIdx.x * 2 + 1];
+      s_u[0] = uniforms[(size_t)at * 2];
+      s_u[1] = uniforms[(size_t)at * 2 + 1];
     } else {
-      const int req = req_ids[blockIdx.x];
+      const int req = req_ids[at];
       const int d = draws[req];
       s_u[0] = counter_uniform(seed, req, d, 0);
       s_u[1] = counter_uniform(seed, req, d, 1);
       draws[req] = d + 1;
     }
   }
-  __syncthreads();
-  const float* row = logits + (size_t)blockIdx.x * V;
-  {
-    __shared__ Small sm;
-    const int k_eff = (top_k > 0 && top_k < V) ? top_k : V;
+  const float* row = logits + (size_t)at * V;
+  const int k_eff = (top_k > 0 && top_k < V) ? top_k : V;
+  if (k_eff <= CAND_MAX || top_p < 1.0f || min_p > 0.f) {
+    const int n_c = gather_candidates(row, V, min(k_eff, CAND_MAX), sm);
+    if (rank != 0) return;
     int picked_small = 0;
-    if ((k_eff <= CAND_MAX || top_p < 1.0f || min_p > 0.f) &&
-        sample_small(row, V, k_eff, temp, top_p, min_p, xtc_probability, xtc_threshold, xtc_min_keep, s_u[0], s_u[1], sh,
-                     sm, &picked_small)) {
-      if (threadIdx.x == 0) out[blockIdx.x] = picked_small;
+    if (n_c <= CAND_MAX && sample_small(row, V, k_eff, temp, top_p, min_p, xtc_probability, xtc_threshold, xtc_min_keep, s_u[0],
+                                        s_u[1], sh, sm, n_c, &picked_small)) {
+      if (threadIdx.x == 0) out[at] = picked_small;
       return;
     }
-    __syncthreads();
   }
+  if (rank != 0) return;
+  __syncthreads();
   float mx = -INFINITY;
   for (int i = threadIdx.x; i < V; i += blockDim.x) {
     const float v = row[i];
@@ -753,7 +834,7 @@ __global__ void __launch_bounds__(SAMP_THREADS)
     last_member = max(last_member, sh.ired[w]);
   }
   if (target_warp < 0) {        // rounding left the target a hair above the whole sum
-    if (threadIdx.x == 0) out[blockIdx.x] = max(last_member, 0);
+    if (threadIdx.x == 0) out[at] = max(last_member, 0);
     return;
   }
   if (warp == target_warp) {
@@ -772,7 +853,7 @@ __global__ void __launch_bounds__(SAMP_THREADS)
       if (hits) picked = base + __ffs(hits) - 1;
       offset += __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (lane == 0) out[blockIdx.x] = picked >= 0 ? picked : wlast;   // wlast: the stretch's last survivor
+    if (lane == 0) out[at] = picked >= 0 ? picked : wlast;   // wlast: the stretch's last survivor
   }
 }
 
@@ -862,9 +943,21 @@ int zk_sample(const float* logits, int n, int V, float temp, int top_k, float to
               long long seed, const int* req_ids, int* draws, int* out, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (V <= 0 || !(temp > 0.f) || top_k < 0 || (!uniforms && (!req_ids || !draws))) return ZK_EINVAL;
-  sample_kernel<<<n, SAMP_THREADS, 0, stream>>>(logits, V, temp, top_k, top_p, min_p, xtc_probability, xtc_threshold,
-                                                xtc_min_keep, uniforms, (unsigned long long)seed, req_ids, draws, out);
-  return ZK_LAUNCH_STATUS();
+  // Shorter rows are a single trip to memory per thread and pass for one block; a cluster's barriers cost more than it saves.
+  const int split = V >= 8192 ? 8 : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n * split);
+  cfg.blockDim = dim3(SAMP_THREADS);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = split;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, sample_kernel, logits, V, temp, top_k, top_p, min_p, xtc_probability, xtc_threshold,
+                                 xtc_min_keep, uniforms, (unsigned long long)seed, req_ids, draws, out);
 }
 
 }  // extern "C"
