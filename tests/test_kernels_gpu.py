@@ -1167,3 +1167,58 @@ def test_experts_of_few_rows(k, D, F, E, top, n, kind):
     assert int(status.item()) == 0
     for i in sorted({0, n // 2, n - 1}):                  # a token's result is the same bits alone
         assert torch.equal(call(i, i + 1, old[i:i + 1].clone().cuda())[0], got[i])
+
+
+@pytest.mark.parametrize("H,Hkv,hd,vd", [(4, 2, 64, 64), (6, 1, 36, 32), (5, 5, 128, 128), (20, 1, 96, 96), (3, 3, 20, 64), (2, 1, 4, 128)])
+@pytest.mark.parametrize("opts", [dict(), dict(window=45, keep_first=7), dict(window=40), dict(bias=True), dict(softcap=3.0, sink=True),
+                                  dict(dist=True, gate=True), dict(chunk=48), dict(talk=True)])
+def test_float32_attention_in_16_byte_pieces(k, H, Hkv, hd, vd, opts):
+    """The float32 kernel that copies whole tiles, on pages of one tile and of several, against the general kernel (pages of 16) over
+    the options: prompts with and without a past, of less than a tile, of many; single tokens with their keys in one
+    piece and cut, cuts behind a sequence's end.  Both make every sum in the same order; the bound leaves the scores (up to 20)
+    8 ulp of themselves, which the exponential hands on, and the outputs 16 ulp of the values' sum."""
+    from zinfer_b200.parts.attention import query_tiles as attn_tiles_host
+    T = 200
+    if opts.get("talk") and vd != hd:
+        opts = dict()
+    lens = [1, 31, 33, 96, T]
+    kk, v = [rnd((l, Hkv, hd), 10 + l, torch.float32) for l in lens], [rnd((l, Hkv, vd), 40 + l, torch.float32) for l in lens]
+    bq, _ = k.attn_tile_shape(H, Hkv)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32).cuda()
+    kw = dict(window=opts.get("window", 0), keep_first=opts.get("keep_first", 0), softcap=opts.get("softcap", 0.0), value_dim=vd)
+    kw["chunk"] = opts.get("chunk", 0)
+    if "bias" in opts:
+        kw["bias"] = (rnd((H,), 1, torch.float32).abs().cuda(), rnd((H,), 2, torch.float32).abs().cuda())
+    if "sink" in opts:
+        kw["sink"] = rnd((H,), 3, torch.float32).cuda()
+    if "dist" in opts:
+        kw["distance_table"] = k.DistanceTable(rnd((H, 70), 4, torch.float32).cuda())
+    if "talk" in opts:
+        kw["talk"] = (torch.eye(H) + rnd((H, H), 5, torch.float32, 0.1)).cuda()
+
+    def run(page, ends, counts, splits=1, split_keys=0):
+        """Queries of the last counts[i] positions before ends[i]."""
+        slots = list(range(len(lens)))[::-1]
+        setup = PagedSetup(lens, slots, len(lens), page, Hkv, hd, torch.float32, seed=page)
+        kc, vc = torch.full(setup.k.shape, float("nan")), torch.full(setup.k.shape[:3] + (vd,), float("nan"))
+        for i, l in enumerate(lens):
+            for p in range(min(l, ends[i])):
+                at = int(setup.table[slots[i], p // page])
+                kc[at, :, p % page], vc[at, :, p % page] = kk[i][p], v[i][p]
+        q = torch.cat([rnd((l, H * hd), 70 + l, torch.float32, hd ** -0.5)[e - c:e] for l, e, c in zip(lens, ends, counts)]).cuda()
+        tiles = torch.from_numpy(attn_tiles_host(counts, bq)).cuda()
+        gate = {"gate": rnd((sum(counts), H), 6, torch.float32).cuda()} if "gate" in opts else {}
+        return k.attention(q, kc.cuda(), vc.cuda(), tiles[0].contiguous(), tiles[1].contiguous(), i32([0] + list(np.cumsum(counts))),
+                           i32([e - c for e, c in zip(ends, counts)]), i32(slots), setup.table_dev, H, Hkv, hd, 1.0,
+                           num_splits=splits, split_keys=split_keys, **kw, **gate)
+
+    talk = 2.0 if "talk" in opts else 1.0
+    for ends, counts, cut in ((lens, lens, ()), (lens, [1, 7, 33, 40, 170], ()), (lens, [1] * 5, ()), (lens, [1] * 5, (4, 64)),
+                              ([1, 20, 32, 90, 129], [1] * 5, (9, 32))):
+        if cut and opts.get("chunk"):
+            cut = (2, 32)                      # cuts count from the first key a query sees
+        want = run(16, ends, counts, *cut)
+        assert torch.isfinite(want).all()
+        bound = 2.0 ** -23 * (8 * 20 + 16) * talk * max(x.abs().max().item() for x in v)
+        for page in (32, 96):
+            assert ((run(page, ends, counts, *cut) - want).abs() <= bound).all()

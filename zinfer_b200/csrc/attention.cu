@@ -596,6 +596,271 @@ __global__ void __launch_bounds__(ATT_WARPS * 32)
   }
 }
 
+// (2b) The same attention over a float32 cache whose rows come in 16-byte pieces: head sizes of a multiple of 4, values 32, 64, 96
+// or 128 wide, pages of whole key tiles.  Block, rows, options and every sum are attn_fwd_kernel's (each score one accumulator over
+// d in order, each output one over the keys in order), so both give the same bits.
+// What bounded the general kernel was neither bytes nor FMAs but waiting: a tile was requested value by value when the one
+// before it was done with, and five shared-memory loads fed four FMAs.  Here the tiles are under way as 16-byte asynchronous
+// copies while others are worked on (`stages` of them; a tile lies in one page, whose number is looked up a tile ahead), scores
+// take four entries of a key row and of four query rows per load, and the weights go through shared memory, four keys to a load,
+// instead of a shuffle per row and key.  Warps without a row (single tokens) only copy.
+// 16 heads on 8, 64 wide, microseconds with attn_fwd_kernel and with this: prompts of 150 and 300 tokens 151 -> 46; two single
+// tokens over 150 and 300 keys in chunks of 128 94 -> 11.
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool in) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = in ? 16 : 0;                      // fewer source bytes than 16: the rest is zero-filled
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+
+template <int N> struct Count { static constexpr int value = N; };
+
+template <int NPL>
+__device__ __forceinline__ void load_value(const float* row, int lane, float (&v)[NPL]) {
+  if constexpr (NPL == 2) {
+    const float2 t = *reinterpret_cast<const float2*>(row + 2 * lane);
+    v[0] = t.x; v[1] = t.y;
+  } else if constexpr (NPL == 4) {
+    const float4 t = *reinterpret_cast<const float4*>(row + 4 * lane);
+    v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+  } else {
+#pragma unroll
+    for (int c = 0; c < NPL; ++c) v[c] = row[lane + 32 * c];
+  }
+}
+
+template <int NPL>
+__global__ void __launch_bounds__(ATT_WARPS * 32)
+    attn_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
+                    float* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml,
+                    const int* __restrict__ tile_seq, const int* __restrict__ tile_q0, const int* __restrict__ cu_q,
+                    const int* __restrict__ seq_start, const int* __restrict__ seq_slot,
+                    const int* __restrict__ page_table, int pt_stride, int n_tokens, int H, int Hkv, int hd,
+                    int page_size, int window, float scale, int bq, int gc, int num_splits, int split_keys,
+                    const float* __restrict__ bias_r1, const float* __restrict__ bias_r2, int cross, int keep,
+                    const float* __restrict__ sink, float softcap, const float* __restrict__ dist,
+                    int dist_len, int mask_chunk, const float* __restrict__ gate, int ld_gate, int stages) {
+  constexpr int VD = 32 * NPL;
+  const int k_ld = hd + 4;                        // eight adjacent rows of 16 bytes fall into different banks
+  extern __shared__ __align__(16) float smem[];
+  float* qs = smem;                               // [ATT_ROWS][hd]
+  float* ps = qs + ATT_ROWS * hd;                 // [ATT_ROWS][ATT_TK] weights of this tile
+  float* tiles = ps + ATT_ROWS * ATT_TK;          // stages x ([ATT_TK][k_ld] keys, [ATT_TK][VD] values)
+  const int stage_n = ATT_TK * (k_ld + VD);
+
+  zk_let_next_start();
+  zk_wait_prior();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = H / Hkv;
+  const int chunks = (g + gc - 1) / gc;
+  const int kvh = (blockIdx.y / chunks) % Hkv, chunk = blockIdx.y % chunks;
+  const int VH = cross ? Hkv : 1;
+  const int vh = cross ? blockIdx.y / (chunks * Hkv) : kvh;      // the key/value head whose values this block reads
+  const int b = tile_seq[blockIdx.x], q0 = tile_q0[blockIdx.x];
+  const int split = blockIdx.z;
+  const int t_base = cu_q[b], Tq = cu_q[b + 1] - t_base;
+  const int start = seq_start[b];
+  const int* pt = page_table + (size_t)seq_slot[b] * pt_stride;
+
+  // key range of the block, as in attn_fwd_kernel
+  const int last_tq = min(q0 + bq, Tq) - 1;
+  int k_end = start + last_tq + 1;
+  int k_begin = 0;
+  if (window > 0) {
+    const int first_hi = start + q0 + 1;
+    k_begin = first_hi > window ? first_hi - window : 0;
+  }
+  const int cut0 = mask_chunk > 0 ? (start + q0) / mask_chunk * mask_chunk : 0;
+  if (mask_chunk > 0) k_begin = cut0;
+  int a_lo = 0, a_hi = (keep > 0 && k_begin > 0) ? min(keep, k_begin) : 0;
+  if (num_splits > 1) {
+    k_begin = max(k_begin, cut0 + split * split_keys);
+    k_end = min(k_end, cut0 + (split + 1) * split_keys);
+    a_lo = split * split_keys;
+    a_hi = min(a_hi, (split + 1) * split_keys);
+  }
+  k_begin = (k_begin / ATT_TK) * ATT_TK;
+  a_hi = min(a_hi, k_begin);
+  const int split_lo = num_splits > 1 ? cut0 + split * split_keys : 0;
+  const int n_kept = a_hi > a_lo ? (a_hi - a_lo + ATT_TK - 1) / ATT_TK : 0;       // tiles of kept first tokens, then the others
+  const int n_tiles = n_kept + (k_end > k_begin ? (k_end - k_begin + ATT_TK - 1) / ATT_TK : 0);
+  auto tile_begin = [&](int t) { return t < n_kept ? a_lo + t * ATT_TK : k_begin + (t - n_kept) * ATT_TK; };
+  auto page_of = [&](int t) { return t < n_tiles ? pt[tile_begin(t) / page_size] : -1; };
+
+  int page_next = page_of(0), slot_next = 0;      // page and stage of the tile that is requested next
+  auto request = [&](int t) {
+    if (t < n_tiles) {
+      const int kb = tile_begin(t), page = page_next;
+      float* Ks = tiles + (size_t)slot_next * stage_n;
+      float* Vs = Ks + ATT_TK * k_ld;
+      const size_t in_page = kb % page_size;
+      const float* ksrc = k_cache + (((size_t)max(page, 0) * Hkv + kvh) * page_size + in_page) * hd;
+      const float* vsrc = v_cache + (((size_t)max(page, 0) * Hkv + vh) * page_size + in_page) * VD;
+      const int valid = page >= 0 ? min(k_end - kb, ATT_TK) : 0;                  // rows beyond are filled with zeros
+      const int per = hd / 4;
+      for (int i = tid; i < ATT_TK * per; i += ATT_WARPS * 32) {
+        const int j = i / per, d = (i - j * per) * 4;
+        cp_async16(Ks + j * k_ld + d, ksrc + (j < valid ? j * hd + d : 0), j < valid);
+      }
+#pragma unroll
+      for (int l = 0; l < ATT_TK * VD / 4 / (ATT_WARPS * 32); ++l) {
+        const int i = tid + l * ATT_WARPS * 32, j = i / (VD / 4), d = i % (VD / 4) * 4;
+        cp_async16(Vs + j * VD + d, vsrc + (j < valid ? j * VD + d : 0), j < valid);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    page_next = page_of(t + 1);
+    slot_next = slot_next + 1 == stages ? 0 : slot_next + 1;
+  };
+  for (int t = 0; t < stages - 1; ++t) request(t);
+
+  // rows of this warp: r = warp + 4*i
+  int row_t[4], row_h[4], row_lo[4], row_hi[4];
+  bool row_ok[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = warp + ATT_WARPS * i;
+    const int tq = r / gc, hl = r % gc;
+    row_ok[i] = (tq < bq) && (q0 + tq < Tq) && (chunk * gc + hl < g);
+    row_t[i] = t_base + q0 + tq;
+    row_h[i] = kvh * g + chunk * gc + hl;
+    row_hi[i] = start + q0 + tq + 1;
+    row_lo[i] = (window > 0 && row_hi[i] > window) ? row_hi[i] - window : 0;
+    if (mask_chunk > 0) row_lo[i] = (row_hi[i] - 1) / mask_chunk * mask_chunk;
+  }
+  const bool biased = bias_r1 != nullptr && bias_r2 != nullptr;
+  float r1[4], r2[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    r1[i] = (biased && row_ok[i]) ? bias_r1[row_h[i]] : 0.f;
+    r2[i] = (biased && row_ok[i]) ? bias_r2[row_h[i]] : 0.f;
+  }
+  for (int idx = tid; idx < ATT_ROWS * hd; idx += ATT_WARPS * 32) {
+    const int r = idx / hd, d = idx - r * hd;
+    const int tq = r / gc, hl = r % gc;
+    const bool ok = (tq < bq) && (q0 + tq < Tq) && (chunk * gc + hl < g);
+    qs[idx] = ok ? q[(size_t)(t_base + q0 + tq) * H * hd + (size_t)(kvh * g + chunk * gc + hl) * hd + d] : 0.f;
+  }
+
+  float m[4], l[4], o[4][NPL];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.f;
+#pragma unroll
+    for (int c = 0; c < NPL; ++c) o[i][c] = 0.f;
+  }
+
+  int stage = 0;
+  int page = page_of(0);
+  // rows 0 .. R-1 of this warp against tile t
+  auto work = [&](auto count, int t) {
+    constexpr int R = decltype(count)::value;
+    const float* Ks = tiles + (size_t)stage * stage_n;
+    const float* Vs = Ks + ATT_TK * k_ld;
+    const int kb = tile_begin(t);
+    float s[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) s[i] = 0.f;
+    const float* kr = Ks + lane * k_ld;
+#pragma unroll 4
+    for (int d = 0; d < hd; d += 4) {
+      const float4 kd = *reinterpret_cast<const float4*>(kr + d);
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const float4 qd = *reinterpret_cast<const float4*>(qs + (warp + ATT_WARPS * i) * hd + d);
+        s[i] = fmaf(qd.x, kd.x, s[i]);
+        s[i] = fmaf(qd.y, kd.y, s[i]);
+        s[i] = fmaf(qd.z, kd.z, s[i]);
+        s[i] = fmaf(qd.w, kd.w, s[i]);
+      }
+    }
+    const int kp = kb + lane;
+    const bool key_ok = kp < k_end && kp >= split_lo && page >= 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const bool ok = row_ok[i] && key_ok && (kp >= row_lo[i] || kp < keep) && kp < row_hi[i];
+      float sc = -INFINITY;
+      if (ok) {
+        sc = s[i] * scale;
+        if (softcap > 0.f) sc = softcap * tanhf(sc / softcap);
+        if (biased) sc -= r1[i] * log1pf(r2[i] * (float)(row_hi[i] - 1 - kp));
+        if (dist) sc += dist[(size_t)row_h[i] * dist_len + min(row_hi[i] - 1 - kp, dist_len - 1)];
+      }
+      const float mt = warp_max(sc);
+      float p = 0.f;
+      if (mt != -INFINITY) {                      // else no key of this tile is visible to this row
+        const float m_new = fmaxf(m[i], mt);
+        const float alpha = expf(m[i] - m_new);
+        p = ok ? expf(sc - m_new) : 0.f;
+        l[i] = l[i] * alpha + warp_sum(p);
+        m[i] = m_new;
+#pragma unroll
+        for (int c = 0; c < NPL; ++c) o[i][c] *= alpha;
+      }
+      ps[(warp + ATT_WARPS * i) * ATT_TK + lane] = p;
+    }
+    __syncwarp();
+#pragma unroll 2
+    for (int j = 0; j < ATT_TK; j += 4) {
+      float p[R][4], v[4][NPL];
+#pragma unroll
+      for (int i = 0; i < R; ++i) {
+        const float4 t4 = *reinterpret_cast<const float4*>(ps + (warp + ATT_WARPS * i) * ATT_TK + j);
+        p[i][0] = t4.x; p[i][1] = t4.y; p[i][2] = t4.z; p[i][3] = t4.w;
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) load_value<NPL>(Vs + (j + e) * VD, lane, v[e]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+          for (int c = 0; c < NPL; ++c) o[i][c] = fmaf(p[i][e], v[e][c], o[i][c]);
+    }
+    __syncwarp();                                 // the weights have been read
+  };
+  for (int t = 0; t < n_tiles; ++t) {
+    if (stages == 2) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    else asm volatile("cp.async.wait_group 2;" ::: "memory");
+    __syncthreads();                              // tile t is here (and qs, first time), and nobody reads the one before it
+    request(t + stages - 1);
+    if (row_ok[1] || row_ok[2] || row_ok[3]) work(Count<4>{}, t);
+    else if (row_ok[0]) work(Count<1>{}, t);
+    page = page_of(t + 1);
+    stage = stage + 1 == stages ? 0 : stage + 1;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    if (!row_ok[i]) continue;
+    float* dst;
+    float by = 1.0f;
+    if (num_splits == 1 && !cross) {
+      if (sink) {                                 // one more term of the denominator
+        const float sk = sink[row_h[i]];
+        const float m_fin = fmaxf(m[i], sk);
+        const float alpha = m[i] == -INFINITY ? 0.f : expf(m[i] - m_fin);
+        l[i] = l[i] * alpha + expf(sk - m_fin);
+#pragma unroll
+        for (int c = 0; c < NPL; ++c) o[i][c] *= alpha;
+      }
+      by = l[i] > 0.f ? 1.0f / l[i] : 0.f;
+      if (gate) by /= 1.0f + expf(-gate[(size_t)row_t[i] * ld_gate + row_h[i]]);
+      dst = out + ((size_t)row_t[i] * H + row_h[i]) * VD;
+    } else {
+      const size_t row = (((size_t)split * n_tokens + row_t[i]) * H + row_h[i]) * VH + (cross ? vh : 0);
+      dst = part_o + row * VD;
+      if (lane == 0) {
+        part_ml[row * 2] = m[i];
+        part_ml[row * 2 + 1] = l[i];
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < NPL; ++c) dst[NPL == 2 || NPL == 4 ? lane * NPL + c : lane + 32 * c] = o[i][c] * by;
+  }
+}
+
 // (3) merge: out = sum_s e^{m_s - M} o_s / sum_s e^{m_s - M} l_s.  One warp per (token, head).
 // A lane holds the (m, l) of one chunk (32 chunks at a time), so that the loads of all chunks are
 // under way together; the sums run over the chunks in ascending order whatever the timing.
@@ -771,6 +1036,24 @@ int launch_attn(const void* q, const void* k_cache, const void* v_cache, void* o
                 int dist_len, int mask_chunk, const void* gate, int ld_gate, cudaStream_t stream) {
   const size_t smem = attn_smem_bytes(hd, v_from_k ? 0 : vd);
   if (smem > 227 * 1024) return ZK_EINVAL;
+  if constexpr (sizeof(T) == 4 && NPL <= 4) {
+    auto pieces = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    if (hd % 4 == 0 && hd <= 128 && vd == 32 * NPL && page_size % ATT_TK == 0 && !v_from_k && pieces(k_cache) && pieces(v_cache)) {
+      // Single tokens: a chunk of keys is few tiles, all of which are requested at once.  Prompts: more blocks per SM instead.
+      const int stages = num_splits > 1 ? 4 : 2;
+      auto bytes = [&](int st) { return sizeof(float) * (size_t)(ATT_ROWS * hd + ATT_ROWS * ATT_TK + st * ATT_TK * (hd + 4 + vd)); };
+      auto fast = attn_f32_kernel<NPL>;
+      cudaError_t e = cudaFuncSetAttribute(fast, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(sizeof(float) * (ATT_ROWS * 128 + ATT_ROWS * ATT_TK + 4 * ATT_TK * (132 + 32 * NPL))));
+      if (e != cudaSuccess) return (int)e;
+      const int heads = H / Hkv;
+      return zk_launch_dependent(fast, dim3(n_tiles, Hkv * ((heads + gc - 1) / gc) * (cross ? Hkv : 1), num_splits), dim3(ATT_WARPS * 32),
+                                 bytes(stages), stream, (const float*)q, (const float*)k_cache, (const float*)v_cache, (float*)out,
+                                 part_o, part_ml, tile_seq, tile_q0, cu_q, seq_start, seq_slot, page_table, pt_stride, n_tokens, H,
+                                 Hkv, hd, page_size, window, scale, bq, gc, num_splits, split_keys, r1, r2, cross, keep, sink, softcap,
+                                 dist, dist_len, mask_chunk, (const float*)gate, ld_gate, stages);
+    }
+  }
   auto kern = attn_fwd_kernel<T, NPL>;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
