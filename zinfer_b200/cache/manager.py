@@ -76,6 +76,13 @@ class KVView:
     group: int
 
 
+def _staged(host: torch.Tensor, device) -> torch.Tensor:
+    """A pinned copy of host values for a copy to the device that the host does not wait for: from pageable memory it waited for
+    all that was queued before, in every step that gave a sequence a page (with 64 sequences, in two steps of three).  PyTorch's
+    pinned allocator uses the memory again only when that copy has run."""
+    return host.pin_memory() if torch.device(device).type == "cuda" else host
+
+
 class KVGroup:
     def __init__(self, request: KVRequest, n_layers: int, num_pages: int, page_size: int, max_slots: int,
                  max_pages_per_seq: int, dtype: torch.dtype, device):
@@ -133,7 +140,7 @@ class KVGroup:
 
     def sync(self) -> None:
         if self.dirty:
-            self.table_dev.copy_(torch.from_numpy(self.table_host), non_blocking=False)
+            self.table_dev.copy_(_staged(torch.from_numpy(self.table_host), self.table_dev.device), non_blocking=True)
             self.dirty = False
 
 
@@ -240,7 +247,7 @@ class CacheManager:
             self.active[s] = True
             self.lengths[s] = 0
         if slots and self.state_tensors:
-            idx = torch.tensor(slots, dtype=torch.int64, device=self.device)
+            idx = _staged(torch.tensor(slots, dtype=torch.int64), self.device).to(self.device, non_blocking=True)
             for st in self.state_tensors:
                 st.index_fill_(1, idx, 0)
         return slots
