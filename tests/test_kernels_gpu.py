@@ -1222,3 +1222,40 @@ def test_float32_attention_in_16_byte_pieces(k, H, Hkv, hd, vd, opts):
         bound = 2.0 ** -23 * (8 * 20 + 16) * talk * max(x.abs().max().item() for x in v)
         for page in (32, 96):
             assert ((run(page, ends, counts, *cut) - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("H,Hkv,hd", [(8, 1, 64), (12, 3, 64), (4, 4, 64), (8, 2, 128)])
+@pytest.mark.parametrize("opts", [dict(), dict(window=100), dict(window=70, keep_first=9, bias=True), dict(bias=True), dict(softcap=4.0, bias=True),
+                                  dict(dist=True), dict(dist=True, bias=True), dict(chunk=96, sink=True), dict(talk=True, bias=True)])
+def test_prompt_attention_variants_against_the_general_kernel(k, H, Hkv, hd, opts):
+    """The prompt kernel's three variants of the scores (plain, a staged bias, everything) on prompts of less than a tile, of
+    whole tiles, behind a past, with tiles inside, at and beyond the edge of the window or stretch, against the general kernel on
+    the same bfloat16 rows.  The weights and the result are rounded to bfloat16 once each (2^-8 of themselves at most), the
+    exponentials' arguments (up to 30 on base 2) to float32: 2^-7 + 30 * 2^-22 of the largest value; the talk mix sums H heads."""
+    from zinfer_b200.parts.attention import query_tiles as attn_tiles_host
+    lens, counts, page = [5, 64, 130, 333], [5, 64, 67, 200], 64
+    setup = PagedSetup(lens, [2, 0, 3, 1], 4, page, Hkv, hd, torch.bfloat16, seed=4)
+    setup.k.copy_(rnd(setup.k.shape, 2, torch.bfloat16))
+    setup.v.copy_(rnd(setup.v.shape, 3, torch.bfloat16))
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32).cuda()
+    kw = dict(window=opts.get("window", 0), keep_first=opts.get("keep_first", 0), softcap=opts.get("softcap", 0.0), chunk=opts.get("chunk", 0))
+    if "bias" in opts:
+        kw["bias"] = (rnd((H,), 1, torch.float32).abs().cuda(), rnd((H,), 2, torch.float32).abs().cuda())
+    if "sink" in opts:
+        kw["sink"] = rnd((H,), 3, torch.float32).cuda()
+    if "dist" in opts:
+        kw["distance_table"] = k.DistanceTable(rnd((H, 70), 4, torch.float32).cuda())
+    if "talk" in opts:
+        kw["talk"] = (torch.eye(H) + rnd((H, H), 5, torch.float32, 0.1)).cuda()
+    q = rnd((sum(counts), H * hd), 7, torch.bfloat16).cuda()
+
+    def run(kind, bq):
+        tiles = torch.from_numpy(attn_tiles_host(counts, bq)).cuda()
+        return k.attention(q, setup.k, setup.v, tiles[0].contiguous(), tiles[1].contiguous(), i32([0] + list(np.cumsum(counts))),
+                           i32([l - c for l, c in zip(lens, counts)]), i32([2, 0, 3, 1]), setup.table_dev, H, Hkv, hd, hd ** -0.5,
+                           kind=kind, **kw).float()
+
+    want = run("general", k.attn_tile_shape(H, Hkv)[0])
+    got = run("prompt_tc", k._fn("attention_prefill", "zk_attn_prefill_tile_tokens")(H, Hkv))
+    top = setup.v.float().abs().max().item() * (kw["talk"].abs().sum(1).max().item() if "talk" in opts else 1.0)
+    assert torch.isfinite(want).all() and (got - want).abs().max().item() <= (2 * 2.0 ** -7 + 30 * 2.0 ** -22) * top

@@ -55,8 +55,23 @@ __device__ __forceinline__ int swz(int r, int ch) {
 
 // HD: head_dim, 64 or 128 (rows of a tile are whole 128-byte lines, which the swizzle assumes).  HDV: width of a
 // value row, 64 or 128.  GP: heads of a KV group packed into one block.
-template <int HD, int HDV, int GP>
-__global__ void __launch_bounds__(PF_WARPS * 32)
+// What bounds the kernel is the arithmetic on the scores, not the MMAs: so exponentials of one instruction, masks in tiles at an
+// edge only, logarithms of the bias once per head and distance of a tile (they were one per score), and registers for three
+// or four blocks of 64-wide heads per SM.  8 prompts of 600 tokens, 32 heads on 8, window 1024, microseconds before and now: 202
+// -> 95, with the bias 251 -> 117; one of 4,000 380 -> 185 and 492 -> 220; 128-wide heads 304 -> 161 and 354 -> 186.
+// SCORES: what is done with a scaled score besides the mask.  Left to itself the compiler gave the general variant 242 registers
+// (two blocks); with four blocks the biased one spills (127 us for the 117), the plain one does not lose by it (95; 99 with three).
+enum { SCORES_PLAIN = 0, SCORES_BIAS = 1, SCORES_ANY = 2 };
+
+// 2^x on the special-function unit (x <= 0 here; -inf gives 0)
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+template <int HD, int HDV, int GP, int SCORES>
+__global__ void __launch_bounds__(PF_WARPS * 32, HD == 64 ? (SCORES == SCORES_PLAIN ? 4 : 3) : 1)
     attn_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache,
                         bf16* __restrict__ out, const int* __restrict__ tile_seq, const int* __restrict__ tile_q0,
                         const int* __restrict__ cu_q, const int* __restrict__ seq_start,
@@ -120,12 +135,21 @@ __global__ void __launch_bounds__(PF_WARPS * 32)
     if (mask_chunk > 0) row_lo[h] = (row_hi[h] - 1) / mask_chunk * mask_chunk;
     row_dist[h] = hl * (PF_TK + BQ) + tq + PF_TK - 1;
   }
-  const bool biased = bias_r1 != nullptr;
-  float r1[2] = {0.f, 0.f}, r2[2] = {0.f, 0.f};
+  // The softmax runs on base 2: scores are scaled by scale * log2(e), the exponentials are ex2.approx; the maxima go back to base e
+  // when they leave the loop.
+  constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
+  if (SCORES != SCORES_ANY) {
+    softcap = 0.f;
+    dist = nullptr;
+  }
+  const float scale2 = scale * LOG2E, cap2 = softcap * LOG2E, scale_cap = softcap > 0.f ? scale / softcap : 0.f;
+  const bool biased = SCORES == SCORES_BIAS || (SCORES == SCORES_ANY && bias_r1 != nullptr);
+  const bool staged_log = SCORES == SCORES_BIAS || (biased && !dist);   // dist_sm then holds the bias's logarithms
+  float r1_2[2] = {0.f, 0.f}, r2[2] = {0.f, 0.f};
   if (biased) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      r1[h] = bias_r1[row_head[h]];
+      r1_2[h] = bias_r1[row_head[h]] * LOG2E;
       r2[h] = bias_r2[row_head[h]];
     }
   }
@@ -154,6 +178,10 @@ __global__ void __launch_bounds__(PF_WARPS * 32)
   const int a_hi = (keep > 0 && k_begin > 0) ? min(keep, k_begin) : 0;
   const int a_tiles = (a_hi + PF_TK - 1) / PF_TK;
   const int n_tiles = a_tiles + (k_end - k_begin + PF_TK - 1) / PF_TK;
+  // every row sees the keys [edge_lo, edge_hi) (rows that do not exist are not stored)
+  const int edge_hi = start + q0 + 1;
+  int edge_lo = window > 0 ? max(k_end - window, 0) : 0;
+  if (mask_chunk > 0) edge_lo = (k_end - 1) / mask_chunk * mask_chunk;
 
   auto load_tile = [&](int t, int buf) {
     const int kb = t < a_tiles ? t * PF_TK : k_begin + (t - a_tiles) * PF_TK;
@@ -197,6 +225,12 @@ __global__ void __launch_bounds__(PF_WARPS * 32)
         const int hl = i / (PF_TK + BQ), n = d0 + i % (PF_TK + BQ);
         (&dist_sm[0][0])[i] = dist[(size_t)(kvh * G + chunk * GP + hl) * dist_len + min(max(n, 0), dist_len - 1)];
       }
+    } else if (staged_log) {       // ln(1 + r2 * distance): one per head and distance of the tile instead of one per score
+      const int d0 = start + q0 - kb - (PF_TK - 1);
+      for (int i = tid; i < GP * (PF_TK + BQ); i += PF_WARPS * 32) {
+        const int hl = i / (PF_TK + BQ), n = d0 + i % (PF_TK + BQ);
+        (&dist_sm[0][0])[i] = log1pf(bias_r2[kvh * G + chunk * GP + hl] * (float)max(n, 0));
+      }
     }
     __syncthreads();
 
@@ -219,8 +253,9 @@ __global__ void __launch_bounds__(PF_WARPS * 32)
       }
     }
 
-    // scale, mask, online softmax; each row's 64 scores sit in the 4 lanes of a quad
-    const float inv_cap = softcap > 0.f ? 1.0f / softcap : 0.f;
+    // scale, mask, online softmax; each row's 64 scores sit in the 4 lanes of a quad.  Only tiles at the edges hold keys that
+    // some row of the block does not see.
+    const bool edge = kb < edge_lo || kb + PF_TK > edge_hi;
     float m_new[2] = {m_run[0], m_run[1]};
 #pragma unroll
     for (int j = 0; j < 8; ++j)
@@ -228,27 +263,33 @@ __global__ void __launch_bounds__(PF_WARPS * 32)
       for (int i = 0; i < 4; ++i) {
         const int h = i >> 1;
         const int kp = kb + 8 * j + 2 * c + (i & 1);
-        const bool vis = row_ok[h] && (kp >= row_lo[h] || kp < keep) && kp < row_hi[h];
-        float sc = s[j][i] * scale;
-        if (softcap > 0.f) sc = softcap * fast_tanh(sc * inv_cap);     // capped scores
-        if (biased && vis) sc -= r1[h] * log1pf(r2[h] * (float)(row_hi[h] - 1 - kp));
-        if (dist) sc += (&dist_sm[0][0])[row_dist[h] - (kp - kb)];
-        s[j][i] = vis ? sc : -INFINITY;
+        float sc = s[j][i] * scale2;
+        if (softcap > 0.f) sc = cap2 * fast_tanh(s[j][i] * scale_cap);     // capped scores
+        if (staged_log) sc -= r1_2[h] * (&dist_sm[0][0])[row_dist[h] - (kp - kb)];
+        else if (biased) sc -= r1_2[h] * log1pf(r2[h] * (float)max(row_hi[h] - 1 - kp, 0));
+        if (dist) sc = fmaf((&dist_sm[0][0])[row_dist[h] - (kp - kb)], LOG2E, sc);
+        if (edge) {
+          const bool vis = row_ok[h] && (kp >= row_lo[h] || kp < keep) && kp < row_hi[h];
+          s[j][i] = vis ? sc : -INFINITY;
+        } else {
+          s[j][i] = sc;
+        }
         m_new[h] = fmaxf(m_new[h], s[j][i]);
       }
-    float alpha[2], row_sum[2] = {0.f, 0.f};
+    float alpha[2], row_sum[2] = {0.f, 0.f}, m_sub[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       m_new[h] = fmaxf(m_new[h], __shfl_xor_sync(0xffffffffu, m_new[h], 1));
       m_new[h] = fmaxf(m_new[h], __shfl_xor_sync(0xffffffffu, m_new[h], 2));
-      alpha[h] = m_new[h] == -INFINITY ? 1.f : expf(m_run[h] - m_new[h]);
+      alpha[h] = m_new[h] == -INFINITY ? 1.f : ex2(m_run[h] - m_new[h]);
+      m_sub[h] = m_new[h] == -INFINITY ? 0.f : m_new[h];               // scores of -inf have a weight of 0 in such a row too
     }
 #pragma unroll
     for (int j = 0; j < 8; ++j)
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int h = i >> 1;
-        const float p = s[j][i] == -INFINITY ? 0.f : expf(s[j][i] - m_new[h]);
+        const float p = ex2(s[j][i] - m_sub[h]);
         s[j][i] = p;
         row_sum[h] += p;
       }
@@ -259,12 +300,15 @@ __global__ void __launch_bounds__(PF_WARPS * 32)
       l_run[h] = l_run[h] * alpha[h] + row_sum[h];
       m_run[h] = m_new[h];
     }
+    // o * 1.0f is o: where no row of the warp found a new maximum the multiplications are left out
+    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
 #pragma unroll
-    for (int j = 0; j < HDV / 8; ++j) {
-      o[j][0] *= alpha[0];
-      o[j][1] *= alpha[0];
-      o[j][2] *= alpha[1];
-      o[j][3] *= alpha[1];
+      for (int j = 0; j < HDV / 8; ++j) {
+        o[j][0] *= alpha[0];
+        o[j][1] *= alpha[0];
+        o[j][2] *= alpha[1];
+        o[j][3] *= alpha[1];
+      }
     }
 
     // O += P V: 4 key steps of 16, HDV/8 column groups (two per ldmatrix)
@@ -290,6 +334,7 @@ __global__ void __launch_bounds__(PF_WARPS * 32)
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     if (!row_ok[h]) continue;
+    m_run[h] *= LN2;
     if (cross) {
       const size_t row = ((size_t)row_tok[h] * H + row_head[h]) * Hkv + vh;
       float* dst = part_o + row * HDV;
@@ -315,13 +360,13 @@ __global__ void __launch_bounds__(PF_WARPS * 32)
   }
 }
 
-template <int HD, int HDV, int GP>
-int launch(const void* q, const void* k_cache, const void* v_cache, void* out, const int* tile_seq, const int* tile_q0,
+template <int HD, int HDV, int GP, int SCORES>
+int launch_scores(const void* q, const void* k_cache, const void* v_cache, void* out, const int* tile_seq, const int* tile_q0,
            const int* cu_q, const int* seq_start, const int* seq_slot, const int* page_table, int pt_stride, int n_tiles,
            int H, int Hkv, int page_size, int window, float scale, const float* r1, const float* r2, float* part_o,
            float* part_ml, int keep, const float* sink, float softcap, const float* dist, int dist_len, int mask_chunk,
            const void* gate, int ld_gate, cudaStream_t stream) {
-  auto kern = attn_prefill_kernel<HD, HDV, GP>;
+  auto kern = attn_prefill_kernel<HD, HDV, GP, SCORES>;
   const size_t smem = 2 * (size_t)PF_TK * (HD + HDV) * 2;
   if (smem + sizeof(float) * (PF_TK * GP + PF_ROWS) > 48 * 1024) {       // with the static slice of the distance table
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -333,6 +378,22 @@ int launch(const void* q, const void* k_cache, const void* v_cache, void* out, c
                                               Hkv, page_size, window, scale, r1, r2, part_o, part_ml, keep, sink, softcap, dist,
                                               dist_len, mask_chunk, (const bf16*)gate, ld_gate);
   return ZK_LAUNCH_STATUS();
+}
+
+template <int HD, int HDV, int GP>
+int launch(const void* q, const void* k_cache, const void* v_cache, void* out, const int* tile_seq, const int* tile_q0,
+           const int* cu_q, const int* seq_start, const int* seq_slot, const int* page_table, int pt_stride, int n_tiles,
+           int H, int Hkv, int page_size, int window, float scale, const float* r1, const float* r2, float* part_o,
+           float* part_ml, int keep, const float* sink, float softcap, const float* dist, int dist_len, int mask_chunk,
+           const void* gate, int ld_gate, cudaStream_t stream) {
+#define ZK_PF_SCORES(S)                                                                                                  \
+  return launch_scores<HD, HDV, GP, S>(q, k_cache, v_cache, out, tile_seq, tile_q0, cu_q, seq_start, seq_slot, page_table,    \
+                                       pt_stride, n_tiles, H, Hkv, page_size, window, scale, r1, r2, part_o, part_ml, keep, \
+                                       sink, softcap, dist, dist_len, mask_chunk, gate, ld_gate, stream)
+  if (softcap > 0.f || dist) ZK_PF_SCORES(SCORES_ANY);
+  if (r1) ZK_PF_SCORES(SCORES_BIAS);
+  ZK_PF_SCORES(SCORES_PLAIN);
+#undef ZK_PF_SCORES
 }
 
 int packed_heads(int G) {
