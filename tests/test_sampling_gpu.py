@@ -276,3 +276,15 @@ def test_rows_cut_over_a_cluster(k, V, opts):
             exact += 1
         assert int(k.sample(dev[i:i + 1].clone(), du[i:i + 1], **opts)) == got[i]
     assert exact >= n - 1
+
+
+def test_rows_on_clusters_of_every_size(k):
+    """The number of rows decides how many blocks share a row (8, 4, 2 or 1): the same draws in any batch."""
+    V, n = 20004, 12
+    x, u = logits_rows(n, V, 9), np.random.default_rng(4).random((n, 2)).astype(np.float32)
+    x[3, ::7], x[4], x[5, 40:] = np.nan, 1.25, -np.inf
+    dev, du = torch.from_numpy(x).cuda(), torch.from_numpy(u).cuda()
+    opts = dict(temp=0.8, top_k=40, top_p=0.95, min_p=0.01)
+    want = k.sample(dev, du, **opts)
+    for times in (2, 3, 5, 6):
+        assert torch.equal(k.sample(dev.repeat(times, 1), du.repeat(times, 1), **opts), want.repeat(times))

@@ -1,4 +1,4 @@
-// Sampling on the device, one thread block (a cluster of 8 for long rows) per row of float32 logits [n, V].
+// Sampling on the device, one thread block (a cluster of up to 8 for few long rows) per row of float32 logits [n, V].
 //
 // The reference's chain (src/sampler.zig:36-37, 190-276): repetition penalty, DRY penalty,
 // greedy if temp <= 0, else top-k, top-p and min-p on untempered probabilities relative to the
@@ -427,7 +427,7 @@ __device__ __forceinline__ float counter_uniform(unsigned long long seed, int re
 // words of shared memory, 64 loads a thread.  So the blocks of a cluster take a piece of the row each: every block adds up the
 // cluster's histograms for itself, gathers its piece's candidates, and block 0 fetches the lists and goes on alone.  Which
 // tokens are candidates, and every sum over them, is what one block made of the whole row: the same bits.
-// Temperature, top-k 40, top-p and min-p over 8 rows of 65,536 logits, microseconds: 35.7 -> 20.0.
+// Temperature, top-k 40, top-p and min-p over 8 rows of 65,536 logits, microseconds: 35.7 -> 14.
 constexpr int CAND_MAX = 1024;
 constexpr int HIST_BITS = 11, HIST_BINS = 1 << HIST_BITS;
 
@@ -444,11 +444,19 @@ struct __align__(16) Small {
   int count, bin, n_c;       // what this block gathered; the deciding bin; candidates of the whole row
 };
 
-__device__ __forceinline__ int ld_cluster(const int* local, unsigned rank) {
+__device__ __forceinline__ unsigned in_cluster(const void* local, unsigned rank) {
   unsigned remote;
-  int v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(rank));
-  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(remote) : "memory");
+  return remote;
+}
+__device__ __forceinline__ int ld_cluster(const int* local, unsigned rank) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(in_cluster(local, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ int2 ld_cluster(const int2* local, unsigned rank) {
+  int2 v;
+  asm volatile("ld.shared::cluster.v2.s32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(in_cluster(local, rank)) : "memory");
   return v;
 }
 
@@ -487,14 +495,13 @@ __device__ __forceinline__ void walk_piece(const float* row, int lo, int hi, boo
 
 // The candidates of a row, all that lie at or above the bin of the k_list-th best, in block 0's l2 and idx2 (in any order);
 // returns their number in block 0, 0 in the others, or more than CAND_MAX, with no list, in all of them if too many values
-// share the deciding bin.  Every block of the cluster calls it.
-__device__ __forceinline__ int gather_candidates(const float* row, int V, int k_list, Small& sm) {
+// share the deciding bin.  Every block of the cluster calls it.  A load from another block takes most of a microsecond, so all that
+// a thread needs from the others is requested before the first is used.
+template <int RANKS>
+__device__ __forceinline__ int gather_candidates(const float* row, int V, int k_list, int rank, Small& sm) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  unsigned rank, ranks;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
-  const int per = ((V + (int)ranks - 1) / (int)ranks + 3) & ~3;
-  const int lo = min(V, (int)rank * per), hi = min(V, lo + per);
+  const int per = ((V + RANKS - 1) / RANKS + 3) & ~3;
+  const int lo = min(V, rank * per), hi = min(V, lo + per);
   const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
   // 1. histogram of the upper bits
   for (int b = tid; b < HIST_BINS; b += SAMP_THREADS) sm.hist[b] = 0;
@@ -506,10 +513,14 @@ __device__ __forceinline__ int gather_candidates(const float* row, int V, int k_
   //    threads runs down the values.
   static_assert(HIST_BINS == 2 * SAMP_THREADS, "two bins per thread");
   const int top = HIST_BINS - 2 * tid;
+  int2 bins[RANKS];
+#pragma unroll
+  for (int r = 0; r < RANKS; ++r) bins[r] = ld_cluster(reinterpret_cast<const int2*>(&sm.hist[top - 2]), r);
   int upper = 0, lower = 0;
-  for (unsigned r = 0; r < ranks; ++r) {
-    upper += ld_cluster(&sm.hist[top - 1], r);
-    lower += ld_cluster(&sm.hist[top - 2], r);
+#pragma unroll
+  for (int r = 0; r < RANKS; ++r) {
+    lower += bins[r].x;
+    upper += bins[r].y;
   }
   int incl = upper + lower;
 #pragma unroll
@@ -541,17 +552,25 @@ __device__ __forceinline__ int gather_candidates(const float* row, int V, int k_
       }
     });
   }
-  if (ranks > 1) {
+  if constexpr (RANKS > 1) {
     cluster_barrier();
-    if (rank == 0 && n_c <= CAND_MAX) {                // the other blocks' lists behind this one's
-      int at = sm.count;
-      for (unsigned r = 1; r < ranks; ++r) {
-        const int n = ld_cluster(&sm.count, r);
-        if (tid < n) {
-          sm.l2[at + tid] = __int_as_float(ld_cluster(reinterpret_cast<const int*>(&sm.l2[tid]), r));
-          sm.idx2[at + tid] = ld_cluster(&sm.idx2[tid], r);
+    if (rank == 0 && n_c <= CAND_MAX) {                // the other blocks' lists behind this one's: thread t fetches the t-th of all
+      int count[RANKS];
+#pragma unroll
+      for (int r = 0; r < RANKS; ++r) count[r] = ld_cluster(&sm.count, r);
+      int from = 0, at = 0, base = 0;
+#pragma unroll
+      for (int r = 0; r < RANKS; ++r) {
+        if (tid >= base && tid < base + count[r]) {
+          from = r;
+          at = tid - base;
         }
-        at += n;
+        base += count[r];
+      }
+      if (from > 0) {
+        const int bits = ld_cluster(reinterpret_cast<const int*>(&sm.l2[at]), from), idx = ld_cluster(&sm.idx2[at], from);
+        sm.l2[tid] = __int_as_float(bits);
+        sm.idx2[tid] = idx;
       }
     }
     cluster_barrier();                                 // nobody leaves while its list may still be read
@@ -641,10 +660,11 @@ __device__ bool sample_small(const float* row, int V, int k_eff, float temp, flo
   __syncthreads();
   sm.w[tid] = wgt;
   float total = block_reduce_sum(wgt, sh);
-  const int n_keep = block_reduce_isum(member ? 1 : 0, sh);
   // 8. XTC (src/sampler.zig:244-268): drop every survivor whose probability reaches the threshold
   //    except the least probable of them
-  if (xtc_probability > 0.f && xtc_threshold <= 0.5f && n_keep >= 2 && total > 0.f && u_xtc <= xtc_probability) {
+  const bool xtc = xtc_probability > 0.f && xtc_threshold <= 0.5f && total > 0.f && u_xtc <= xtc_probability;
+  const int n_keep = xtc ? block_reduce_isum(member ? 1 : 0, sh) : 0;
+  if (n_keep >= 2) {
     const float inv_tot = 1.0f / total;
     const bool is_top = member && wgt * inv_tot >= xtc_threshold;
     const int n_top = block_reduce_isum(is_top ? 1 : 0, sh);
@@ -676,15 +696,15 @@ __device__ bool sample_small(const float* row, int V, int k_eff, float temp, flo
       incl += j + 3 <= tid ? w.w : 0.f;
     }
   const int picked = block_reduce_imin((member && incl >= r) ? sm.idx[tid] : 0x7fffffff, sh);
-  const int last_member = block_reduce_imax(member ? sm.idx[tid] : -1, sh);
-  *picked_out = picked != 0x7fffffff ? picked : max(last_member, 0);
+  *picked_out = picked != 0x7fffffff ? picked : max(block_reduce_imax(member ? sm.idx[tid] : -1, sh), 0);
   return true;
 }
 
 // One draw per row, a cluster each.  Its two uniforms in [0, 1) (one for the draw, one for the XTC chance) are
 // uniforms[row] if given; else they are computed here from (seed, req_ids[row], draws[req_ids[row]]),
 // and that request's count of draws goes up by one: the host then has nothing to send per step.
-__global__ void __launch_bounds__(SAMP_THREADS)
+template <int RANKS>
+__global__ void __launch_bounds__(SAMP_THREADS, 1)
     sample_kernel(const float* __restrict__ logits, int V, float temp, int top_k, float top_p, float min_p,
                   float xtc_probability, float xtc_threshold, int xtc_min_keep, const float* __restrict__ uniforms,
                   unsigned long long seed, const int* __restrict__ req_ids, int* __restrict__ draws,
@@ -692,10 +712,7 @@ __global__ void __launch_bounds__(SAMP_THREADS)
   __shared__ Shared sh;
   __shared__ float s_u[2];
   __shared__ Small sm;
-  unsigned rank, ranks;        // block 0 of a row's cluster makes the draw
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
-  const int at = blockIdx.x / ranks;
+  const int at = blockIdx.x / RANKS, rank = blockIdx.x % RANKS;       // block 0 of a row's cluster makes the draw
   if (rank == 0 && threadIdx.x == 0) {
     if (uniforms) {
       s_u[0] = uniforms[(size_t)at * 2];
@@ -711,7 +728,7 @@ __global__ void __launch_bounds__(SAMP_THREADS)
   const float* row = logits + (size_t)at * V;
   const int k_eff = (top_k > 0 && top_k < V) ? top_k : V;
   if (k_eff <= CAND_MAX || top_p < 1.0f || min_p > 0.f) {
-    const int n_c = gather_candidates(row, V, min(k_eff, CAND_MAX), sm);
+    const int n_c = gather_candidates<RANKS>(row, V, min(k_eff, CAND_MAX), rank, sm);
     if (rank != 0) return;
     int picked_small = 0;
     if (n_c <= CAND_MAX && sample_small(row, V, k_eff, temp, top_p, min_p, xtc_probability, xtc_threshold, xtc_min_keep, s_u[0],
@@ -943,8 +960,11 @@ int zk_sample(const float* logits, int n, int V, float temp, int top_k, float to
               long long seed, const int* req_ids, int* draws, int* out, cudaStream_t stream) {
   if (n <= 0) return 0;
   if (V <= 0 || !(temp > 0.f) || top_k < 0 || (!uniforms && (!req_ids || !draws))) return ZK_EINVAL;
-  // Shorter rows are a single trip to memory per thread and pass for one block; a cluster's barriers cost more than it saves.
-  const int split = V >= 8192 ? 8 : 1;
+  // As many blocks to a row as all rows' blocks find an SM each (at 1,024 threads of 44 registers one fits, and clusters leave some
+  // SMs of a processing cluster free): a second round of blocks costs more than the smaller pieces save.  Rows below 8,192
+  // logits are a single trip to memory per thread.
+  const int split = V < 8192 ? 1 : (8 * n <= 128 ? 8 : (4 * n <= 128 ? 4 : (2 * n <= 128 ? 2 : 1)));
+  auto kern = split == 8 ? sample_kernel<8> : (split == 4 ? sample_kernel<4> : (split == 2 ? sample_kernel<2> : sample_kernel<1>));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(n * split);
   cfg.blockDim = dim3(SAMP_THREADS);
@@ -956,7 +976,7 @@ int zk_sample(const float* logits, int n, int V, float temp, int top_k, float to
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, sample_kernel, logits, V, temp, top_k, top_p, min_p, xtc_probability, xtc_threshold,
+  return (int)cudaLaunchKernelEx(&cfg, kern, logits, V, temp, top_k, top_p, min_p, xtc_probability, xtc_threshold,
                                  xtc_min_keep, uniforms, (unsigned long long)seed, req_ids, draws, out);
 }
 
