@@ -221,9 +221,10 @@ namespace {
 // fragments of mma.m16n8k16, and multiplies them with up to 16 of the expert's rows (8 to a fragment).  The products of
 // bfloat16 values are exact and the sums float32, as before.  A lane takes 16 contiguous bytes of a weight row and of an
 // input row for two MMAs; both use the same order of k inside 32, which a sum does not see.  K is split over the block's
-// warps and over the blocks of a cluster, so that all SMs stream whatever the sizes; the loads of the next expert are under way
-// while this one is multiplied (a ring of registers that runs on across experts).  All partial sums wait in shared
-// memory and are added in the order of warps, then of blocks; a result depends on K and the cluster's size alone, which the
+// warps; where that leaves SMs idle, a cluster's blocks split K further (`k_parts`, while every warp keeps 128 k or more: what a
+// warp does per expert besides must pay) and then share the experts out among themselves.  The loads of the next expert are
+// under way while this one is multiplied (a ring of registers that runs on across experts).  All partial sums wait in shared
+// memory and are added in the order of warps, then of blocks; a result depends on how K is split alone, which the
 // sizes of the model decide: not on the step's other tokens.  Everything a token needs is in one cluster, so its experts are
 // added in the order of k without another kernel.
 // 8 tokens with 2 of 16 experts each (10 different ones), D = F = 2048, one layer of a single-token step, microseconds before and
@@ -243,7 +244,8 @@ struct ExpertArgs {
   const float* route_w;      // DOWN: weight of each pair, or null
   const float* in_w;         // UP: weight of each pair's input, or null
   int* status;
-  int n, D, F, top, vocab, n_experts, n_ident, il, act, accumulate, chunk;   // chunk: tokens per cluster
+  int n, D, F, top, vocab, n_experts, n_ident, il, act, accumulate;
+  int chunk, k_parts;        // tokens per cluster; blocks of a cluster over which K is split (the others of each share its experts)
   float weight;
 };
 
@@ -272,21 +274,23 @@ __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+constexpr size_t EXPERT_HEAD = sizeof(int) * (8 * PAIRS_MAX + 4);
 template <int TILES> constexpr int EXPERT_LD = TILES * 16 + 4;   // floats per pair and warp: adjacent pairs' rows in other banks
 
 // NG: groups of 8 input rows multiplied at once (1 where no expert can have more than 8 pairs); RING: loads of 32 k under way.
-// Shared memory: PAIRS_MAX ints each of experts by pair, pairs in sorted order, places by pair, walks; then the partial
-// sums [warp][pair in sorted order][row of the tiles].
+// Shared memory: the walks, PAIRS_MAX ints each of experts by pair, input rows in sorted order, places by pair, walks by place; then
+// the partial sums [warp][pair in sorted order][row of the tiles].
 template <int MODE, int NG, int RING>
 __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const ExpertArgs a) {
   constexpr int TILES = MODE == EXPERT_GATED ? 2 : 1, LD = EXPERT_LD<TILES>;
   extern __shared__ __align__(16) float ex_smem[];
-  int* pair_expert = reinterpret_cast<int*>(ex_smem);
+  int4* walks = reinterpret_cast<int4*>(ex_smem);  // first place, place behind the last, expert
+  int* pair_expert = reinterpret_cast<int*>(ex_smem) + 4 * PAIRS_MAX;
   int* sorted = pair_expert + PAIRS_MAX;
   int* place = sorted + PAIRS_MAX;
-  int* walks = place + PAIRS_MAX;                  // first place of each walk
-  int* n_walks_p = walks + PAIRS_MAX;
-  float* part = ex_smem + 4 * PAIRS_MAX + 4;
+  int* walk_of = place + PAIRS_MAX;
+  int* n_walks_p = walk_of + PAIRS_MAX;
+  float* part = ex_smem + EXPERT_HEAD / sizeof(float);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, c = lane & 3;
   unsigned rank, ranks;
@@ -319,70 +323,73 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const Ex
   __syncthreads();
   for (int i = tid; i < n_pairs; i += MOE_WARPS * 32) {
     const int e = pair_expert[i];
-    int p = 0;
-    for (int j = 0; j < n_pairs; ++j) p += pair_expert[j] < e || (pair_expert[j] == e && j < i);
-    sorted[p] = i;
+    int p = 0, before = 0;           // place; pairs of the same expert in front
+    for (int j = 0; j < n_pairs; ++j) {
+      const int o = pair_expert[j];
+      before += o == e && j < i;
+      p += o < e;
+    }
+    p += before;
+    sorted[p] = MODE == EXPERT_DOWN ? i : i / a.top;       // the row of the input that the pair reads
     place[i] = p;
+    walk_of[p] = e < a.n_experts && before % (8 * NG) == 0 ? e : -1;   // a walk begins at every 8 NG-th pair of an expert
   }
   __syncthreads();
-  if (warp == 0) {           // a walk begins at every 8 NG-th pair of an expert
+  if (warp == 0) {
     int n_walks = 0;
     for (int base = 0; base < n_pairs; base += 32) {
-      const int p = base + lane;
-      bool head = false;
-      if (p < n_pairs) {
-        const int i = sorted[p], e = pair_expert[i];
-        if (e < a.n_experts) {
-          int before = 0;    // pairs of the same expert in front of this one
-          while (before < p && pair_expert[sorted[p - before - 1]] == e) ++before;
-          head = before % (8 * NG) == 0;
-        }
-      }
-      const unsigned heads = __ballot_sync(0xffffffffu, head);
-      if (head) walks[n_walks + __popc(heads & ((1u << lane) - 1))] = p;
+      const int p = base + lane, e = p < n_pairs ? walk_of[p] : -1;
+      const unsigned heads = __ballot_sync(0xffffffffu, e >= 0);
+      if (e >= 0) walks[n_walks + __popc(heads & ((1u << lane) - 1))] = make_int4(p, n_pairs, e, 0);
       n_walks += __popc(heads);
     }
     if (lane == 0) *n_walks_p = n_walks;
   }
   __syncthreads();
   const int n_walks = *n_walks_p;
+  // every pair's walk, and where each walk ends (the identity experts' pairs stand behind the last)
+  for (int w = tid; w < n_walks; w += MOE_WARPS * 32) {
+    const int p0 = walks[w].x;
+    int p1 = w + 1 < n_walks ? walks[w + 1].x : n_pairs;
+    if (p1 > p0 + 8 * NG) p1 = p0 + 8 * NG;                 // only in front of identity experts' pairs
+    walks[w].y = p1;
+    for (int p = p0; p < p1; ++p) walk_of[p] = w;
+  }
+  __syncthreads();
 
-  // this warp's stretch of K, in steps of 32
-  const int steps = (K + 31) / 32, shares = (int)ranks * MOE_WARPS, share = (int)rank * MOE_WARPS + warp;
+  // this warp's stretch of K, in steps of 32, and this block's share of the walks
+  const int k_parts = a.k_parts, shares_w = (int)ranks / k_parts, part_k = (int)rank % k_parts, share_w = (int)rank / k_parts;
+  const int steps = (K + 31) / 32, shares = k_parts * MOE_WARPS, share = part_k * MOE_WARPS + warp;
   const int s0 = steps * share / shares, s1 = steps * (share + 1) / shares;
 
   struct Stage { uint4 w[TILES][2], x[NG]; };
   Stage ring[RING];
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   // the fetching walk: its expert's rows of this lane, and the input rows of this lane's columns
-  int fetch_walk = 0, fetch_s = s0;
+  int fetch_walk = share_w, fetch_s = s0;
   const bf16* wrow[TILES][2];
   const bf16* xrow[NG];
   bool wok[2];
+  int row[TILES][2];                               // this lane's weight rows of any expert
 #pragma unroll
-  for (int h = 0; h < 2; ++h) wok[h] = unit0 + g + 8 * h < units;
+  for (int h = 0; h < 2; ++h) {
+    wok[h] = unit0 + g + 8 * h < units;
+    const int f = wok[h] ? unit0 + g + 8 * h : 0;
+    row[0][h] = MODE == EXPERT_GATED && a.il ? (f / a.il) * 2 * a.il + f % a.il : f;
+    if (MODE == EXPERT_GATED) row[TILES - 1][h] = a.il ? row[0][h] + a.il : a.F + f;
+  }
   auto enter = [&](int walk) {
-    const int first = walks[walk], e = pair_expert[sorted[first]];
+    const int4 at = walks[walk];
+    const int first = at.x, e = at.z;
     const bf16* base = a.w + (size_t)e * (MODE == EXPERT_GATED ? 2 : 1) * units * K;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int f = wok[h] ? unit0 + g + 8 * h : 0;
-      if constexpr (MODE == EXPERT_GATED) {
-        const int grow = a.il ? (f / a.il) * 2 * a.il + f % a.il : f;
-        wrow[0][h] = base + (size_t)grow * K;
-        wrow[TILES - 1][h] = base + (size_t)(a.il ? grow + a.il : a.F + f) * K;
-      } else {
-        wrow[0][h] = base + (size_t)f * K;
-      }
-    }
+    for (int t = 0; t < TILES; ++t)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) wrow[t][h] = base + (size_t)row[t][h] * K;
 #pragma unroll
     for (int t = 0; t < NG; ++t) {
       const int p = first + t * 8 + g;
-      xrow[t] = nullptr;
-      if (p < n_pairs && pair_expert[sorted[p]] == e) {
-        const int i = sorted[p];
-        xrow[t] = MODE == EXPERT_DOWN ? a.h_in + ((size_t)t0 * a.top + i) * K : a.x + (size_t)(t0 + i / a.top) * K;
-      }
+      xrow[t] = p < at.y ? (MODE == EXPERT_DOWN ? a.h_in + (size_t)t0 * a.top * K : a.x + (size_t)t0 * K) + (size_t)sorted[p] * K : nullptr;
     }
   };
   auto fetch = [&](Stage& st) {
@@ -398,7 +405,7 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const Ex
     for (int t = 0; t < NG; ++t) st.x[t] = in && xrow[t] ? *reinterpret_cast<const uint4*>(xrow[t] + k) : zero;
     if (++fetch_s == s1) {
       fetch_s = s0;
-      ++fetch_walk;
+      fetch_walk += shares_w;
     }
   };
 
@@ -412,7 +419,7 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const Ex
       for (int u = 0; u < NG; ++u)
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[t][u][j] = 0.f;
-    int walk = 0, s = s0;
+    int walk = share_w, s = s0;
     while (walk < n_walks) {
 #pragma unroll
       for (int r = 0; r < RING; ++r) {
@@ -428,7 +435,7 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const Ex
         fetch(ring[r]);
         if (++s < s1) continue;
         // this warp's share of the walk: rows g and g + 8 of each tile, columns 2c and 2c + 1 of each 8
-        const int first = walks[walk], last = walk + 1 < n_walks ? walks[walk + 1] : n_pairs;
+        const int first = walks[walk].x, last = walks[walk].y;
 #pragma unroll
         for (int u = 0; u < NG; ++u)
 #pragma unroll
@@ -441,7 +448,7 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const Ex
             }
           }
         s = s0;
-        ++walk;
+        walk += shares_w;
       }
     }
   } else {                                         // fewer steps than warps: nothing of K is this warp's
@@ -449,6 +456,7 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const Ex
   }
   __syncthreads();
   for (int i = tid; i < n_pairs * TILES * 16; i += MOE_WARPS * 32) {
+    if (walk_of[i / (TILES * 16)] % shares_w != share_w) continue;     // another block's
     const int at = i / (TILES * 16) * LD + i % (TILES * 16);
     float v = 0.f;
 #pragma unroll
@@ -456,10 +464,12 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const Ex
     part[at] = v;
   }
   cluster_barrier();
-  auto sum = [&](int pair, int row) {
-    const float* p = part + place[pair] * LD + row;
+  auto sum = [&](int pair, int row) {              // from the blocks that had the pair's walk
+    const int at = place[pair];
+    const float* p = part + at * LD + row;
+    const unsigned r0 = (unsigned)(walk_of[at] % shares_w) * k_parts;
     float v = 0.f;
-    for (unsigned r = 0; r < ranks; ++r) v += ld_cluster(p, r);
+    for (int r = 0; r < k_parts; ++r) v += ld_cluster(p, r0 + r);
     return v;
   };
   if constexpr (MODE != EXPERT_DOWN) {
@@ -683,25 +693,27 @@ __global__ void __launch_bounds__(MOE_WARPS * 32)
 
 namespace {
 
-// Blocks of a cluster over which K is split: as many as give two blocks to (nearly) every SM, while every warp has 32 k or
-// more.  The model's sizes alone decide, so that a token's sums are the same in every step.
-int expert_split(int units, int K) {
+// The cluster of one slice of 16 units: as many blocks as give (nearly) every SM two.  K is split over them while every warp keeps
+// four steps of 32 k, the rest share the experts.  The model's sizes alone decide, so that a token's sums are the same in every step.
+void expert_cluster(int units, int K, int& k_parts, int& blocks) {
   const int slices = ceil_div_i(units, 16), steps = ceil_div_i(K, 32);
-  int split = 1;
-  while (split < 8 && slices * split < 200 && steps >= 2 * split * MOE_WARPS) split *= 2;
-  return split;
+  k_parts = 1;
+  while (k_parts < 8 && slices * k_parts < 200 && steps >= 8 * k_parts * MOE_WARPS) k_parts *= 2;
+  blocks = k_parts;
+  while (blocks < 8 && slices * blocks < 200) blocks *= 2;
 }
 
 template <int MODE, int NG, int RING>
-int launch_experts(const ExpertArgs& a, cudaStream_t stream) {
+int launch_experts(ExpertArgs a, cudaStream_t stream) {
   const int units = MODE == EXPERT_DOWN ? a.D : a.F, K = MODE == EXPERT_DOWN ? a.F : a.D;
-  constexpr size_t HEAD = sizeof(float) * (4 * PAIRS_MAX + 4);
+  constexpr size_t HEAD = EXPERT_HEAD;
   constexpr size_t PAIR = sizeof(float) * MOE_WARPS * EXPERT_LD<MODE == EXPERT_GATED ? 2 : 1>;
   // The limit is shared by all threads of the process: always what the most pairs need.
   cudaError_t e = cudaFuncSetAttribute(expert_rows_kernel<MODE, NG, RING>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)(HEAD + PAIR * PAIRS_MAX));
   if (e != cudaSuccess) return (int)e;
-  const int split = expert_split(units, K);
+  int split;
+  expert_cluster(units, K, a.k_parts, split);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ceil_div_i(units, 16) * split, ceil_div_i(a.n, a.chunk));
   cfg.blockDim = dim3(MOE_WARPS * 32);
@@ -770,7 +782,10 @@ int launch_moe(const void* x, const int* tokens, const int* table, const void* w
   ea.w = (const bf16*)w_gu; ea.route_w = route_w; ea.in_w = in_w; ea.status = status;
   ea.n = n; ea.D = D; ea.F = F; ea.top = top; ea.vocab = vocab; ea.n_experts = n_experts; ea.n_ident = n_ident; ea.il = il;
   ea.act = act; ea.accumulate = accumulate; ea.weight = in_w ? 1.0f : 1.0f / (float)top;
-  ea.chunk = by_expert ? PAIRS_MAX / top : 0;
+  if (by_expert) {                 // as many tokens to a cluster as its pairs allow, every cluster (nearly) as many as any other
+    const int chunks = ceil_div_i(n, PAIRS_MAX / top);
+    ea.chunk = ceil_div_i(n, chunks);
+  }
   const bool few = n <= 8;         // then no expert has more than 8 rows (unless a table names one twice: another walk)
   if (up_by_expert) {
     if (act < 0) rc = few ? launch_experts<EXPERT_GATED, 1, 3>(ea, stream) : launch_experts<EXPERT_GATED, 2, 2>(ea, stream);
