@@ -108,11 +108,32 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// Two float32 values in a 64-bit register, and the instructions that work on both; each is rounded as fmaf and * round.
+typedef unsigned long long Pair;
+__device__ __forceinline__ Pair pair(float a, float b) {
+  Pair p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(a), "f"(b));
+  return p;
+}
+__device__ __forceinline__ float first(Pair p) { return __uint_as_float((unsigned)p); }
+__device__ __forceinline__ float second(Pair p) { return __uint_as_float((unsigned)(p >> 32)); }
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+  Pair d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+  Pair d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 // DPT: channels per warp; TT: tokens staged at once (sixteen, or eight or four where more do not fit shared memory).
 // REC_KEYED: the recurrence of a retention layer instead, S_t = decay_h S_{t-1} + k_t v_t^T with one fixed decay per head
 // (`decay` [H]); the row's second part then holds the keys k_t in place of the gates.
-template <int DPT, int TT, int REC>
-__global__ void __launch_bounds__(HG_R * 32)
+// BLOCKS: how many of them an SM is to hold.
+template <int DPT, int TT, int REC, int BLOCKS>
+__global__ void __launch_bounds__(HG_R * 32, BLOCKS)
     hgrn2_scan_kernel(const float* __restrict__ qfv, int ld, float* __restrict__ state, long long state_stride,
                       float* __restrict__ o, const int* __restrict__ cu_q, const int* __restrict__ seq_slot, int H, int d,
                       int e, const float* __restrict__ decay, Stepped sp, Capped cp) {
@@ -143,9 +164,18 @@ __global__ void __launch_bounds__(HG_R * 32)
   float* st_max = REC == REC_CAPPED ? state + (size_t)seq_slot[b] * state_stride + cp.max_at + (size_t)h * gridDim.z + blockIdx.z : nullptr;
   float m_run = REC == REC_CAPPED ? *st_max : 0.f;      // the running maximum before the group that is staged next
   const float bias_i = REC == REC_CAPPED ? cp.bi[h] : 0.f, bias_f = REC == REC_CAPPED ? cp.bf[h] : 0.f;
-  float S[DPT];
+  // The rows of S, two to a packed register where a warp has a multiple of four
+  constexpr bool PACKED = DPT % 4 == 0;
+  float S[PACKED ? 1 : DPT];
+  Pair S2[PACKED ? DPT / 2 : 1];
+  auto stored = [&](int k) { return (col && row0 + k < d) ? st[(size_t)(row0 + k) * e + c] : 0.f; };
+  if constexpr (PACKED) {
 #pragma unroll
-  for (int k = 0; k < DPT; ++k) S[k] = (col && row0 + k < d) ? st[(size_t)(row0 + k) * e + c] : 0.f;
+    for (int k = 0; k < DPT; k += 2) S2[k / 2] = pair(stored(k), stored(k + 1));
+  } else {
+#pragma unroll
+    for (int k = 0; k < DPT; ++k) S[k] = stored(k);
+  }
 
   const int head_q = REC == REC_STEPPED ? sp.off_q + h / sp.heads_per_group * d : h * d;       // columns of this head's q
   const int off_f = REC == REC_STEPPED ? sp.off_k - sp.off_q : H * d, off_v = REC == REC_STEPPED ? 0 : 2 * H * d;
@@ -241,18 +271,22 @@ __global__ void __launch_bounds__(HG_R * 32)
         v *= __shfl_sync(0xffffffffu, lane_dt, tt);
       }
       if constexpr (DPT % 4 == 0) {
+        const Pair v2 = pair(v, v), nv2 = pair(-v, -v), keep2 = pair(keep, keep);
+        Pair acc2 = pair(acc, 0.f);
 #pragma unroll
         for (int k4 = 0; k4 < DPT; k4 += 4) {
-          const float4 f4 = *reinterpret_cast<const float4*>(&fs[buf][tt][row0 + k4]);
-          const float4 q4 = *reinterpret_cast<const float4*>(&qs[buf][tt][row0 + k4]);
-          const float ff[4] = {f4.x, f4.y, f4.z, f4.w}, qq[4] = {q4.x, q4.y, q4.z, q4.w};
+          const ulonglong2 f4 = *reinterpret_cast<const ulonglong2*>(&fs[buf][tt][row0 + k4]);
+          const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(&qs[buf][tt][row0 + k4]);
+          const Pair ff[2] = {f4.x, f4.y}, qq[2] = {q4.x, q4.y};
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (REC != REC_GATED) S[k4 + j] = fmaf(keep, S[k4 + j], ff[j] * v);   // decay S + k v
-            else S[k4 + j] = fmaf(ff[j], S[k4 + j], fmaf(-ff[j], v, v));        // f S + (1 - f) v
-            acc = fmaf(S[k4 + j], qq[j], acc);
+          for (int j = 0; j < 2; ++j) {
+            Pair& s2 = S2[k4 / 2 + j];
+            if (REC != REC_GATED) s2 = fma2(keep2, s2, mul2(ff[j], v2));   // decay S + k v
+            else s2 = fma2(ff[j], s2, fma2(ff[j], nv2, v2));               // f S + (1 - f) v
+            acc2 = fma2(s2, qq[j], acc2);
           }
         }
+        acc = first(acc2) + second(acc2);
       } else {
 #pragma unroll
         for (int k = 0; k < DPT; ++k) {
@@ -290,11 +324,32 @@ __global__ void __launch_bounds__(HG_R * 32)
   zk_let_next_start();
   if (col) {
 #pragma unroll
-    for (int k = 0; k < DPT; ++k)
-      if (row0 + k < d) st[(size_t)(row0 + k) * e + c] = S[k];
+    for (int k = 0; k < DPT; ++k) {
+      float s;
+      if constexpr (PACKED) s = k % 2 ? second(S2[k / 2]) : first(S2[k / 2]);
+      else s = S[k];
+      if (row0 + k < d) st[(size_t)(row0 + k) * e + c] = s;
+    }
   }
   if (REC == REC_CAPPED && tid == 0) *st_max = m_run;
 }
+
+namespace {
+
+// With 8 to 32 channels a warp the kernel takes 128 to some 140 registers, which leaves an SM one block.  Where there are more blocks
+// than SMs two of them are worth the few values that then spill; a few long sequences are a chain that the spills lengthen.
+// Microseconds, one float32 value to an instruction / two values with one block / two values with two: 16 heads of 128 x 128, 8 x 600
+// tokens 410 / 389 / 345, 64 single tokens 90 / 88 / 58, 1 x 4,000 tokens 627 / 605 / 1025; of 64 x 64, 64 single tokens
+// @@H64@@.
+template <int DP, int REC>
+auto scan_kernel(dim3 grid) {
+  constexpr int TT = DP > 32 ? 4 : (DP > 16 ? 8 : 16);
+  if constexpr (DP >= 8 && DP <= 32)
+    if ((long long)grid.x * grid.y * grid.z > 148) return hgrn2_scan_kernel<DP, TT, REC, 2>;
+  return hgrn2_scan_kernel<DP, TT, REC, 1>;
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -318,7 +373,7 @@ int zk_hgrn2_scan(float* qfv, int ld, const float* f_bias, const float* lower, f
   }
   dim3 grid(n_seqs, H, (e + 31) / 32);
 #define ZK_HG(DP)                                                                                                    \
-  return zk_launch_dependent(hgrn2_scan_kernel<DP, (DP > 32 ? 4 : (DP > 16 ? 8 : 16)), REC_GATED>, grid, dim3(HG_R * 32), 0, stream, (const float*)qfv, ld, \
+  return zk_launch_dependent(scan_kernel<DP, REC_GATED>(grid), grid, dim3(HG_R * 32), 0, stream, (const float*)qfv, ld, \
                              state, state_stride, o, cu_q, seq_slot, H, d, e, (const float*)nullptr, Stepped{}, Capped{})
   const int dpt = (d + HG_R - 1) / HG_R;
   if (dpt <= 1) ZK_HG(1);
@@ -349,7 +404,7 @@ int zk_retention_scan(float* qkv, int ld, const float* decay, const float* inv_f
   }
   dim3 grid(n_seqs, H, (e + 31) / 32);
 #define ZK_RT(DP)                                                                                                    \
-  return zk_launch_dependent(hgrn2_scan_kernel<DP, (DP > 32 ? 4 : (DP > 16 ? 8 : 16)), REC_KEYED>, grid, dim3(HG_R * 32), 0, stream, (const float*)qkv, ld, \
+  return zk_launch_dependent(scan_kernel<DP, REC_KEYED>(grid), grid, dim3(HG_R * 32), 0, stream, (const float*)qkv, ld, \
                              state, state_stride, o, cu_q, seq_slot, H, d, e, decay, Stepped{}, Capped{})
   const int dpt = (d + HG_R - 1) / HG_R;
   if (dpt <= 1) ZK_RT(1);
@@ -374,7 +429,7 @@ int zk_ssd_scan(const float* xbc, int ld, const float* z, int ld_z, const float*
   const Stepped sp{z, dt_bias, a_log, skip, ld_z, H * e, H * e + groups * d, H / groups};
   dim3 grid(n_seqs, H, (e + 31) / 32);
 #define ZK_SS(DP)                                                                                                    \
-  return zk_launch_dependent(hgrn2_scan_kernel<DP, (DP > 32 ? 4 : (DP > 16 ? 8 : 16)), REC_STEPPED>, grid, dim3(HG_R * 32), 0, stream, xbc, ld, \
+  return zk_launch_dependent(scan_kernel<DP, REC_STEPPED>(grid), grid, dim3(HG_R * 32), 0, stream, xbc, ld, \
                              state, state_stride, o, cu_q, seq_slot, H, d, e, (const float*)nullptr, sp, Capped{})
   const int dpt = (d + HG_R - 1) / HG_R;
   if (dpt <= 1) ZK_SS(1);
@@ -403,7 +458,7 @@ int zk_mlstm_scan(const float* qkv, int ld, const float* zi, const float* zf, in
   const Capped cp{zi, zf, bi, bf, m_out, cap, ld_z, e, (long long)H * d * (e + 1)};
   dim3 grid(n_seqs, H, (e + 1 + 31) / 32);
 #define ZK_ML(DP)                                                                                                    \
-  return zk_launch_dependent(hgrn2_scan_kernel<DP, (DP > 32 ? 4 : (DP > 16 ? 8 : 16)), REC_CAPPED>, grid, dim3(HG_R * 32), 0, stream, qkv, ld, \
+  return zk_launch_dependent(scan_kernel<DP, REC_CAPPED>(grid), grid, dim3(HG_R * 32), 0, stream, qkv, ld, \
                              state, state_stride, o, cu_q, seq_slot, H, d, e + 1, (const float*)nullptr, Stepped{}, cp)
   const int dpt = (d + HG_R - 1) / HG_R;
   if (dpt <= 1) ZK_ML(1);
