@@ -1259,3 +1259,19 @@ def test_prompt_attention_variants_against_the_general_kernel(k, H, Hkv, hd, opt
     got = run("prompt_tc", k._fn("attention_prefill", "zk_attn_prefill_tile_tokens")(H, Hkv))
     top = setup.v.float().abs().max().item() * (kw["talk"].abs().sum(1).max().item() if "talk" in opts else 1.0)
     assert torch.isfinite(want).all() and (got - want).abs().max().item() <= (2 * 2.0 ** -7 + 30 * 2.0 ** -22) * top
+
+
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+@pytest.mark.parametrize("F,K", [(4752, 2048), (9472, 2056), (10752, 2048)])
+def test_skinny_gated_units_across_tasks(k, M, F, K):
+    """Gated units of a few rows with more tasks of 8 units than blocks: blocks with one task more than others, K of no whole slab.
+    Against float64 within the bound of K float32 sums and one rounding to bfloat16 (2^-8); the same bits as a row alone."""
+    x, w = rnd((M, K), 1, torch.bfloat16).cuda(), rnd((2 * F, K), 5, torch.bfloat16, K ** -0.5).cuda()
+    both, terms = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T * (K + 8) * 2.0 ** -23
+    g, u = (both.reshape(M, F // 16, 2, 16)[:, :, i].reshape(M, F) for i in (0, 1))
+    eg, eu = (terms.reshape(M, F // 16, 2, 16)[:, :, i].reshape(M, F) for i in (0, 1))
+    h = g * torch.sigmoid(g) * u
+    bound = 1.1 * eg * (u.abs() + eu) + (g * torch.sigmoid(g)).abs() * eu + (2.0 ** -8 + 2.0 ** -19) * h.abs() + 1e-30
+    got = k.gemm_skinny_swiglu(x, w)
+    assert ((got.double() - h).abs() <= 1.01 * bound).all()
+    assert torch.equal(k.gemm_skinny_swiglu(x[-1:], w)[0], got[-1])

@@ -435,6 +435,127 @@ __global__ void __launch_bounds__(WARPS * 32, skinny_min_blocks(WARPS, NT, EPI))
   }
 }
 
+// Gated units where N gives more tasks than blocks fit beside one another: as many blocks as fit walk the tasks, 16 weight rows
+// each, and the loads run on across them.
+// What bounded skinny_kernel there: its blocks request their weights, wait, multiply, add up the warps' sums and leave, and
+// the block that takes the place starts with an empty pipe; between two rounds of blocks nothing was under way.  Here every
+// slab's registers are filled with the slab U further on, of this task or the next, as soon as its MMAs are issued, so that a warp
+// has U slabs under way all the time, the sums' barrier and the epilogue included (the warps' sums have two buffers: one barrier a
+// task).  A task is 8 units, the gates on rows 0..7 of the fragment and their ups on rows 8..15.  The split of K over the
+// warps and every order of sums are skinny_kernel's: the same bits.
+template <int NT, int U, int NORM_MODE>
+__global__ void __launch_bounds__(256, 2) skinny_stream_kernel(const Args a) {
+  constexpr int WARPS = 8, RED_LD = NT * 8 + 1, TASK_COLS = 8;
+  constexpr int XU = NT == 1 ? U : 2;                      // slabs whose input rows are read together
+  __shared__ float red[2][WARPS][16][RED_LD];
+  __shared__ float row_scale[NT * 8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, c = lane & 3;
+  const int M = a.M, N = a.N, K = a.K;
+  const int n_tasks = (N + TASK_COLS - 1) / TASK_COLS;
+  const int slabs = (K + 31) / 32, per = (slabs + WARPS - 1) / WARPS;
+  const int s_begin = warp * per, s_end = min(slabs, s_begin + per);
+  const int groups = (per + U - 1) / U;                    // of U slabs a task; what a warp has less is zeros
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+
+  uint4 wv[U][2];
+  const bf16* w_task[2];
+  auto aim = [&](int task) {                               // the rows of a task that is fetched
+#pragma unroll
+    for (int h = 0; h < 2; ++h)      // of a group's 32 rows the first 16 are gates
+      w_task[h] = a.W + ((size_t)(task >> 1) * 32 + (task & 1) * 8 + 16 * h + g) * a.ldw + 8 * c;
+  };
+  auto load_w = [&](int u, int task, int s) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const bool ok = task < n_tasks && s < s_end && s * 32 + 8 * c < K;
+      wv[u][h] = ok ? ld16_stream(w_task[h] + s * 32) : zero;
+    }
+  };
+  int task = blockIdx.x;
+  aim(task);
+#pragma unroll
+  for (int u = 0; u < U; ++u) load_w(u, task, s_begin + u);
+  zk_let_next_start();
+  zk_wait_prior();   // the rows and C are the kernels' before
+
+  if constexpr (NORM_MODE == NORM_SCALED) {
+    // one warp per row adds the row's partial sums in a fixed order; read after the first task's barrier
+    for (int m = warp; m < M; m += WARPS) {
+      float t = 0.f;
+      for (int p = lane; p < a.ssq_parts; p += 32) t += a.ssq_in[(size_t)m * a.ssq_parts + p];
+      t = warp_sum(t);
+      if (lane == 0) row_scale[m] = 1.0f / sqrtf(t / (float)K + a.eps);
+    }
+  }
+  bool xok[NT];
+  const bf16* xrow[NT];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    xok[t] = t * 8 + g < M;
+    xrow[t] = a.X + (size_t)(xok[t] ? t * 8 + g : 0) * a.ldx + 8 * c;
+  }
+
+  int buf = 0;
+  for (; task < n_tasks; task += gridDim.x) {
+    float acc[NT][4];
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[t][i] = 0.f;
+    for (int grp = 0; grp < groups; ++grp) {
+      const int s = s_begin + grp * U;
+      const bool last = grp + 1 == groups;
+      const int f_task = last ? task + gridDim.x : task, f_s = last ? s_begin : s + U;
+      if (last && f_task < n_tasks) aim(f_task);
+#pragma unroll
+      for (int u0 = 0; u0 < U; u0 += XU) {
+        uint4 xv[XU][NT];
+#pragma unroll
+        for (int u = 0; u < XU; ++u)
+#pragma unroll
+          for (int t = 0; t < NT; ++t)
+            xv[u][t] = xok[t] && s + u0 + u < s_end && (s + u0 + u) * 32 + 8 * c < K ? ld16(xrow[t] + (s + u0 + u) * 32) : zero;
+#pragma unroll
+        for (int u = 0; u < XU; ++u) {
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            mma16816(acc[t], wv[u0 + u][0].x, wv[u0 + u][1].x, wv[u0 + u][0].y, wv[u0 + u][1].y, xv[u][t].x, xv[u][t].y);
+            mma16816(acc[t], wv[u0 + u][0].z, wv[u0 + u][1].z, wv[u0 + u][0].w, wv[u0 + u][1].w, xv[u][t].z, xv[u][t].w);
+          }
+          load_w(u0 + u, f_task, f_s + u0 + u);
+        }
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) red[buf][warp][g + 8 * (i >> 1)][t * 8 + 2 * c + (i & 1)] = acc[t][i];
+    __syncthreads();
+    auto total = [&](int row, int m) {
+      float v = 0.f;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) v += red[buf][w][row][m];
+      if (NORM_MODE == NORM_SCALED) v *= row_scale[m];     // the rows came without their scale
+      return v;
+    };
+    for (int idx = threadIdx.x; idx < TASK_COLS * NT * 8; idx += WARPS * 32) {
+      const int m = idx / TASK_COLS, i = idx % TASK_COLS, n = task * TASK_COLS + i;
+      if (m >= M || n >= N) continue;
+      const float gate = total(i, m), up = total(8 + i, m);
+      const float gv = a.act ? fmaxf(gate, 0.f) : gate / (1.0f + expf(-gate));
+      reinterpret_cast<bf16*>(a.C)[(size_t)m * a.ldc + n] = __float2bfloat16_rn(gv * up);
+    }
+    buf ^= 1;
+  }
+}
+
+template <int NT, int U, int NORM_MODE>
+int launch_stream(const Args& a, cudaStream_t stream) {
+  const int tasks = ceil_div_i(a.N, 8), at_once = 148 * 2;
+  return zk_launch_dependent(skinny_stream_kernel<NT, U, NORM_MODE>, dim3(tasks < at_once ? tasks : at_once), dim3(256), 0, stream, a);
+}
+
 // Most blocks of a kernel with the norm prologue: two per SM.  Measured on the LFM2-1.2B shapes at
 // one row (where every contraction takes the norm itself): 0.698 ms a step with 296 blocks, 0.771
 // with 148, 0.730 with 444, 0.779 with one block per task.
@@ -524,6 +645,18 @@ int dispatch_plain_any(const Args& a, cudaStream_t stream) {
 
 template <int RG, int EPI, int NORM_MODE>
 int dispatch_fused_mode(const Args& a, cudaStream_t stream) {
+  // Loads that run on across tasks need several slabs per warp and task (K), and rounds of blocks to run on across.  With two
+  // groups of tokens the registers hold only four slabs under way, which pays where the last round of skinny_kernel's blocks (two
+  // per SM) would leave most of the SMs idle.  Whole steps, us, skinny_kernel / this: the 2.6B shape (672 tasks of 32 rows for
+  // 296 places) 1 row 1164 / 1104, 8 rows 1312 / 1218, 16 rows 1655 / 1595; the 1.2B shape (512) 1 row 563 / 557 to 566, 8 rows
+  // 627 / 611 to 623, but 16 rows 778 / 790; the 350M shape (K = 1024, 288) 1 row 312 / 329.
+  if constexpr (EPI == EPI_SWIGLU && NORM_MODE != NORM_FUSED) {
+    const int tasks = a.N / 16, places = 2 * 148;
+    if (a.K >= 2048 && tasks > places) {
+      if (a.M <= 8) return launch_stream<1, 8, NORM_MODE>(a, stream);
+      if (a.M <= 16 && 2 * (tasks % places) < places) return launch_stream<2, 4, NORM_MODE>(a, stream);
+    }
+  }
   if (a.M <= 8) return launch<8, RG, 1, 4, EPI, NORM_MODE, bf16>(a, stream);
   if (a.M <= 16) return launch<8, RG, 2, 2, EPI, NORM_MODE, bf16>(a, stream);
   return ZK_EINVAL;
