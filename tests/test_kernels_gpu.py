@@ -1275,3 +1275,29 @@ def test_skinny_gated_units_across_tasks(k, M, F, K):
     got = k.gemm_skinny_swiglu(x, w)
     assert ((got.double() - h).abs() <= 1.01 * bound).all()
     assert torch.equal(k.gemm_skinny_swiglu(x[-1:], w)[0], got[-1])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M,N,K", [(1, 1024, 1024), (2, 40, 1032), (8, 1000, 4608), (9, 33, 1048), (64, 2368, 1024), (65, 65, 1025), (130, 300, 4099),
+                                   (450, 1024, 1024), (450, 1024, 4608), (20, 2372, 1024), (3, 2384, 4096), (33, 2000, 4616), (450, 2300, 1030),
+                                   (1030, 2304, 1028), (4, 9000, 256)])
+def test_gemm_simt_cut_into_stretches_of_k(k, dtype, M, N, K):
+    """Contractions with few outputs are summed in four stretches, a block of a cluster each or one after the other, in every form (and
+    some that are not cut): the same bits alone and in any batch, with a bias and summed into what is there, within the bound of K
+    float32 sums."""
+    a = rnd((M, K), 5, dtype).cuda()
+    w = rnd((N, K), 6, dtype, 0.1).cuda()
+    bias, old = rnd((N,), 7, torch.float32).cuda(), rnd((M, N), 8, torch.float32).cuda()
+    ref = a.double() @ w.double().T
+    sums = K * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T) + 1e-30
+    got = k.gemm_simt(a, w, out_dtype=torch.float32)
+    assert ((got.double() - ref).abs() <= sums).all()
+    for r in sorted({0, M // 2, M - 1}):
+        assert torch.equal(k.gemm_simt(a[r:r + 1], w, out_dtype=torch.float32)[0], got[r])
+    wide = torch.empty((M, K + 3), dtype=dtype, device="cuda")[:, 3:]      # rows that no 16-byte load can take
+    wide.copy_(a)
+    assert torch.equal(k.gemm_simt(wide, w, out_dtype=torch.float32), got)
+    out = old.clone()
+    k.gemm_simt(a, w, out=out, accumulate=True, bias=bias)
+    terms = ref.abs() + 2 * bias.double().abs() + old.double().abs()
+    assert ((out.double() - (ref + bias.double() + old.double())).abs() <= sums + 2 * 2.0 ** -24 * terms).all()
