@@ -739,9 +739,14 @@ int launch_moe(const void* x, const int* tokens, const int* table, const void* w
   auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
   const bool vec_gu = D % 8 == 0 && D % per == 0 && aligned(w_gu);
   const bool vec_dn = F % 8 == 0 && F % per == 0 && aligned(w_down);
-  // Rows of bfloat16 in 16-byte pieces: each expert's matrix is read once per chunk of tokens.  Otherwise (float32, whose sums
-  // stay chains of float32 FMAs, and sizes or addresses without such pieces) once per pair.
-  const bool by_expert = sizeof(T) == 2 && top <= PAIRS_MAX;
+  // Rows of bfloat16 in 16-byte pieces: each expert's matrix is read once per chunk of tokens, where the model's sizes let that
+  // pay: every warp has four steps of 32 k (with fewer its work per expert is less than its bookkeeping), and a full chunk has two and a
+  // half pairs to an expert (with fewer the chunks of a larger step read nearly every expert each).  The step's tokens do not enter:
+  // a token's result is the same in any step.  Both kernels, microseconds once per pair / per expert: 16 experts of 2048 x 2048, top 2, 1 / 8
+  // / 64 tokens 41 / 18, 76 / 53, 413 / 121; 32 of 1024 x 1024, top 4, 30 / 14, 56 / 35, 233 / 138; 64 of 1024 x 1024, top 6, 49 / 18, 75 / 51,
+  // 317 / 408; 16 of 1024 x 512, top 2, 10 / 12, 18 / 21, 62 / 46; of 512 x 256 7 / 10, 9 / 12, 20 / 25.
+  const int chunks = ceil_div_i(n, top <= PAIRS_MAX ? PAIRS_MAX / top : 1), chunk = ceil_div_i(n, chunks);
+  const bool by_expert = sizeof(T) == 2 && top <= PAIRS_MAX && D >= 1024 && F >= 1024 && 2 * (PAIRS_MAX / top * top) >= 5 * n_experts;
   const bool up_by_expert = by_expert && vec_gu && aligned(x), down_by_expert = by_expert && vec_dn && aligned(h);
   // enough blocks to fill the GPU when the tokens are few, whole experts per block when they are many
   int units = F, outs = D;
@@ -782,10 +787,7 @@ int launch_moe(const void* x, const int* tokens, const int* table, const void* w
   ea.w = (const bf16*)w_gu; ea.route_w = route_w; ea.in_w = in_w; ea.status = status;
   ea.n = n; ea.D = D; ea.F = F; ea.top = top; ea.vocab = vocab; ea.n_experts = n_experts; ea.n_ident = n_ident; ea.il = il;
   ea.act = act; ea.accumulate = accumulate; ea.weight = in_w ? 1.0f : 1.0f / (float)top;
-  if (by_expert) {                 // as many tokens to a cluster as its pairs allow, every cluster (nearly) as many as any other
-    const int chunks = ceil_div_i(n, PAIRS_MAX / top);
-    ea.chunk = ceil_div_i(n, chunks);
-  }
+  ea.chunk = chunk;                // as many tokens to a cluster as its pairs allow, every cluster (nearly) as many as any other
   const bool few = n <= 8;         // then no expert has more than 8 rows (unless a table names one twice: another walk)
   if (up_by_expert) {
     if (act < 0) rc = few ? launch_experts<EXPERT_GATED, 1, 3>(ea, stream) : launch_experts<EXPERT_GATED, 2, 2>(ea, stream);
