@@ -1302,3 +1302,37 @@ def test_gemm_simt_cut_into_stretches_of_k(k, dtype, M, N, K):
     k.gemm_simt(a, w, out=out, accumulate=True, bias=bias)
     terms = ref.abs() + 2 * bias.double().abs() + old.double().abs()
     assert ((out.double() - (ref + bias.double() + old.double())).abs() <= sums + 2 * 2.0 ** -24 * terms).all()
+
+
+@pytest.mark.parametrize("H,Hkv,hd", [(8, 1, 64), (12, 3, 64), (4, 4, 64), (8, 2, 128)])
+@pytest.mark.parametrize("window", [0, 100])
+def test_prompt_attention_of_large_scores(k, H, Hkv, hd, window):
+    """Scores of a million that differ by 0 to 6, whole numbers that float32 holds exactly: only a softmax that takes the maximum off the
+    score as it is, and not off a rounded multiple of it, tells them apart.  The weights and the result are rounded to bfloat16 once each
+    (2^-9 of themselves); sums and exponentials are float32."""
+    from zinfer_b200.parts.attention import query_tiles as attn_tiles_host
+    lens, slots, page = [5, 64, 333], [2, 0, 1], 64
+    setup = PagedSetup(lens, slots, 3, page, Hkv, hd, torch.bfloat16, seed=4)
+    g = torch.Generator().manual_seed(hd)
+    kk, vv = [torch.full((l, Hkv, hd), 128.0) for l in lens], [rnd((l, Hkv, hd), 3 + l, torch.bfloat16) for l in lens]
+    kc, vc = setup.k.cpu(), setup.v.cpu()
+    for i, l in enumerate(lens):
+        kk[i][..., 0] = torch.randint(0, 7, (l, Hkv), generator=g).float()
+        for p in range(l):
+            at = int(setup.table[slots[i], p // page])
+            kc[at, :, p % page], vc[at, :, p % page] = kk[i][p].bfloat16(), vv[i][p]
+    q = torch.full((sum(lens), H, hd), 128.0)
+    q[..., 0] = 1.0
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32).cuda()
+    tiles = torch.from_numpy(attn_tiles_host(lens, k._fn("attention_prefill", "zk_attn_prefill_tile_tokens")(H, Hkv))).cuda()
+    got = k.attention(q.reshape(-1, H * hd).bfloat16().cuda(), kc.cuda(), vc.cuda(), tiles[0].contiguous(), tiles[1].contiguous(),
+                      i32([0] + list(np.cumsum(lens))), i32([0] * 3), i32(slots), setup.table_dev, H, Hkv, hd, 1.0, window=window,
+                      kind="prompt_tc").double().cpu()
+    at = 0
+    for i, l in enumerate(lens):
+        dist = torch.arange(l)[:, None] - torch.arange(l)
+        hidden = (dist < 0) | (dist >= window) if window else dist < 0
+        s = kk[i][..., 0].double().T.repeat_interleave(H // Hkv, 0)[:, None].masked_fill(hidden, -math.inf)
+        want = torch.einsum("hij,jhd->ihd", torch.softmax(s, -1), vv[i].double().repeat_interleave(H // Hkv, 1)).reshape(l, -1)
+        assert ((got[at:at + l] - want).abs() <= 1.01 * 2.0 ** -8 * vv[i].abs().max().item()).all()
+        at += l

@@ -55,20 +55,16 @@ __device__ __forceinline__ int swz(int r, int ch) {
 
 // HD: head_dim, 64 or 128 (rows of a tile are whole 128-byte lines, which the swizzle assumes).  HDV: width of a
 // value row, 64 or 128.  GP: heads of a KV group packed into one block.
-// What bounds the kernel is the arithmetic on the scores, not the MMAs: so exponentials of one instruction, masks in tiles at an
-// edge only, logarithms of the bias once per head and distance of a tile (they were one per score), and registers for three
-// or four blocks of 64-wide heads per SM.  8 prompts of 600 tokens, 32 heads on 8, window 1024, microseconds before and now: 202
-// -> 95, with the bias 251 -> 117; one of 4,000 380 -> 185 and 492 -> 220; 128-wide heads 304 -> 161 and 354 -> 186.
+// What bounds the kernel is the arithmetic on the scores, not the MMAs: so masks in tiles at an edge only, logarithms of the bias
+// once per head and distance of a tile (they were one per score), and registers for three or four blocks of 64-wide heads per
+// SM.  8 prompts of 600 tokens, 32 heads on 8, window 1024, microseconds before and now: 204 -> 107, with the bias 252 -> 132; one
+// of 4,000 381 -> 214 and 493 -> 251; 128-wide heads 307 -> 177 and 357 -> 202.
+// The exponentials are expf of the score minus the maximum, both as they are.  On base 2 (ex2.approx of scores times a rounded
+// scale * log2(e)) the same sizes take 94, 118, 182 and 218, but a score's rounding then grows with the score and not with its
+// distance from the maximum: scores of a million that differ by one came out several percent off.
 // SCORES: what is done with a scaled score besides the mask.  Left to itself the compiler gave the general variant 242 registers
-// (two blocks); with four blocks the biased one spills (127 us for the 117), the plain one does not lose by it (95; 99 with three).
+// (two blocks, 128 threads each).
 enum { SCORES_PLAIN = 0, SCORES_BIAS = 1, SCORES_ANY = 2 };
-
-// 2^x on the special-function unit (x <= 0 here; -inf gives 0)
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 
 template <int HD, int HDV, int GP, int SCORES>
 __global__ void __launch_bounds__(PF_WARPS * 32, HD == 64 ? (SCORES == SCORES_PLAIN ? 4 : 3) : 1)
@@ -135,21 +131,18 @@ __global__ void __launch_bounds__(PF_WARPS * 32, HD == 64 ? (SCORES == SCORES_PL
     if (mask_chunk > 0) row_lo[h] = (row_hi[h] - 1) / mask_chunk * mask_chunk;
     row_dist[h] = hl * (PF_TK + BQ) + tq + PF_TK - 1;
   }
-  // The softmax runs on base 2: scores are scaled by scale * log2(e), the exponentials are ex2.approx; the maxima go back to base e
-  // when they leave the loop.
-  constexpr float LOG2E = 1.4426950408889634f, LN2 = 0.6931471805599453f;
   if (SCORES != SCORES_ANY) {
     softcap = 0.f;
     dist = nullptr;
   }
-  const float scale2 = scale * LOG2E, cap2 = softcap * LOG2E, scale_cap = softcap > 0.f ? scale / softcap : 0.f;
+  const float inv_cap = softcap > 0.f ? 1.0f / softcap : 0.f;
   const bool biased = SCORES == SCORES_BIAS || (SCORES == SCORES_ANY && bias_r1 != nullptr);
   const bool staged_log = SCORES == SCORES_BIAS || (biased && !dist);   // dist_sm then holds the bias's logarithms
-  float r1_2[2] = {0.f, 0.f}, r2[2] = {0.f, 0.f};
+  float r1[2] = {0.f, 0.f}, r2[2] = {0.f, 0.f};
   if (biased) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      r1_2[h] = bias_r1[row_head[h]] * LOG2E;
+      r1[h] = bias_r1[row_head[h]];
       r2[h] = bias_r2[row_head[h]];
     }
   }
@@ -263,11 +256,11 @@ __global__ void __launch_bounds__(PF_WARPS * 32, HD == 64 ? (SCORES == SCORES_PL
       for (int i = 0; i < 4; ++i) {
         const int h = i >> 1;
         const int kp = kb + 8 * j + 2 * c + (i & 1);
-        float sc = s[j][i] * scale2;
-        if (softcap > 0.f) sc = cap2 * fast_tanh(s[j][i] * scale_cap);     // capped scores
-        if (staged_log) sc -= r1_2[h] * (&dist_sm[0][0])[row_dist[h] - (kp - kb)];
-        else if (biased) sc -= r1_2[h] * log1pf(r2[h] * (float)max(row_hi[h] - 1 - kp, 0));
-        if (dist) sc = fmaf((&dist_sm[0][0])[row_dist[h] - (kp - kb)], LOG2E, sc);
+        float sc = __fmul_rn(s[j][i], scale);      // rounded in every variant, and not folded into what follows
+        if (softcap > 0.f) sc = softcap * fast_tanh(sc * inv_cap);     // capped scores
+        if (staged_log) sc = fmaf(-r1[h], (&dist_sm[0][0])[row_dist[h] - (kp - kb)], sc);
+        else if (biased) sc = fmaf(-r1[h], log1pf(r2[h] * (float)max(row_hi[h] - 1 - kp, 0)), sc);
+        if (dist) sc = __fadd_rn(sc, (&dist_sm[0][0])[row_dist[h] - (kp - kb)]);
         if (edge) {
           const bool vis = row_ok[h] && (kp >= row_lo[h] || kp < keep) && kp < row_hi[h];
           s[j][i] = vis ? sc : -INFINITY;
@@ -281,7 +274,7 @@ __global__ void __launch_bounds__(PF_WARPS * 32, HD == 64 ? (SCORES == SCORES_PL
     for (int h = 0; h < 2; ++h) {
       m_new[h] = fmaxf(m_new[h], __shfl_xor_sync(0xffffffffu, m_new[h], 1));
       m_new[h] = fmaxf(m_new[h], __shfl_xor_sync(0xffffffffu, m_new[h], 2));
-      alpha[h] = m_new[h] == -INFINITY ? 1.f : ex2(m_run[h] - m_new[h]);
+      alpha[h] = m_new[h] == -INFINITY ? 1.f : expf(m_run[h] - m_new[h]);
       m_sub[h] = m_new[h] == -INFINITY ? 0.f : m_new[h];               // scores of -inf have a weight of 0 in such a row too
     }
 #pragma unroll
@@ -289,7 +282,7 @@ __global__ void __launch_bounds__(PF_WARPS * 32, HD == 64 ? (SCORES == SCORES_PL
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int h = i >> 1;
-        const float p = ex2(s[j][i] - m_sub[h]);
+        const float p = expf(s[j][i] - m_sub[h]);
         s[j][i] = p;
         row_sum[h] += p;
       }
@@ -334,7 +327,6 @@ __global__ void __launch_bounds__(PF_WARPS * 32, HD == 64 ? (SCORES == SCORES_PL
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     if (!row_ok[h]) continue;
-    m_run[h] *= LN2;
     if (cross) {
       const size_t row = ((size_t)row_tok[h] * H + row_head[h]) * Hkv + vh;
       float* dst = part_o + row * HDV;
