@@ -1336,3 +1336,23 @@ def test_prompt_attention_of_large_scores(k, H, Hkv, hd, window):
         want = torch.einsum("hij,jhd->ihd", torch.softmax(s, -1), vv[i].double().repeat_interleave(H // Hkv, 1)).reshape(l, -1)
         assert ((got[at:at + l] - want).abs() <= 1.01 * 2.0 ** -8 * vv[i].abs().max().item()).all()
         at += l
+
+
+@pytest.mark.parametrize("D,F,E,top,n", [(2048, 2048, 16, 2, 8), (1024, 1024, 16, 2, 64), (4104, 4104, 5, 2, 8), (1024, 4104, 4, 2, 9), (4104, 1032, 4, 2, 1)])
+def test_experts_of_few_rows_sum_in_float32(k, D, F, E, top, n):
+    """The products of an expert's second matrix against 64 bits on the hidden rows as they were stored.  A warp adds the sums of 32 products
+    one after the other, then come 8 warps, up to 4 blocks and `top` experts: each of these n additions, and the 32 products' own
+    sum, rounds to nearest, 2^-24 / sqrt(3) of partial sums that are no larger than the whole.  (The tensor core's own accumulator cuts
+    off instead of rounding: over 32 steps of k it is 2 to 5 times further off.)"""
+    x, w1 = rnd((n, D), 1, torch.bfloat16).cuda(), rnd((E, 2 * F, D), 2, torch.bfloat16, D ** -0.5).cuda()
+    w2 = rnd((E, D, F), 3, torch.bfloat16, F ** -0.5).cuda()
+    g = torch.Generator().manual_seed(n)
+    ids = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(n)]).int().cuda()
+    wts, status = (torch.rand((n, top), generator=g) + 0.1).cuda(), k.status_word("cuda")
+    h, y = torch.empty((n, top, F), dtype=torch.bfloat16, device="cuda"), torch.empty((n, D), device="cuda")
+    k._check(k._fn("moe", "zk_moe_routed")(k._ptr(x), k._ptr(ids), k._ptr(wts), k._ptr(w1), 0, k._ptr(w2), k._ptr(h), k._ptr(y), n, D, F, top, E, 0,
+                                           k.dtype_code(x.dtype), k._ptr(status), 0, -1, 0, k._stream()), "moe_routed")
+    ref = torch.stack([sum(wts[t, j].double() * (w2[int(ids[t, j])].double() @ h[t, j].double()) for j in range(top)) for t in range(n)])
+    additions = -(-F // 256) + 8 + 4 + top + 1
+    assert ((y.double() - ref).norm() / ref.norm()).item() <= 2.0 ** -24 * (additions / 3) ** 0.5
+    assert int(status.item()) == 0

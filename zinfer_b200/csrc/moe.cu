@@ -219,7 +219,9 @@ namespace {
 // each matrix once from memory, so here a block owns 16 output units (hidden units, or outputs) of EVERY expert: it sorts
 // the step's pairs by expert in shared memory, walks the experts that have any, reads 16 rows of each once, straight into the
 // fragments of mma.m16n8k16, and multiplies them with up to 16 of the expert's rows (8 to a fragment).  The products of
-// bfloat16 values are exact and the sums float32, as before.  A lane takes 16 contiguous bytes of a weight row and of an
+// bfloat16 values are exact.  The tensor core adds up 32 of them; those sums are added in float32, rounded to nearest, because its own
+// accumulator cuts off: carried over all of a warp's k it was 1.7e-7 of the result off for K = 1024 to 4096 and 6.1e-7 with 16
+// steps of k a warp (K = 4104), where the kernels above are 0.9e-7 to 1.25e-7 off.  A lane takes 16 contiguous bytes of a weight row and of an
 // input row for two MMAs; both use the same order of k inside 32, which a sum does not see.  K is split over the block's
 // warps; where that leaves SMs idle, a cluster's blocks split K further (`k_parts`, while every warp keeps 128 k or more: what a
 // warp does per expert besides must pay) and then share the experts out among themselves.  The loads of the next expert are
@@ -255,11 +257,12 @@ __device__ __forceinline__ uint4 ld_weights(const bf16* p) {
   return v;
 }
 
-__device__ __forceinline__ void mma_bf16(float c[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+// d = A B + c
+__device__ __forceinline__ void mma_bf16(float d[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1, const float c[4]) {
   asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
 }
 
 __device__ __forceinline__ float ld_cluster(const float* local, unsigned rank) {
@@ -429,8 +432,12 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const Ex
         for (int t = 0; t < TILES; ++t)
 #pragma unroll
           for (int u = 0; u < NG; ++u) {
-            mma_bf16(acc[t][u], st.w[t][0].x, st.w[t][1].x, st.w[t][0].y, st.w[t][1].y, st.x[u].x, st.x[u].y);
-            mma_bf16(acc[t][u], st.w[t][0].z, st.w[t][1].z, st.w[t][0].w, st.w[t][1].w, st.x[u].z, st.x[u].w);
+            const float none[4] = {0.f, 0.f, 0.f, 0.f};
+            float sum[4];                          // of these 32 k
+            mma_bf16(sum, st.w[t][0].x, st.w[t][1].x, st.w[t][0].y, st.w[t][1].y, st.x[u].x, st.x[u].y, none);
+            mma_bf16(sum, st.w[t][0].z, st.w[t][1].z, st.w[t][0].w, st.w[t][1].w, st.x[u].z, st.x[u].w, sum);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[t][u][j] += sum[j];
           }
         fetch(ring[r]);
         if (++s < s1) continue;
