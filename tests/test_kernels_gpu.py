@@ -1356,3 +1356,110 @@ def test_experts_of_few_rows_sum_in_float32(k, D, F, E, top, n):
     additions = -(-F // 256) + 8 + 4 + top + 1
     assert ((y.double() - ref).norm() / ref.norm()).item() <= 2.0 ** -24 * (additions / 3) ** 0.5
     assert int(status.item()) == 0
+
+
+def _recurrence(k, kind, lens, H, d, e, seed):
+    """Inputs of one of the four gated recurrences: (run, o, bound), run(sequences) giving the kernel's outputs and states for those
+    sequences, o in 64 bits for all.  The bound: d products and T updates of the absolute terms, each with the few ulp of its gates (the
+    exponentials of `capped` take arguments of up to 15, hence 16 ulp more)."""
+    g = torch.Generator().manual_seed(seed)
+    r = lambda *s: torch.randn(s, generator=g)
+    n, B, cu = sum(lens), len(lens), [0] + [int(x) for x in np.cumsum(lens)]
+    rows, state = r(n, H * (2 * d + e)) * d ** -0.25, r(B, H, d, e) * 0.1
+    a, b, z, z2 = r(H), r(H), r(n, H), r(n, H) + 2.0
+    f_bias, lower = r(H * d), torch.rand((H * d,), generator=g) * 0.9
+    q, f, v = (t.double() for t in (rows[:, :H * d], rows[:, H * d:2 * H * d], rows[:, 2 * H * d:]))
+    if kind == "stepped":                                # a row is [values | keys | queries]
+        rows = torch.cat([rows[:, 2 * H * d:], rows[:, H * d:2 * H * d], rows[:, :H * d]], 1)
+    stored = torch.zeros((B, k.mlstm_state_floats(H, d, e))) if kind == "capped" else state.reshape(B, -1)
+
+    def run(seqs):
+        seqs = list(seqs)
+        at = torch.cat([torch.arange(cu[s], cu[s + 1]) for s in seqs])
+        counts, st = [lens[s] for s in seqs], stored[seqs].clone().cuda()
+        i32, c = (lambda x: torch.tensor(x, dtype=torch.int32).cuda()), (lambda t: t.contiguous().cuda())
+        own = c(rows[at])
+        where = (i32([0] + [int(x) for x in np.cumsum(counts)]), i32(list(range(len(seqs)))), len(seqs), H)
+        if kind == "gated":
+            out = [k.hgrn2_scan(own, c(f_bias), c(lower), st, *where, d, e)]
+        elif kind == "keyed":
+            out = [k.retention_scan(own, c(0.5 + 0.5 * torch.sigmoid(a)), None, 0, 1.0, i32([p for m in counts for p in range(m)]), st, *where, d, e)]
+        elif kind == "stepped":
+            out = [k.ssd_scan(own, c(z[at]), c(a - 1), c(0.3 * b - 1), c(b), st, *where, H, d, e)]
+        else:
+            out = list(k.mlstm_scan(own, c(z[at]), c(z2[at]), c(a), c(b), 15.0, st, *where, d, e))
+        return [x.cpu() for x in out] + [st.cpu()]
+
+    if kind == "gated":
+        q = q * torch.sigmoid(q)
+        f = lower.double() + (1 - lower.double()) * torch.sigmoid(f + f_bias.double())
+    q, f, v = q.reshape(n, H, d), f.reshape(n, H, d), v.reshape(n, H, e)
+    if kind == "capped":
+        v = torch.cat([v, torch.ones((n, H, 1), dtype=torch.float64)], -1)
+    ref, bound = torch.empty_like(v), torch.empty_like(v)
+    for s in range(B):
+        S = torch.zeros((H, d, e + 1), dtype=torch.float64) if kind == "capped" else state[s].double()
+        A, m = S.abs(), torch.zeros(H, dtype=torch.float64)
+        for t in range(cu[s], cu[s + 1]):
+            if kind == "gated":
+                keep, new, most = f[t][..., None], (1 - f[t])[..., None] * v[t][:, None], (1 + f[t])[..., None] * v[t][:, None].abs()
+            else:
+                if kind == "keyed":
+                    keep, by = 0.5 + 0.5 * torch.sigmoid(a.double()), torch.ones(H, dtype=torch.float64)
+                elif kind == "stepped":
+                    by = torch.nn.functional.softplus(z[t].double() + a.double() - 1)
+                    keep = torch.exp(-torch.exp(0.3 * b.double() - 1) * by)
+                else:
+                    li = 15 * torch.tanh((z[t] + a).double() / 15)
+                    lf = torch.nn.functional.logsigmoid(15 * torch.tanh((z2[t] + b).double() / 15))
+                    m_new = torch.maximum(lf + m, li)
+                    keep, by, m = torch.exp(lf + m - m_new), torch.exp(li - m_new), m_new
+                keep, new = keep[:, None, None], by[:, None, None] * f[t][..., None] * v[t][:, None]
+                most = new.abs()
+            S, A = keep * S + new, keep * A + most
+            extra = b.double()[:, None] * v[t] if kind == "stepped" else torch.zeros_like(v[t])
+            ref[t] = (S * q[t][..., None]).sum(1) + extra
+            ulps = d + 8 + (24 if kind == "capped" else 8) * (t - cu[s] + 1)
+            bound[t] = ulps * 2.0 ** -23 * ((A * q[t].abs()[..., None]).sum(1) + extra.abs())
+    return run, ref.reshape(n, -1), bound.reshape(n, -1)
+
+
+@pytest.mark.parametrize("d,e", [(24, 40), (40, 40), (64, 33), (100, 72), (128, 64), (200, 48)])
+@pytest.mark.parametrize("kind", ["gated", "keyed", "stepped", "capped"])
+def test_recurrences_with_more_blocks_than_sms(k, kind, d, e):
+    """4 to 32 channels a warp: with more blocks than SMs the variant runs that leaves registers for two blocks an SM, a sequence alone
+    takes the other.  Unequal lengths, columns that are no whole block: the same bits alone and in the batch, outputs and states, and
+    the outputs within their bound of 64 bits."""
+    lens, H = [33, 1, 16, 17, 2, 40, 15, 1, 31, 5, 48], 8
+    run, ref, bound = _recurrence(k, kind, lens, H, d, e, d + e)
+    everyone = run(range(len(lens)))
+    assert 148 < len(lens) * H * -(-(e + (kind == "capped")) // 32) <= 296
+    assert ((everyone[0].double() - ref).abs() <= bound).all()
+    for s in (0, 1, 5, 10):
+        at, alone = slice(sum(lens[:s]), sum(lens[:s + 1])), run([s])
+        assert torch.equal(alone[-1][0], everyone[-1][s])
+        for x, y in zip(alone[:-1], everyone[:-1]):
+            assert torch.equal(x, y[at])
+
+
+@pytest.mark.parametrize("d", [32, 64, 128, 256])
+def test_gated_recurrence_adds_channels_in_order(k, d):
+    """A warp adds its channels one after the other into one float32 sum, whatever the registers pack: with one token, a gate of 0.5 and a
+    state of zero, o = sum_w ((q_0 S_0) + q_1 S_1 + ...) with fused multiply-adds, which 64 bits rounded after every step give exactly
+    for inputs of 8 bits."""
+    H, e, g = 2, 40, torch.Generator().manual_seed(d)
+    per = d // 8
+    keys, vals = (torch.randint(-127, 128, s, generator=g).float() * c for s, c in (((H, d), 2.0 ** -6), ((H, e), 2.0 ** -5)))
+    qs = torch.randint(-127, 128, (H, d), generator=g).float() * torch.exp2(torch.randint(-12, 12, (H, d), generator=g).float())
+    rows = torch.cat([qs.reshape(1, -1), keys.reshape(1, -1), vals.reshape(1, -1)], 1).cuda()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32).cuda()
+    state = torch.zeros((1, H * d * e), device="cuda")
+    got = k.retention_scan(rows, torch.full((H,), 0.5).cuda(), None, 0, 1.0, i32([0]), state, i32([0, 1]), i32([0]), 1, H, d, e).cpu()
+    S = keys[:, :, None] * vals[:, None]                 # products of 7-bit whole numbers: exact
+    total = torch.zeros((H, e))
+    for w in range(8):
+        acc = torch.zeros((H, e))
+        for i in range(w * per, (w + 1) * per):
+            acc = (acc.double() + qs[:, i, None].double() * S[:, i].double()).float()
+        total = total + acc
+    assert torch.equal(got.reshape(H, e), total)

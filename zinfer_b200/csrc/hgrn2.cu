@@ -128,11 +128,13 @@ __device__ __forceinline__ Pair mul2(Pair a, Pair b) {
   return d;
 }
 
+template <int N> struct Count { static constexpr int value = N; };
+
 // DPT: channels per warp; TT: tokens staged at once (sixteen, or eight or four where more do not fit shared memory).
 // REC_KEYED: the recurrence of a retention layer instead, S_t = decay_h S_{t-1} + k_t v_t^T with one fixed decay per head
 // (`decay` [H]); the row's second part then holds the keys k_t in place of the gates.
-// BLOCKS: how many of them an SM is to hold.
-template <int DPT, int TT, int REC, int BLOCKS>
+// BLOCKS: how many of them an SM is to hold.  SIDE: tokens of a whole group that are worked on side by side, each with a sum of its own.
+template <int DPT, int TT, int REC, int BLOCKS, int SIDE = 1>
 __global__ void __launch_bounds__(HG_R * 32, BLOCKS)
     hgrn2_scan_kernel(const float* __restrict__ qfv, int ld, float* __restrict__ state, long long state_stride,
                       float* __restrict__ o, const int* __restrict__ cu_q, const int* __restrict__ seq_slot, int H, int d,
@@ -258,53 +260,69 @@ __global__ void __launch_bounds__(HG_R * 32, BLOCKS)
     const int nt = min(TT, t1 - tb);
     const bool more = tb + TT < t1;
     if (more) fetch(tb + TT);       // under way while this group is worked on
-    auto token = [&](int tt) {
-      float v = v_cur[tt], keep = dk;
-      float acc = 0.f;
-      if (REC == REC_STEPPED) {
-        if (warp == 0) acc = skip * v;
-        keep = __shfl_sync(0xffffffffu, lane_decay, tt);
-        v *= __shfl_sync(0xffffffffu, lane_dt, tt);
-      }
-      if (REC == REC_CAPPED) {
-        keep = __shfl_sync(0xffffffffu, lane_decay, tt);
-        v *= __shfl_sync(0xffffffffu, lane_dt, tt);
+    auto tokens = [&](int first_tt, auto count) {
+      constexpr int N = decltype(count)::value;
+      float v[N], keep[N], acc[N];
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const int tt = first_tt + i;
+        v[i] = v_cur[tt];
+        keep[i] = dk;
+        acc[i] = 0.f;
+        if (REC == REC_STEPPED) {
+          if (warp == 0) acc[i] = skip * v[i];
+          keep[i] = __shfl_sync(0xffffffffu, lane_decay, tt);
+          v[i] *= __shfl_sync(0xffffffffu, lane_dt, tt);
+        }
+        if (REC == REC_CAPPED) {
+          keep[i] = __shfl_sync(0xffffffffu, lane_decay, tt);
+          v[i] *= __shfl_sync(0xffffffffu, lane_dt, tt);
+        }
       }
       if constexpr (DPT % 4 == 0) {
-        const Pair v2 = pair(v, v), nv2 = pair(-v, -v), keep2 = pair(keep, keep);
-        Pair acc2 = pair(acc, 0.f);
 #pragma unroll
         for (int k4 = 0; k4 < DPT; k4 += 4) {
-          const ulonglong2 f4 = *reinterpret_cast<const ulonglong2*>(&fs[buf][tt][row0 + k4]);
-          const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(&qs[buf][tt][row0 + k4]);
-          const Pair ff[2] = {f4.x, f4.y}, qq[2] = {q4.x, q4.y};
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            Pair& s2 = S2[k4 / 2 + j];
-            if (REC != REC_GATED) s2 = fma2(keep2, s2, mul2(ff[j], v2));   // decay S + k v
-            else s2 = fma2(ff[j], s2, fma2(ff[j], nv2, v2));               // f S + (1 - f) v
-            acc2 = fma2(s2, qq[j], acc2);
+          for (int i = 0; i < N; ++i) {
+            const int tt = first_tt + i;
+            const Pair v2 = pair(v[i], v[i]), nv2 = pair(-v[i], -v[i]), keep2 = pair(keep[i], keep[i]);
+            const ulonglong2 f4 = *reinterpret_cast<const ulonglong2*>(&fs[buf][tt][row0 + k4]);
+            const float4 q4 = *reinterpret_cast<const float4*>(&qs[buf][tt][row0 + k4]);
+            const Pair ff[2] = {f4.x, f4.y};
+            const float qq[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              Pair& s2 = S2[k4 / 2 + j];
+              if (REC != REC_GATED) s2 = fma2(keep2, s2, mul2(ff[j], v2));   // decay S + k v
+              else s2 = fma2(ff[j], s2, fma2(ff[j], nv2, v2));               // f S + (1 - f) v
+              acc[i] = fmaf(first(s2), qq[2 * j], acc[i]);                   // one sum, in the order of the channels
+              acc[i] = fmaf(second(s2), qq[2 * j + 1], acc[i]);
+            }
           }
         }
-        acc = first(acc2) + second(acc2);
       } else {
 #pragma unroll
-        for (int k = 0; k < DPT; ++k) {
-          const float f = fs[buf][tt][row0 + k];
-          if (REC != REC_GATED) S[k] = fmaf(keep, S[k], f * v);
-          else S[k] = fmaf(f, S[k], fmaf(-f, v, v));
-          acc = fmaf(S[k], qs[buf][tt][row0 + k], acc);
+        for (int i = 0; i < N; ++i) {
+          const int tt = first_tt + i;
+#pragma unroll
+          for (int k = 0; k < DPT; ++k) {
+            const float f = fs[buf][tt][row0 + k];
+            if (REC != REC_GATED) S[k] = fmaf(keep[i], S[k], f * v[i]);
+            else S[k] = fmaf(f, S[k], fmaf(-f, v[i], v[i]));
+            acc[i] = fmaf(S[k], qs[buf][tt][row0 + k], acc[i]);
+          }
         }
       }
-      part[tt][warp][lane] = acc;
+#pragma unroll
+      for (int i = 0; i < N; ++i) part[first_tt + i][warp][lane] = acc[i];
     };
     if (nt == TT) {          // a whole group: no branch between the tokens, so their loads and sums interleave
 #pragma unroll
-      for (int tt = 0; tt < TT; ++tt) token(tt);
+      for (int tt = 0; tt < TT; tt += SIDE) tokens(tt, Count<SIDE>{});
     } else {
 #pragma unroll
       for (int tt = 0; tt < TT; ++tt)
-        if (tt < nt) token(tt);
+        if (tt < nt) tokens(tt, Count<1>{});
     }
     __syncthreads();
 #pragma unroll
@@ -336,16 +354,27 @@ __global__ void __launch_bounds__(HG_R * 32, BLOCKS)
 
 namespace {
 
-// With 8 to 32 channels a warp the kernel takes 128 to some 140 registers, which leaves an SM one block.  Where there are more blocks
-// than SMs two of them are worth the few values that then spill; a few long sequences are a chain that the spills lengthen.
-// Microseconds, one float32 value to an instruction / two values with one block / two values with two: 16 heads of 128 x 128, 8 x 600
-// tokens 410 / 389 / 345, 64 single tokens 90 / 88 / 58, 1 x 4,000 tokens 627 / 605 / 1025; of 64 x 64, 64 single tokens
-// @@H64@@.
+// Which of the variants, all of which give the same bits.  From 16 channels a warp on the kernel takes 186 to 234 registers, which
+// leaves an SM one block of 256 threads; with 8 channels the STEPPED and the CAPPED recurrence take 136 and 140.  Where there are
+// more blocks than SMs, two of them beside each other are worth the few values that then spill; up to an SM each, one block is the
+// faster.  GATED and KEYED with 8 channels fit two as they are; while there is a block per SM at most, a warp's chain of sums is what they
+// wait for, and two tokens side by side (142 registers) hide it.
+// Microseconds of a step, 16 heads, one float32 value to an instruction / one block an SM / two:
+//   GATED 128 x 128, sequences of 600 tokens: 4 (256 blocks) 203 / 194 / 174, 5 301 / 287 / 267, 8 410 / 393 / 348, 1 99 / 94 / 160; 64 single
+//   tokens 90 / 77 / 59; 1 x 4,000 628 / 597 / 1029, 5 x 4,000 1956 / 1869 / 1760;
+//   8 x 600, 128 x 128: KEYED 375 / 344 / 308, STEPPED 420 / 362 / 326, CAPPED 533 / 484 / 400; 256 x 128: GATED 738 / 717 / 629, CAPPED 920 / 863 / 689;
+//   16 x 600, 64 x 64: STEPPED 233 / 315 / 224, CAPPED 266 / 363 / 255.
+// GATED 64 x 64, one token after the other / two side by side: 1 x 600 tokens 91 / 59, 1 x 4,000 577 / 364, 16 x 600 216 / 266.
 template <int DP, int REC>
 auto scan_kernel(dim3 grid) {
   constexpr int TT = DP > 32 ? 4 : (DP > 16 ? 8 : 16);
-  if constexpr (DP >= 8 && DP <= 32)
-    if ((long long)grid.x * grid.y * grid.z > 148) return hgrn2_scan_kernel<DP, TT, REC, 2>;
+  constexpr bool light = DP == 8 && (REC == REC_GATED || REC == REC_KEYED);
+  const bool waits = (long long)grid.x * grid.y * grid.z > 148;        // some blocks wait for an SM if each wants one for itself
+  if constexpr (light) {
+    if (!waits) return hgrn2_scan_kernel<DP, TT, REC, 1, 2>;
+  } else if constexpr (DP >= 8 && DP <= 32) {
+    if (waits) return hgrn2_scan_kernel<DP, TT, REC, 2>;
+  }
   return hgrn2_scan_kernel<DP, TT, REC, 1>;
 }
 
