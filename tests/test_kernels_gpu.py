@@ -1104,11 +1104,11 @@ def test_gemm_tc_gated_units_over_the_whole_range(k, M, splits, glu):
 
 @pytest.mark.parametrize("D,F,E,top,n", [(1024, 1032, 5, 2, 1), (1032, 1024, 3, 3, 8), (2048, 1032, 4, 2, 9), (1024, 2048, 16, 2, 64), (1040, 1056, 6, 4, 33),
                                          (1024, 1032, 40, 8, 10), (1024, 1024, 2, 1, 129), (1024, 1032, 34, 33, 5), (3208, 1024, 4, 2, 3),
-                                         (1024, 1016, 5, 2, 2), (48, 1032, 130, 8, 16)])
+                                         (1024, 4104, 4, 2, 5), (4104, 1032, 4, 2, 9), (1024, 1016, 5, 2, 2), (48, 1032, 130, 8, 16)])
 @pytest.mark.parametrize("kind", ["table", "routed", "ungated", "weight_in"])
 def test_experts_of_few_rows(k, D, F, E, top, n, kind):
     """The bfloat16 kernels that read an expert's weights once for all of its rows (from 1,024 k; the last two sizes go to the others):
-    output units beyond the last 16, K of no whole 32, clusters of 1 to 8, experts with no row, one, more than 8 and more than
+    output units beyond the last 16, K of no whole 32, clusters of 1 to 4 that split K, the experts or both, experts with no row, one, more than 8 and more than
     16, tokens cut at 128 pairs, identity experts, a table that names an expert twice.  The bound: two float32 sums (K 2^-23 of
     the absolute terms), the unit's slope of at most 1.1 and its own few ulp, one rounding of h to bfloat16 (2^-8)."""
     g = torch.Generator().manual_seed(D + F + n)

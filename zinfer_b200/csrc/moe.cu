@@ -1,11 +1,12 @@
 // Mixture of small gated feed-forwards whose experts are picked by a TABLE indexed with the token id
 // (no router): token t uses experts table[token_t][0 .. top), each with weight 1/top.
 //   y_t = (1/top) * sum_k W_down[e_k] (silu(W_gate[e_k] x_t) * (W_up[e_k] x_t))
-// Two weight-streaming kernels, for float32 and for rows that come in no 16-byte pieces.  (1) gate/up: one block per
+// Two weight-streaming kernels, which read an expert's rows once per (token, k) pair.  (1) gate/up: one block per
 // (token, k) and slice of the expert's hidden units; a warp owns a hidden unit at a time, its lanes walk the input row, sums
 // in float32, silu in float32.  (2) down: one block per token and slice of the outputs; the `top` experts are
-// added in the order of k, so a token's result does not depend on the rest of the batch.  bfloat16 rows in such pieces take
-// expert_rows_kernel instead, which reads an expert's weights once for all of its rows.
+// added in the order of k, so a token's result does not depend on the rest of the batch.  expert_rows_kernel, which reads an expert's
+// weights once for all of its rows, takes their place in bfloat16 models whose rows come in 16-byte pieces, with D and F of 1,024
+// and more and two and a half pairs or more to an expert in a full chunk of tokens (launch_moe has the rule and what it rests on).
 // Weights are stacked in the run dtype: gate and up as ONE tensor [experts, 2F, D] whose rows are
 // [gate (F) | up (F)] (il = 0) or groups of il gate rows followed by their il up rows (il > 0, the layout
 // the contraction kernels with an activation epilogue want), down as [experts, D, F]; x and h are the run
@@ -229,8 +230,7 @@ namespace {
 // memory and are added in the order of warps, then of blocks; a result depends on how K is split alone, which the
 // sizes of the model decide: not on the step's other tokens.  Everything a token needs is in one cluster, so its experts are
 // added in the order of k without another kernel.
-// 8 tokens with 2 of 16 experts each (10 different ones), D = F = 2048, one layer of a single-token step, microseconds before and
-// now: gate/up 50 -> 37 (174 MB of weights: 4.7 TB/s), both kernels 102 -> 71; the step 1.00 -> 0.79 ms.
+// 8 tokens with 2 of 16 experts each (11 different ones), D = F = 2048, both kernels in a chain: times to come.
 constexpr int PAIRS_MAX = 128;       // pairs a cluster takes (tokens are cut into grid.y chunks of PAIRS_MAX / top)
 
 enum { EXPERT_GATED = 0, EXPERT_UNGATED = 1, EXPERT_DOWN = 2 };
@@ -412,54 +412,50 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const Ex
     }
   };
 
-  if (s0 < s1) {
 #pragma unroll
-    for (int r = 0; r < RING; ++r) fetch(ring[r]);
-    float acc[TILES][NG][4];
+  for (int r = 0; r < RING; ++r) fetch(ring[r]);
+  float acc[TILES][NG][4];
 #pragma unroll
-    for (int t = 0; t < TILES; ++t)
+  for (int t = 0; t < TILES; ++t)
+#pragma unroll
+    for (int u = 0; u < NG; ++u)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[t][u][j] = 0.f;
+  int walk = share_w, s = s0;
+  while (walk < n_walks) {
+#pragma unroll
+    for (int r = 0; r < RING; ++r) {
+      if (walk >= n_walks) break;
+      const Stage& st = ring[r];
+#pragma unroll
+      for (int t = 0; t < TILES; ++t)
+#pragma unroll
+        for (int u = 0; u < NG; ++u) {
+          const float none[4] = {0.f, 0.f, 0.f, 0.f};
+          float sum[4];                          // of these 32 k
+          mma_bf16(sum, st.w[t][0].x, st.w[t][1].x, st.w[t][0].y, st.w[t][1].y, st.x[u].x, st.x[u].y, none);
+          mma_bf16(sum, st.w[t][0].z, st.w[t][1].z, st.w[t][0].w, st.w[t][1].w, st.x[u].z, st.x[u].w, sum);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[t][u][j] += sum[j];
+        }
+      fetch(ring[r]);
+      if (++s < s1) continue;
+      // this warp's share of the walk: rows g and g + 8 of each tile, columns 2c and 2c + 1 of each 8
+      const int first = walks[walk].x, last = walks[walk].y;
 #pragma unroll
       for (int u = 0; u < NG; ++u)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[t][u][j] = 0.f;
-    int walk = share_w, s = s0;
-    while (walk < n_walks) {
+        for (int j = 0; j < 4; ++j) {
+          const int p = first + u * 8 + 2 * c + (j & 1);
 #pragma unroll
-      for (int r = 0; r < RING; ++r) {
-        if (walk >= n_walks) break;
-        const Stage& st = ring[r];
-#pragma unroll
-        for (int t = 0; t < TILES; ++t)
-#pragma unroll
-          for (int u = 0; u < NG; ++u) {
-            const float none[4] = {0.f, 0.f, 0.f, 0.f};
-            float sum[4];                          // of these 32 k
-            mma_bf16(sum, st.w[t][0].x, st.w[t][1].x, st.w[t][0].y, st.w[t][1].y, st.x[u].x, st.x[u].y, none);
-            mma_bf16(sum, st.w[t][0].z, st.w[t][1].z, st.w[t][0].w, st.w[t][1].w, st.x[u].z, st.x[u].w, sum);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[t][u][j] += sum[j];
+          for (int t = 0; t < TILES; ++t) {
+            if (p < last) part[((size_t)warp * n_pairs + p) * LD + t * 16 + g + 8 * (j >> 1)] = acc[t][u][j];
+            acc[t][u][j] = 0.f;
           }
-        fetch(ring[r]);
-        if (++s < s1) continue;
-        // this warp's share of the walk: rows g and g + 8 of each tile, columns 2c and 2c + 1 of each 8
-        const int first = walks[walk].x, last = walks[walk].y;
-#pragma unroll
-        for (int u = 0; u < NG; ++u)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const int p = first + u * 8 + 2 * c + (j & 1);
-#pragma unroll
-            for (int t = 0; t < TILES; ++t) {
-              if (p < last) part[((size_t)warp * n_pairs + p) * LD + t * 16 + g + 8 * (j >> 1)] = acc[t][u][j];
-              acc[t][u][j] = 0.f;
-            }
-          }
-        s = s0;
-        walk += shares_w;
-      }
+        }
+      s = s0;
+      walk += shares_w;
     }
-  } else {                                         // fewer steps than warps: nothing of K is this warp's
-    for (int i = lane; i < n_pairs * LD; i += 32) part[(size_t)warp * n_pairs * LD + i] = 0.f;
   }
   __syncthreads();
   for (int i = tid; i < n_pairs * TILES * 16; i += MOE_WARPS * 32) {
@@ -700,14 +696,15 @@ __global__ void __launch_bounds__(MOE_WARPS * 32)
 
 namespace {
 
-// The cluster of one slice of 16 units: as many blocks as give (nearly) every SM two.  K is split over them while every warp keeps
-// four steps of 32 k, the rest share the experts.  The model's sizes alone decide, so that a token's sums are the same in every step.
+// The cluster of one slice of 16 units: as many blocks as give (nearly) every SM two, at most 4 for the 64 slices and more that
+// come here.  K is split over them while every warp keeps four steps of 32 k, the rest share the experts.  The model's sizes alone
+// decide, so that a token's sums are the same in every step.
 void expert_cluster(int units, int K, int& k_parts, int& blocks) {
   const int slices = ceil_div_i(units, 16), steps = ceil_div_i(K, 32);
   k_parts = 1;
-  while (k_parts < 8 && slices * k_parts < 200 && steps >= 8 * k_parts * MOE_WARPS) k_parts *= 2;
+  while (slices * k_parts < 200 && steps >= 8 * k_parts * MOE_WARPS) k_parts *= 2;
   blocks = k_parts;
-  while (blocks < 8 && slices * blocks < 200) blocks *= 2;
+  while (slices * blocks < 200) blocks *= 2;
 }
 
 template <int MODE, int NG, int RING>

@@ -9,8 +9,9 @@ per token: y_t += sigmoid(g . x_t) * Shared(x_t), the gate in float32 on the flo
 The experts' matrices are stacked at load (gate and up as one [experts, 2F, D] tensor in the layout of
 `SwiGLU`, down as [experts, D, F]).  Two ways to run, which agree to rounding:
 
-* few tokens (single-token steps): two weight-streaming kernels find a token's experts through the table
-  on the device (`ctx.tokens`), so the step needs nothing from the host and can be recorded;
+* few tokens (single-token steps): two kernels find a token's experts through the table on the device
+  (`ctx.tokens`), so the step needs nothing from the host and can be recorded; where the model's sizes let
+  that pay they read an expert's weights once for all of its rows, else once per (token, k);
 * many tokens (prompt steps): which expert a token takes is a function of its id alone, and the ids of a
   prompt step are known on the host when the step is packed (`ctx.host_tokens`).  The rows are gathered in
   the order of their experts, every expert's rows padded to whole tiles of 128, and ONE grouped tcgen05
@@ -30,8 +31,9 @@ from .base import FEED_FORWARDS, FeedForward, WeightSpec
 from .feedforward import ActMlp, SwiGLU
 from .linear import FUSION_GROUP, interleave_rows
 
-# From this many tokens on a step whose ids the host knows runs expert by expert.  Below it the streaming
-# kernels, which read an expert's weights once per (token, k), are faster than 2 launches per expert.
+# From this many tokens on a step whose ids the host knows runs expert by expert.  The line was drawn where 2 launches per expert
+# became faster than kernels that read an expert's weights once per (token, k); models whose few-row kernels read them once for
+# all rows of an expert have theirs somewhere above it.
 GROUPED_MIN_TOKENS = 96
 
 
