@@ -230,7 +230,8 @@ namespace {
 // memory and are added in the order of warps, then of blocks; a result depends on how K is split alone, which the
 // sizes of the model decide: not on the step's other tokens.  Everything a token needs is in one cluster, so its experts are
 // added in the order of k without another kernel.
-// 8 tokens with 2 of 16 experts each (11 different ones), D = F = 2048, both kernels in a chain: times to come.
+// 8 tokens with 2 of 16 experts each (11 different ones), D = F = 2048, both kernels in a chain: 77 us once per pair, 53 here (an
+// expert's three matrices are 25 MB: 5.2 TB/s).
 constexpr int PAIRS_MAX = 128;       // pairs a cluster takes (tokens are cut into grid.y chunks of PAIRS_MAX / top)
 
 enum { EXPERT_GATED = 0, EXPERT_UNGATED = 1, EXPERT_DOWN = 2 };
@@ -747,8 +748,9 @@ int launch_moe(const void* x, const int* tokens, const int* table, const void* w
   // pay: every warp has four steps of 32 k (with fewer its work per expert is less than its bookkeeping), and a full chunk has two and a
   // half pairs to an expert (with fewer the chunks of a larger step read nearly every expert each).  The step's tokens do not enter:
   // a token's result is the same in any step.  Both kernels, microseconds once per pair / per expert: 16 experts of 2048 x 2048, top 2, 1 / 8
-  // / 64 tokens 41 / 18, 76 / 53, 413 / 121; 32 of 1024 x 1024, top 4, 30 / 14, 56 / 35, 233 / 138; 64 of 1024 x 1024, top 6, 49 / 18, 75 / 51,
-  // 317 / 408; 16 of 1024 x 512, top 2, 10 / 12, 18 / 21, 62 / 46; of 512 x 256 7 / 10, 9 / 12, 20 / 25.
+  // / 64 tokens 41 / 18, 77 / 53, 413 / 123; 32 of 1024 x 1024, top 4, 31 / 14, 56 / 35, 234 / 140; 8 of 1024 x 4096, top 2, 60 / 18, 97 / 38, 427 / 95;
+  // where the rule says no, 64 of 1024 x 1024, top 6, 49 / 18, 75 / 51, 317 / 408; 16 of 1024 x 512, top 2, 10 / 12, 18 / 21, 62 / 46; of 512 x 256
+  // 7 / 10, 9 / 12, 20 / 25.
   const int chunks = ceil_div_i(n, top <= PAIRS_MAX ? PAIRS_MAX / top : 1), chunk = ceil_div_i(n, chunks);
   const bool by_expert = sizeof(T) == 2 && top <= PAIRS_MAX && D >= 1024 && F >= 1024 && 2 * (PAIRS_MAX / top * top) >= 5 * n_experts;
   const bool up_by_expert = by_expert && vec_gu && aligned(x), down_by_expert = by_expert && vec_dn && aligned(h);
