@@ -1463,3 +1463,32 @@ def test_gated_recurrence_adds_channels_in_order(k, d):
             acc = (acc.double() + qs[:, i, None].double() * S[:, i].double()).float()
         total = total + acc
     assert torch.equal(got.reshape(H, e), total)
+
+
+@pytest.mark.parametrize("act", ["silu", "relu"])
+@pytest.mark.parametrize("norm", [False, True])
+@pytest.mark.parametrize("F,K", [(4752, 2048), (7104, 4096), (8192, 2048), (9472, 2048), (10752, 2048), (10752, 4096)])
+def test_skinny_gated_units_in_both_kernels(k, F, K, norm, act):
+    """Gated units whose loads run on across tasks against the kernel whose blocks have a task at a time, which takes fewer units: the same
+    bits for the first and the last 4,096 units, 1 to 16 rows, with and without prepared norms, and for a row alone."""
+    w = rnd((2 * F, K), 5, torch.bfloat16, K ** -0.5).cuda()
+    x, nw = rnd((16, K), 1, torch.float32).cuda(), (1 + rnd((K,), 2, torch.float32, 0.1)).cuda()
+    rows = (lambda lo, hi: scaled_input(k, x[lo:hi].contiguous(), nw, 1e-6)) if norm else (lambda lo, hi: x[lo:hi].bfloat16())
+    for M in (1, 7, 8, 9, 16):
+        assert not k._fn("gemm_skinny", "zk_gemm_skinny_gated_streams")(M, 4096, K)
+        got = k.gemm_skinny_swiglu(rows(0, M), w, act)
+        assert torch.equal(got[:, :4096], k.gemm_skinny_swiglu(rows(0, M), w[:8192], act))
+        assert torch.equal(got[:, -4096:], k.gemm_skinny_swiglu(rows(0, M), w[-8192:], act))
+        assert torch.equal(got[-1:], k.gemm_skinny_swiglu(rows(M - 1, M), w, act))
+
+
+def test_which_gated_units_run_on_across_tasks(k):
+    """Only where a warp's stretch of K is whole groups of slabs, and where that saves half a round of blocks (of up to eight rows and K = 2048 in a
+    last round that is a quarter empty too): not with a full last round, as 9472 units of 2 x 296 tasks have."""
+    streams = k._fn("gemm_skinny", "zk_gemm_skinny_gated_streams")
+    for M in (1, 8, 9, 16):
+        assert streams(M, 5120, 2048) and streams(M, 10752, 2048) and streams(M, 6144, 4096)
+        for F, K in ((4736, 2048), (9344, 2048), (9472, 2048), (8192, 2304), (10752, 2560), (10752, 3072), (8192, 4096), (10752, 1024)):
+            assert not streams(M, F, K), (M, F, K)
+        assert bool(streams(M, 8192, 2048)) == bool(streams(M, 9600, 2048)) == bool(streams(M, 5120, 8192)) == (M <= 8)
+    assert not streams(17, 10752, 2048)

@@ -441,8 +441,8 @@ __global__ void __launch_bounds__(WARPS * 32, skinny_min_blocks(WARPS, NT, EPI))
 // the block that takes the place starts with an empty pipe; between two rounds of blocks nothing was under way.  Here every
 // slab's registers are filled with the slab U further on, of this task or the next, as soon as its MMAs are issued, so that a warp
 // has U slabs under way all the time, the sums' barrier and the epilogue included (the warps' sums have two buffers: one barrier a
-// task).  A task is 8 units, the gates on rows 0..7 of the fragment and their ups on rows 8..15.  The split of K over the
-// warps and every order of sums are skinny_kernel's: the same bits.
+// task).  A task is 8 units, the gates on rows 0..7 of the fragment and their ups on rows 8..15; a warp's stretch of K is whole
+// groups of U slabs.  The split of K over the warps and every order of sums are skinny_kernel's: the same bits.
 template <int NT, int U, int NORM_MODE>
 __global__ void __launch_bounds__(256, 2) skinny_stream_kernel(const Args a) {
   constexpr int WARPS = 8, RED_LD = NT * 8 + 1, TASK_COLS = 8;
@@ -453,9 +453,8 @@ __global__ void __launch_bounds__(256, 2) skinny_stream_kernel(const Args a) {
   const int g = lane >> 2, c = lane & 3;
   const int M = a.M, N = a.N, K = a.K;
   const int n_tasks = (N + TASK_COLS - 1) / TASK_COLS;
-  const int slabs = (K + 31) / 32, per = (slabs + WARPS - 1) / WARPS;
-  const int s_begin = warp * per, s_end = min(slabs, s_begin + per);
-  const int groups = (per + U - 1) / U;                    // of U slabs a task; what a warp has less is zeros
+  const int per = K / 32 / WARPS, groups = per / U;        // slabs, and groups of U slabs, that a warp has of a task
+  const int s_begin = warp * per;
   const uint4 zero = make_uint4(0, 0, 0, 0);
 
   uint4 wv[U][2];
@@ -467,10 +466,7 @@ __global__ void __launch_bounds__(256, 2) skinny_stream_kernel(const Args a) {
   };
   auto load_w = [&](int u, int task, int s) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const bool ok = task < n_tasks && s < s_end && s * 32 + 8 * c < K;
-      wv[u][h] = ok ? ld16_stream(w_task[h] + s * 32) : zero;
-    }
+    for (int h = 0; h < 2; ++h) wv[u][h] = task < n_tasks ? ld16_stream(w_task[h] + s * 32) : zero;
   };
   int task = blockIdx.x;
   aim(task);
@@ -515,7 +511,7 @@ __global__ void __launch_bounds__(256, 2) skinny_stream_kernel(const Args a) {
         for (int u = 0; u < XU; ++u)
 #pragma unroll
           for (int t = 0; t < NT; ++t)
-            xv[u][t] = xok[t] && s + u0 + u < s_end && (s + u0 + u) * 32 + 8 * c < K ? ld16(xrow[t] + (s + u0 + u) * 32) : zero;
+            xv[u][t] = xok[t] ? ld16(xrow[t] + (s + u0 + u) * 32) : zero;
 #pragma unroll
         for (int u = 0; u < XU; ++u) {
 #pragma unroll
@@ -643,19 +639,31 @@ int dispatch_plain_any(const Args& a, cudaStream_t stream) {
   return dispatch_plain<NORM_NONE, TC>(a, stream);
 }
 
+// Whether gated units run in skinny_stream_kernel: where its blocks, which share the tasks out in halves of skinny_kernel's, save half
+// a round of blocks (two per SM: a last round that is at most half full), and a warp's stretch of K is whole groups of slabs.  With a
+// stretch that is not (K = 2304: 9 slabs in groups of 8) half of what is under way is nothing, and the kernel takes up to 1.18 times
+// skinny_kernel's time.  Microseconds, skinny_kernel / this, 1 and 8 rows:
+//   K = 2048: 5120 units (24 of 296 in the last round) 9.6 / 7.6, 10.7 / 8.9; 7104 (148) 11.1 / 10.4, 12.0 / 11.9; 10752 (80 in the third)
+//   15.5 / 14.9, 18.0 / 15.9.  K = 4096: 5120 18.0 / 16.1, 19.2 / 17.8; 10752 30.0 / 27.8, 31.5 / 30.8.  K = 8192: 10752 58.8 / 56.7, 60.5 / 59.3.
+//   Last round fuller: K = 2048, 8192 units (216) 11.8 / 11.4, 12.7 / 12.1; 9344 (288) 12.9 / 12.7, 13.5 / 14.2; 9472 (all of it) 13.4 / 13.8, 14.4
+//   / 15.1; K = 4096, 8192 21.2 / 22.1, 22.4 / 24.0.  So up to three quarters full where a task is a single group of slabs.
+// With two groups of tokens the registers hold only four slabs under way, and the fuller the tokens the less that hides: 9 and 16 rows,
+// K = 2048: 5120 units 12.6 / 11.6, 12.8 / 12.4; 9600 (8 of 296 in the third round) 18.4 / 17.1, 19.2 / 20.3; 10752 (80) 20.2 / 19.3, 20.9 / 20.5;
+// 9472 15.1 / 15.3, 15.6 / 17.1; K = 4096: 6144 (88 in the second) 23.9 / 21.8, 24.3 / 22.9; 10752 36.4 / 34.7, 36.9 / 37.6.  So in the second round, or
+// in the third where that is an eighth full.
+bool gated_streams(int M, int N, int K) {
+  const int tasks = N / 16, places = 2 * 148, rest = tasks % places;
+  if (M > 16 || tasks <= places || rest == 0 || K % 2048) return false;
+  const bool half = 2 * rest <= places;
+  if (M <= 8) return K <= 8192 && (half || (K == 2048 && 4 * rest <= 3 * places));
+  return half && ((K <= 4096 && tasks < 2 * places) || (K == 2048 && tasks < 3 * places && 8 * rest >= places));
+}
+
 template <int RG, int EPI, int NORM_MODE>
 int dispatch_fused_mode(const Args& a, cudaStream_t stream) {
-  // Loads that run on across tasks need several slabs per warp and task (K), and rounds of blocks to run on across.  With two
-  // groups of tokens the registers hold only four slabs under way, which pays where the last round of skinny_kernel's blocks (two
-  // per SM) would leave most of the SMs idle.  Whole steps, us, skinny_kernel / this: the 2.6B shape (672 tasks of 32 rows for
-  // 296 places) 1 row 1164 / 1104, 8 rows 1312 / 1218, 16 rows 1655 / 1595; the 1.2B shape (512) 1 row 563 / 557 to 566, 8 rows
-  // 627 / 611 to 623, but 16 rows 778 / 790; the 350M shape (K = 1024, 288) 1 row 312 / 329.
   if constexpr (EPI == EPI_SWIGLU && NORM_MODE != NORM_FUSED) {
-    const int tasks = a.N / 16, places = 2 * 148;
-    if (a.K >= 2048 && tasks > places) {
-      if (a.M <= 8) return launch_stream<1, 8, NORM_MODE>(a, stream);
-      if (a.M <= 16 && 2 * (tasks % places) < places) return launch_stream<2, 4, NORM_MODE>(a, stream);
-    }
+    if (gated_streams(a.M, a.N, a.K))
+      return a.M <= 8 ? launch_stream<1, 8, NORM_MODE>(a, stream) : launch_stream<2, 4, NORM_MODE>(a, stream);
   }
   if (a.M <= 8) return launch<8, RG, 1, 4, EPI, NORM_MODE, bf16>(a, stream);
   if (a.M <= 16) return launch<8, RG, 2, 2, EPI, NORM_MODE, bf16>(a, stream);
@@ -687,6 +695,8 @@ extern "C" {
 
 int zk_gemm_skinny_max_m() { return 64; }
 int zk_gemm_skinny_fused_max_m() { return 16; }
+// Whether M rows against the gates and ups of F units run in skinny_stream_kernel (rows that come without a norm to apply).
+int zk_gemm_skinny_gated_streams(int M, int F, int K) { return gated_streams(M, F, K) ? 1 : 0; }
 
 // X [M, K] bfloat16 (or Xf [M, K] float32 + norm_w [K], eps: RMSNorm fused, M <= 16), W [N, K]
 // bfloat16 with K % 8 == 0 and 16-byte aligned rows; C [M, N] bfloat16 or float32.

@@ -95,6 +95,7 @@ _SIGNATURES = {
         "zk_gemm_skinny_conv": "pppfppppppp" + "iiiiiiil" + "pi" + "p",
         "zk_gemm_skinny_max_m": "",
         "zk_gemm_skinny_fused_max_m": "",
+        "zk_gemm_skinny_gated_streams": "iii",
     },
     "gemm_tc": {
         "zk_gemm_tc": "ppppiiiiiiiiii" + "pifppp" + "p" + "pi" + "ff" + "p",
