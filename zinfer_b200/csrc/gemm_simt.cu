@@ -21,11 +21,19 @@ namespace {
 //  * IN_TURN: one block all of them, where there are blocks enough.
 // Float32, microseconds with one accumulator per output and now: N = 1024, K = 4608, 1 / 8 / 64 / 256 / 450 rows 27 / 28 / 82 / 120 / 169 ->
 // 13 / 18 / 47 / 74 / 138; K = 1024, 16 / 450 rows 14 / 44 -> 12 / 41.  The error against 64 bits is smaller (four shorter sums): a model's
-// logits 6.1e-6 -> 4.4e-6.
+// logits 6.1e-6 -> 4.4e-6.  What it costs: from 500 rows on, where blocks are no longer few, IN_TURN is 1 to 5 % slower than one accumulator
+// (2,000 rows, N = 1024, K = 1024, bfloat16 120 -> 125 us), and some sizes of 7 to 48 rows are 3 to 7 % slower.
 constexpr int SEGMENTS = 4;
 enum { WHOLE = 0, BY_CLUSTER = 1, IN_TURN = 2 };
 
-__host__ __device__ inline int segment_of(int K) { return ((K + SEGMENTS - 1) / SEGMENTS + 63) / 64 * 64; }   // whole 16-byte pieces
+// Where stretch i of K begins: the 512-byte blocks of a row that gemm_few_kernel walks, shared out whole (K of 1,024 and more has at least
+// four of them).
+template <typename T>
+__host__ __device__ inline int stretch_at(int K, int i) {
+  constexpr int KC = 512 / (int)sizeof(T);
+  const int at = (K + KC - 1) / KC * i / SEGMENTS * KC;
+  return at < K ? at : K;
+}
 
 __device__ __forceinline__ float ld_cluster(const float* local, unsigned rank) {
   unsigned remote;
@@ -131,11 +139,11 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), TM * TN >= 64 ? 2 : 3)
   const int tid = threadIdx.x;
   const int tx = tid % TX, ty = tid / TX;
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int seg = MODE == WHOLE ? K_all : segment_of(K_all);
-  int K = min(seg, K_all);
+  constexpr bool RUN_ON = MODE == IN_TURN && TM * TN < 64 && PACKED;  // the k blocks under way run on from stretch to stretch
+  int K = MODE == IN_TURN && !RUN_ON ? stretch_at<T>(K_all, 1) : K_all;
   if constexpr (MODE == BY_CLUSTER) {
-    const int k0 = (int)cluster_rank() * seg;
-    K = min(seg, K_all - k0);                               // K_all > 3 seg where the form is taken
+    const int k0 = stretch_at<T>(K_all, (int)cluster_rank());
+    K = stretch_at<T>(K_all, (int)cluster_rank() + 1) - k0;
     A += k0;
     W += k0;
   }
@@ -180,9 +188,12 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), TM * TN >= 64 ? 2 : 3)
     }
   };
 
-  int buf = 0;
+  // PF k blocks are under way in registers; the body of PF rounds is unrolled so that each has registers of its own.  With small
+  // tiles they run on from one stretch to the next.  A thread with 64 sums has no registers left for them while it adds those up (2,000
+  // rows, N = 2304, K = 4608, float32: 930 us, 842 with every stretch begun anew).
+  int buf = 0, k_from = 0, k_to = RUN_ON ? stretch_at<T>(K_all, 1) : K;
   for (int turn = 0; turn < (MODE == IN_TURN ? SEGMENTS : 1); ++turn) {
-    if (MODE == IN_TURN && turn > 0) {                      // the stretch before goes to what is there; its buffers are free
+    if (MODE == IN_TURN && turn > 0) {                      // the stretch before goes to what is there
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -195,22 +206,28 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN), TM * TN >= 64 ? 2 : 3)
           *in_tile(i, j) = v;
           acc[i][2 * j] = acc[i][2 * j + 1] = make_float2(0.f, 0.f);
         }
-      A += seg;
-      W += seg;
-      K = min(seg, K_all - turn * seg);
-      __syncthreads();
-      buf = 0;
+      if (RUN_ON) {
+        k_from = k_to;
+        k_to = stretch_at<T>(K_all, turn + 1);
+      } else {
+        A += K;
+        W += K;
+        k_to = K = stretch_at<T>(K_all, turn + 1) - stretch_at<T>(K_all, turn);
+        __syncthreads();                                    // the buffers are free
+        buf = 0;
+      }
     }
-    // PF k blocks are under way in registers; the body of PF rounds is unrolled so that each has registers of its own
+    if (!RUN_ON || turn == 0) {
 #pragma unroll
-    for (int f = 0; f < PF; ++f) fetch(f * BK, f);            // beyond K: zeros
-    put(0, 0);
-    __syncthreads();
-    for (int kb0 = 0; kb0 < K; kb0 += PF * BK) {
+      for (int f = 0; f < PF; ++f) fetch(f * BK, f);        // beyond K: zeros
+      put(0, 0);
+      __syncthreads();
+    }
+    for (int kb0 = k_from; kb0 < k_to; kb0 += PF * BK) {
 #pragma unroll
       for (int f = 0; f < PF; ++f) {
         const int kb = kb0 + f * BK;
-        if (kb >= K) break;
+        if (kb >= k_to) break;
         fetch(kb + PF * BK, f);                               // this block's values are in shared memory since the round before
 #pragma unroll
         for (int k = 0; k < BK; ++k) {
@@ -341,6 +358,7 @@ __global__ void __launch_bounds__(FEW_ROWS * GROUPS)
     gemm_few_kernel(const T* __restrict__ A, const T* __restrict__ W, TC* __restrict__ C, const float* __restrict__ bias,
                     int M, int N, int K_all, int lda, int ldw, int ldc, int accumulate) {
   constexpr int THREADS = FEW_ROWS * GROUPS;
+  constexpr bool WALKS = MODE == BY_CLUSTER || (MODE == WHOLE && GROUPS <= 2);      // else a block has one task
   constexpr int PIECE = 16 / (int)sizeof(T), KC = 512 / (int)sizeof(T), LD = KC + PIECE;   // 512 bytes of a row per k block
   extern __shared__ __align__(16) unsigned char few_smem[];
   T* ring = reinterpret_cast<T*>(few_smem);
@@ -350,129 +368,103 @@ __global__ void __launch_bounds__(FEW_ROWS * GROUPS)
   const int first_task = blockIdx.x, task_step = gridDim.x;
   int K = K_all;
   if constexpr (MODE == BY_CLUSTER) {
-    const int seg = segment_of(K_all), k0 = (int)cluster_rank() * seg;
-    K = min(seg, K_all - k0);
+    const int k0 = stretch_at<T>(K_all, (int)cluster_rank());
+    K = stretch_at<T>(K_all, (int)cluster_rank() + 1) - k0;
     A += k0;
     W += k0;
   }
-  // k blocks of a task, seg_kb to a stretch (of which the last may have fewer)
-  const int seg = MODE == IN_TURN ? segment_of(K_all) : K, seg_kb = (seg + KC - 1) / KC;
-  const int n_kb = MODE == IN_TURN ? (SEGMENTS - 1) * seg_kb + (K - (SEGMENTS - 1) * seg + KC - 1) / KC : seg_kb;
-  auto place = [&](int kb, int& k, bool& in) {               // this lane's piece of k block kb, and whether it exists
-    if constexpr (MODE == IN_TURN) {
-      const int turn = kb / seg_kb, at = (kb - turn * seg_kb) * KC + (tid & 31) * PIECE;
-      k = turn * seg + at;
-      in = at < seg && k < K;
-    } else {
-      k = kb * KC + (tid & 31) * PIECE;
-      in = k < K;
-    }
-  };
+  const int n_kb = (K + KC - 1) / KC;                        // k blocks of a task
   // a warp copies whole rows (32 pieces of 16 bytes): lane = piece, warps take rows in turn
   const int e = (tid & 31) * PIECE;
-  auto request_w = [&](int task, int kb, int stage) {
+  auto request = [&](int task, int kb, int stage) {
     T* dst = ring + (size_t)stage * rows * LD + e;
-    const int n0 = task * FEW_ROWS;
-    int k;
-    bool k_in;                                               // K is a whole number of pieces
-    place(kb, k, k_in);
+    const int n0 = task * FEW_ROWS, k = kb * KC + e;
+    const bool k_in = k < K;                                 // K is a whole number of pieces
     const T* wk = W + (k_in ? k : 0);
+    const T* ak = A + (k_in ? k : 0);
 #pragma unroll
     for (int r = tid >> 5; r < FEW_ROWS; r += THREADS / 32) {
       const bool in = k_in && n0 + r < N;
       cp16(dst + r * LD, wk + (size_t)(in ? n0 + r : 0) * ldw, in);
     }
+    for (int r = tid >> 5; r < M; r += THREADS / 32) cp16(dst + (FEW_ROWS + r) * LD, ak + (size_t)r * lda, k_in);
   };
-  auto request_a = [&](int kb, int stage) {
-    T* dst = ring + ((size_t)stage * rows + FEW_ROWS) * LD + e;
-    int k;
-    bool k_in;
-    place(kb, k, k_in);
-    const T* ak = A + (k_in ? k : 0);
-    for (int r = tid >> 5; r < M; r += THREADS / 32) cp16(dst + r * LD, ak + (size_t)r * lda, k_in);
-  };
-  // the block that is requested next: its task, k block and stage
+  // Requests the k block that follows those under way: of a block that walks, the next of this task or of the one after it; else kb.
   int r_task = first_task, r_kb = 0, r_stage = 0;
-  auto advance = [&]() {
-    if (++r_kb == n_kb) {
-      r_kb = 0;
-      r_task += task_step;
+  auto request_next = [&](int kb) {
+    if constexpr (WALKS) {
+      if (r_task < tasks) request(r_task, r_kb, r_stage);
+      if (++r_kb == n_kb) {
+        r_kb = 0;
+        r_task += task_step;
+      }
+      if (++r_stage == STAGES) r_stage = 0;
+    } else {
+      if (kb < n_kb) request(first_task, kb, kb % STAGES);
     }
-    if (++r_stage == STAGES) r_stage = 0;
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
   // More than two rows: the next kernel's blocks, let in early, fell unevenly onto the SMs beside this one's ([8, 1024] x 3072 twenty
   // times in a row: 12.8 us, 10.9 without).  The weights are requested behind the wait too: nothing says that no kernel wrote them.
   if (GROUPS <= 2) zk_let_next_start();
   zk_wait_prior();
 #pragma unroll
-  for (int s = 0; s < STAGES - 1; ++s) {
-    if (r_task < tasks) {
-      request_w(r_task, r_kb, r_stage);
-      request_a(r_kb, r_stage);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    advance();
-  }
+  for (int s = 0; s < STAGES - 1; ++s) request_next(s);
   const int row = tid % FEW_ROWS, group = tid / FEW_ROWS;
   float acc[NT], total[MODE == IN_TURN ? NT : 1];
   int at[NT];                                                // where the rows of A lie in a stage
 #pragma unroll
   for (int t = 0; t < NT; ++t) at[t] = (FEW_ROWS + (group + t * GROUPS < M ? group + t * GROUPS : 0)) * LD;   // no such row: another's, not stored
   int stage = 0;
-  for (int task = first_task; task < tasks; task += task_step) {
+  for (int task = first_task; task < tasks; task += WALKS ? task_step : tasks) {
 #pragma unroll
     for (int t = 0; t < NT; ++t) acc[t] = 0.f;
-    for (int kb = 0, left = seg_kb, turn = 0; kb < n_kb; ++kb) {
-      if (MODE == IN_TURN && left == 0) {                    // a stretch ends
+    for (int turn = 0, kb = 0; turn < (MODE == IN_TURN ? SEGMENTS : 1); ++turn) {
+      const int stretch_end = MODE == IN_TURN ? n_kb * (turn + 1) / SEGMENTS : n_kb;
+      for (; kb < stretch_end; ++kb) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();                                     // the k block is here, and nobody reads the one before it
+        const T* st = ring + (size_t)(WALKS ? stage : kb % STAGES) * rows * LD;
+        float4 x[2][4], y[2][NT][4];
+        auto read = [&](int k, int b) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            x[b][i] = four(st + row * LD + k + 4 * i);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) y[b][t][i] = four(st + at[t] + k + 4 * i);
+          }
+        };
+        read(0, 0);
+        request_next(kb + STAGES - 1);
+#pragma unroll
+        for (int k = 0; k < KC; k += 16) {
+          const int b = (k >> 4) & 1;
+          if (k + 16 < KC) read(k + 16, b ^ 1);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+#pragma unroll
+            for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].x, x[b][i].x, acc[t]);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].y, x[b][i].y, acc[t]);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].z, x[b][i].z, acc[t]);
+#pragma unroll
+            for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].w, x[b][i].w, acc[t]);
+          }
+        }
+        if (WALKS && ++stage == STAGES) stage = 0;
+      }
+      if constexpr (MODE == IN_TURN) {                       // a stretch ends
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
           total[t] = turn ? total[t] + acc[t] : acc[t];
           acc[t] = 0.f;
         }
-        ++turn;
-        left = seg_kb;
       }
-      --left;
-      asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
-      __syncthreads();                                       // the k block is here, and nobody reads the one before it
-      const T* st = ring + (size_t)stage * rows * LD;
-      float4 x[2][4], y[2][NT][4];
-      auto read = [&](int k, int b) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          x[b][i] = four(st + row * LD + k + 4 * i);
-#pragma unroll
-          for (int t = 0; t < NT; ++t) y[b][t][i] = four(st + at[t] + k + 4 * i);
-        }
-      };
-      read(0, 0);
-      if (r_task < tasks) {
-        request_w(r_task, r_kb, r_stage);
-        request_a(r_kb, r_stage);
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      advance();
-#pragma unroll
-      for (int k = 0; k < KC; k += 16) {
-        const int b = (k >> 4) & 1;
-        if (k + 16 < KC) read(k + 16, b ^ 1);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-#pragma unroll
-          for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].x, x[b][i].x, acc[t]);
-#pragma unroll
-          for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].y, x[b][i].y, acc[t]);
-#pragma unroll
-          for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].z, x[b][i].z, acc[t]);
-#pragma unroll
-          for (int t = 0; t < NT; ++t) acc[t] = fmaf(y[b][t][i].w, x[b][i].w, acc[t]);
-        }
-      }
-      if (++stage == STAGES) stage = 0;
     }
     if constexpr (MODE == IN_TURN) {
 #pragma unroll
-      for (int t = 0; t < NT; ++t) acc[t] = total[t] + acc[t];
+      for (int t = 0; t < NT; ++t) acc[t] = total[t];
     }
     const int n = task * FEW_ROWS + row;
     if constexpr (MODE == BY_CLUSTER) {
@@ -570,7 +562,7 @@ int launch_few(const void* A, const void* W, void* C, const float* bias, int M, 
   // 8 rows, N = 65536, K = 1024, float32 75 and 114 us, 85 and 123 with blocks that stay.
   const int tasks = ceil_div_i(N, FEW_ROWS), clusters = MODE == BY_CLUSTER ? SEGMENTS : 1;
   const int per_sm = (int)(227 * 1024 / (smem + 1024)), at_once = 148 * (per_sm > 0 ? per_sm : 1) / clusters;
-  const int rounds = MODE == WHOLE && GROUPS > 2 ? 1 : ceil_div_i(tasks, at_once);
+  const int rounds = MODE == IN_TURN || (MODE == WHOLE && GROUPS > 2) ? 1 : ceil_div_i(tasks, at_once);
   return launch_cluster(kern, dim3(ceil_div_i(tasks, rounds), 1, clusters), FEW_ROWS * GROUPS, smem, clusters, true, stream,
                         (const T*)A, (const T*)W, (TC*)C, bias, M, N, K, lda, ldw, ldc, accumulate);
 }
@@ -578,7 +570,9 @@ int launch_few(const void* A, const void* W, void* C, const float* bias, int M, 
 template <int MODE, typename T, typename TC>
 int launch_few_rows(const void* A, const void* W, void* C, const float* bias, int M, int N, int K, int lda, int ldw, int ldc,
                     int accumulate, cudaStream_t stream) {
-  if (M <= 2) return launch_few<2, 1, 4, MODE, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
+  // One or two rows are blocks of a warp, whose bfloat16 products come faster than four stages fill: with three, seven blocks share an
+  // SM instead of five (2 rows, N = 65536, K = 1024: 59 us, 66 with four).
+  if (M <= 2) return launch_few<2, 1, sizeof(T) == 2 ? 3 : 4, MODE, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
   if (M <= 4) return launch_few<4, 1, 6, MODE, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
   if (M <= 8) return launch_few<8, 1, 6, MODE, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
   if (M <= 16) return launch_few<16, 1, 5, MODE, T, TC>(A, W, C, bias, M, N, K, lda, ldw, ldc, accumulate, stream);
@@ -601,9 +595,11 @@ int launch(const void* A, const void* W, void* C, const float* bias, int M, int 
   const bool little = M <= 8, narrow = tasks <= 2 * 148, whole = K * sizeof(T) >= 512;
   if (pieces && M <= FEW_MAX_M && (whole ? little || narrow : little && narrow)) {
     if (!split) return launch_few_rows<WHOLE, T, TC>(ZK_SIMT_ARGS);
-    // A cluster per 16 weight rows while those leave SMs idle, or while the rows are so few that the chain of k is all there is.
-    return tasks <= 74 || M <= (K >= 2048 ? 8 : 4) ? launch_few_rows<BY_CLUSTER, T, TC>(ZK_SIMT_ARGS)
-                                                   : launch_few_rows<IN_TURN, T, TC>(ZK_SIMT_ARGS);
+    // A cluster per 16 weight rows while those leave SMs idle, or while the rows are so few that the chain of k is all there is.  From 57
+    // rows on an SM holds one block, and 74 clusters of four no longer run in two rounds (64 rows, N = 1184, K = 1536, bfloat16: 47 us, 35 in
+    // turn); 8 rows, N = 2304, K = 4608, bfloat16: 32 us, 26 in turn.
+    const bool cluster = tasks <= (M > 56 ? 64 : 74) || M <= 2 || (M <= 4 && K >= 1536) || (M <= 8 && K >= 4096 && tasks <= 128);
+    return cluster ? launch_few_rows<BY_CLUSTER, T, TC>(ZK_SIMT_ARGS) : launch_few_rows<IN_TURN, T, TC>(ZK_SIMT_ARGS);
   }
   // The largest tile that still gives (nearly) every SM a block, and no taller than the rows need: 128 rows of A cost their
   // FMAs whether they exist or not (16 rows, N = 65536, K = 1024: 350 / 190 / 154, and 277 with one buffer).  450 rows, microseconds with 128 x 128 / 64 x 64 / 32 x 32
