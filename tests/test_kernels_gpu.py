@@ -1232,7 +1232,7 @@ def test_prompt_attention_variants_against_the_general_kernel(k, H, Hkv, hd, opt
     """The prompt kernel's three variants of the scores (plain, a staged bias, everything) on prompts of less than a tile, of
     whole tiles, behind a past, with tiles inside, at and beyond the edge of the window or stretch, against the general kernel on
     the same bfloat16 rows.  The weights and the result are rounded to bfloat16 once each (2^-8 of themselves at most), the
-    exponentials' arguments (up to 30 on base 2) to float32: 2^-7 + 30 * 2^-22 of the largest value; the talk mix sums H heads."""
+    exponentials' arguments (up to 30) to float32: 2^-7 + 30 * 2^-22 of the largest value; the talk mix sums H heads."""
     from zinfer_b200.parts.attention import query_tiles as attn_tiles_host
     lens, counts, page = [5, 64, 130, 333], [5, 64, 67, 200], 64
     setup = PagedSetup(lens, [2, 0, 3, 1], 4, page, Hkv, hd, torch.bfloat16, seed=4)
