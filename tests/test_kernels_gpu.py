@@ -1340,8 +1340,8 @@ def test_prompt_attention_of_large_scores(k, H, Hkv, hd, window):
 
 @pytest.mark.parametrize("D,F,E,top,n", [(2048, 2048, 16, 2, 8), (1024, 1024, 16, 2, 64), (4104, 4104, 5, 2, 8), (1024, 4104, 4, 2, 9), (4104, 1032, 4, 2, 1)])
 def test_experts_of_few_rows_sum_in_float32(k, D, F, E, top, n):
-    """The products of an expert's second matrix against 64 bits on the hidden rows as they were stored.  A warp adds the sums of 32 products
-    one after the other, then come 8 warps, up to 4 blocks and `top` experts: each of these n additions, and the 32 products' own
+    """The products of an expert's second matrix against 64 bits on the hidden rows as they were stored.  A warp adds the sums of 2 x 16
+    products one after the other, then come 8 warps, up to 4 blocks and `top` experts: each of these n additions, and the products' own
     sum, rounds to nearest, 2^-24 / sqrt(3) of partial sums that are no larger than the whole.  (The tensor core's own accumulator cuts
     off instead of rounding: over 32 steps of k it is 2 to 5 times further off.)"""
     x, w1 = rnd((n, D), 1, torch.bfloat16).cuda(), rnd((E, 2 * F, D), 2, torch.bfloat16, D ** -0.5).cuda()

@@ -220,14 +220,14 @@ namespace {
 // each matrix once from memory, so here a block owns 16 output units (hidden units, or outputs) of EVERY expert: it sorts
 // the step's pairs by expert in shared memory, walks the experts that have any, reads 16 rows of each once, straight into the
 // fragments of mma.m16n8k16, and multiplies them with up to 16 of the expert's rows (8 to a fragment).  The products of
-// bfloat16 values are exact.  The tensor core adds up 32 of them; those sums are added in float32, rounded to nearest, because its own
+// bfloat16 values are exact.  The tensor core adds up 16 of them; those sums are added in float32, rounded to nearest, because its own
 // accumulator cuts off: carried over all of a warp's k it was 1.7e-7 of the result off for K = 1024 to 4096 and 6.1e-7 with 16
-// steps of k a warp (K = 4104), where the kernels above are 0.9e-7 to 1.25e-7 off.  A lane takes 16 contiguous bytes of a weight row and of an
+// steps of k a warp (K = 4104).  So it is 0.83e-7 (K = 1024) to 1.06e-7 (4104) off, the kernels above are 0.87e-7 to 1.24e-7.  A lane takes 16 contiguous bytes of a weight row and of an
 // input row for two MMAs; both use the same order of k inside 32, which a sum does not see.  K is split over the block's
 // warps; where that leaves SMs idle, a cluster's blocks split K further (`k_parts`, while every warp keeps 128 k or more: what a
 // warp does per expert besides must pay) and then share the experts out among themselves.  The loads of the next expert are
 // under way while this one is multiplied (a ring of registers that runs on across experts).  All partial sums wait in shared
-// memory and are added in the order of warps, then of blocks; a result depends on how K is split alone, which the
+// memory and are added over the warps in pairs, then in the order of blocks; a result depends on how K is split alone, which the
 // sizes of the model decide: not on the step's other tokens.  Everything a token needs is in one cluster, so its experts are
 // added in the order of k without another kernel.
 // 8 tokens with 2 of 16 experts each (11 different ones), D = F = 2048, both kernels in a chain: 77 us once per pair, 53 here (an
@@ -433,11 +433,11 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const Ex
 #pragma unroll
         for (int u = 0; u < NG; ++u) {
           const float none[4] = {0.f, 0.f, 0.f, 0.f};
-          float sum[4];                          // of these 32 k
-          mma_bf16(sum, st.w[t][0].x, st.w[t][1].x, st.w[t][0].y, st.w[t][1].y, st.x[u].x, st.x[u].y, none);
-          mma_bf16(sum, st.w[t][0].z, st.w[t][1].z, st.w[t][0].w, st.w[t][1].w, st.x[u].z, st.x[u].w, sum);
+          float sum[2][4];                       // of 16 k each
+          mma_bf16(sum[0], st.w[t][0].x, st.w[t][1].x, st.w[t][0].y, st.w[t][1].y, st.x[u].x, st.x[u].y, none);
+          mma_bf16(sum[1], st.w[t][0].z, st.w[t][1].z, st.w[t][0].w, st.w[t][1].w, st.x[u].z, st.x[u].w, none);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[t][u][j] += sum[j];
+          for (int j = 0; j < 4; ++j) acc[t][u][j] += sum[0][j] + sum[1][j];
         }
       fetch(ring[r]);
       if (++s < s1) continue;
@@ -462,10 +462,14 @@ __global__ void __launch_bounds__(MOE_WARPS * 32, 2) expert_rows_kernel(const Ex
   for (int i = tid; i < n_pairs * TILES * 16; i += MOE_WARPS * 32) {
     if (walk_of[i / (TILES * 16)] % shares_w != share_w) continue;     // another block's
     const int at = i / (TILES * 16) * LD + i % (TILES * 16);
-    float v = 0.f;
+    float v[MOE_WARPS];                            // added in pairs: fewer roundings of the whole than one warp after the other
 #pragma unroll
-    for (int w = 0; w < MOE_WARPS; ++w) v += part[(size_t)w * n_pairs * LD + at];
-    part[at] = v;
+    for (int w = 0; w < MOE_WARPS; ++w) v[w] = part[(size_t)w * n_pairs * LD + at];
+#pragma unroll
+    for (int step = 1; step < MOE_WARPS; step *= 2)
+#pragma unroll
+      for (int w = 0; w < MOE_WARPS; w += 2 * step) v[w] += v[w + step];
+    part[at] = v[0];
   }
   cluster_barrier();
   auto sum = [&](int pair, int row) {              // from the blocks that had the pair's walk
